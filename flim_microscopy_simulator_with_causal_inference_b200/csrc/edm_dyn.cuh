@@ -27,6 +27,8 @@
 //    reference's order key.
 #pragma once
 
+#include <type_traits>
+
 #include "edm_common.cuh"
 
 namespace edm {
@@ -90,8 +92,8 @@ struct DevState {
   int32_t* pl_index;
   // per species: the density grids (bit g) that sense it in some replica
   uint32_t sensor_grids[EDM_MAX_SPECIES];
-  // the contact search's sweepers of this step (k_sweep_list), block by block
-  int32_t* sw_list;
+  // the contact search's sweepers (slot, replica) of this step (k_sweep_list)
+  int2* sw_list;
   int32_t* sw_count;
   // per global grid cell: the adaptation field w (float64, on the adaptation
   // grid's cells) and the local-recruitment CDF (on a feedback grid's cells)
@@ -1014,21 +1016,18 @@ __global__ void __launch_bounds__(BS, MINB) k_move(const EdmDynParams* __restric
 // * late pairs, whose partner an earlier catalytic pass of the step turns
 //   into S_c, are few: the pass that converts a particle looks up its
 //   enzymes of the later reactions at once (late_contacts).
-// A late pair is filed only when its keyed draw for the pass lies below the
-// pass's threshold (the pass rejects it otherwise); the sweep files every
-// direct pair and leaves the draws to the passes (a Philox per pair inside
-// the sweep measured slower).  A pair can be filed twice (a partner converted
-// away and back); the passes accept a substrate once, so duplicates change
-// nothing.
-constexpr int kContactSmem = 2048;
-
+// A pair is filed only when its keyed draw for the pass lies below the pass's
+// threshold (the pass rejects it otherwise).  A pair can be filed twice (a
+// partner converted away and back); the passes accept a substrate once, so
+// duplicates change nothing.
 struct CatLists {
-  uint32_t sweep_rx[EDM_MAX_SPECIES];        // reactions whose direct pairs the species sweeps for
-  uint32_t sweep_partners[EDM_MAX_SPECIES];  // species those sweeps look for
-  int32_t other[EDM_MAX_CAT];                // species the sweeper of reaction c looks for
-  uint32_t from_enzyme;                      // reactions swept from the enzyme side
-  int n_cat;
+  // byte [sweeper species][other species]: the reactions whose direct pairs
+  // the first sweeps for among the second
+  uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
+  uint32_t partners[EDM_MAX_SPECIES];  // species the sweeper species looks for
+  uint32_t from_enzyme;                // reactions swept from the enzyme side
 };
+static_assert(EDM_MAX_CAT <= 8, "rx_of holds a reaction set per byte");
 
 // Whether pass c's keyed draw for the pair of local ids (a, b) of replica r
 // lies below the pass's threshold.  The pass rejects the pair otherwise,
@@ -1039,283 +1038,288 @@ __device__ __forceinline__ bool cat_draw_passes(const EdmDynParams& p, const Dev
   return draw_u53(p.seed, step, EDM_S_CAT + c, lo, hi) < st.cat_thr[(int64_t)r * EDM_MAX_CAT + c];
 }
 
-// One neighbour j (pre-move cell offset dcx, dcy) of sweeper s: the pair
-// tests, then stage(c, enzyme, substrate) for each reaction of rx it meets.
-// oi_pre / oi_post / (cxs, cys): the sweeper's float32 offsets and post-move
-// cell (float32 path).
-template <bool F64, typename Stage>
-__device__ __forceinline__ void contact_candidate(const EdmDynParams& p, const Geo& g, const DevState& st,
-                                                  const CatLists& L, int64_t s, int j, int dcx, int dcy,
-                                                  uint32_t rx, uint32_t pmask,
-                                                  float2 oi_pre, float2 oi_post, int cxs, int cys, Stage stage) {
-  if (j == s) return;
-  const uint8_t fj = st.flags[j];
-  const int spj = fl_species(fj);
-  if (!fl_alive(fj) || !((pmask >> spj) & 1u)) return;
-  double d2;
-  if constexpr (F64) {
-    if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, s, j, g) < g.cutoff_sq())) return;
-    d2 = sep_sq<F64>(st.pos_post, st.cell_post, s, j, g);
-  } else {
-    // pre-move: j sits in the neighbour cell at (dcx, dcy)
-    const float2 oj = ((const float2*)st.pos_pre)[j];
-    const float fdx = __fmaf_rn(-(float)dcx, g.sxf, oi_pre.x - oj.x);
-    const float fdy = __fmaf_rn(-(float)dcy, g.syf, oi_pre.y - oj.y);
-    if (!((double)__fmaf_rn(fdx, fdx, fdy * fdy) < g.cutoff_sq())) return;
-    float dx, dy;
-    d2 = (double)rel_sq_f32_xy(cxs, cys, oi_post, st.cell_post[j], ((const float2*)st.pos_post)[j], g, dx, dy);
+// Neighbour sweep of one slot by G lanes (G divides 32, one group of G lanes
+// per slot; every lane of the warp calls it, `have` false for a group without
+// a slot).  The alive slots of the 3x3 block around cell c are three
+// consecutive runs, one per neighbour column (and three more where the block
+// wraps in y); the group's lanes take consecutive slots of the runs laid end
+// to end, so neighbouring lanes read neighbouring addresses and a lane is idle
+// only in the last round.  f(j, valid, column, col + cy) is called by the
+// whole warp, column = dcx + 1; the slot's row offset is
+// row_offset(cell_pre[j] - (col + cy), g).
+template <int G, typename F>
+__device__ __forceinline__ void for_neighbour_slots_grouped(const Geo& g, const DevState& st, int c, bool have, F f) {
+  const int lane = threadIdx.x & (G - 1);
+  int cx, cy;
+  split_cell(c, g, cx, cy);
+  int ya = cy - 1, yb = cy + 1, wrapped = -1;  // the row that wraps in y
+  if (ya < 0) {
+    ya = 0;
+    wrapped = g.ny - 1;
+  } else if (yb >= g.ny) {
+    yb = g.ny - 1;
+    wrapped = 0;
   }
-  for (uint32_t bits = rx; bits; bits &= bits - 1) {
-    const int c = __ffs(bits) - 1;
-    if (spj != L.other[c] || d2 > p.cat[c].contact_sq) continue;
-    if ((L.from_enzyme >> c) & 1u) stage(c, (int)s, j);
-    else stage(c, j, (int)s);
+  if (!have || !g.py) wrapped = -1;
+  for (int part = 0; part < 2; ++part) {
+    int lo[3], len[3], base[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      int ncx = cx + d - 1;
+      bool in = have;
+      if (g.px) ncx = ncx < 0 ? ncx + g.nx : (ncx >= g.nx ? ncx - g.nx : ncx);
+      else in = in && ncx >= 0 && ncx < g.nx;
+      lo[d] = len[d] = 0;
+      base[d] = ncx * g.ny + cy;
+      if (in) {
+        const int32_t* b = st.cell_start + g.cbase + ncx * g.ny;
+        lo[d] = b[ya];
+        len[d] = b[yb + 1] - lo[d];
+      }
+    }
+    const int n0 = len[0], n1 = n0 + len[1], n = n1 + len[2];
+    lo[1] -= n0;
+    lo[2] -= n1;
+    const int most = __reduce_max_sync(0xffffffffu, n);
+    for (int q0 = 0; q0 < most; q0 += G) {
+      const int q = q0 + lane;
+      const bool a1 = q >= n0, a2 = q >= n1;
+      f(q + (a2 ? lo[2] : (a1 ? lo[1] : lo[0])), q < n, a2 ? 2 : (a1 ? 1 : 0), a2 ? base[2] : (a1 ? base[1] : base[0]));
+    }
+    if (!__any_sync(0xffffffffu, wrapped >= 0)) break;
+    have = wrapped >= 0;  // the second part: the wrapped row alone
+    ya = yb = wrapped >= 0 ? wrapped : 0;
+    wrapped = -1;
   }
 }
 
-// Shared-memory staging of a block's contact pairs, per reaction, then one
-// global append per reaction; a full stage appends directly.
-struct ContactStage {
-  int2* buf;
-  int* nbuf;
-  int per;
-  __device__ __forceinline__ void operator()(const DevState& st, int c, int e, int sub) const {
-    const int k = atomicAdd(&nbuf[c], 1);
-    if (k < per) {
-      buf[c * per + k] = make_int2(e, sub);
-    } else {
-      const int q = atomicAdd(&st.contact_count[c], 1);
-      if (q < st.contact_cap) st.contacts[(int64_t)c * st.contact_cap + q] = make_int2(e, sub);
-      else set_status(st.status, EDM_STATUS_CONTACT_CAP);
-    }
-  }
-};
-
-__device__ __forceinline__ void flush_contacts(const DevState& st, const CatLists& L, const ContactStage& S,
-                                               int* base) {
-  __syncthreads();
-  if (threadIdx.x < L.n_cat) {
-    const int n = S.nbuf[threadIdx.x] < S.per ? S.nbuf[threadIdx.x] : S.per;
-    base[threadIdx.x] = n > 0 ? atomicAdd(&st.contact_count[threadIdx.x], n) : 0;
-  }
-  __syncthreads();
-  for (int c = 0; c < L.n_cat; ++c) {
-    const int n = S.nbuf[c] < S.per ? S.nbuf[c] : S.per;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const int64_t q = (int64_t)base[c] + k;
-      if (q < st.contact_cap) st.contacts[(int64_t)c * st.contact_cap + q] = S.buf[c * S.per + k];
-      else set_status(st.status, EDM_STATUS_CONTACT_CAP);
-    }
-  }
+__device__ __forceinline__ int row_offset(int d, const Geo& g) {
+  return d > 1 ? d - g.ny : (d < -1 ? d + g.ny : d);
 }
 
-template <bool F64, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_contacts(const EdmDynParams* __restrict__ P, DevState st, Match m,
-                                                     CatLists L) {
-  pdl_enter();
-  __shared__ int2 buf[kContactSmem];
-  __shared__ int nbuf[EDM_MAX_CAT], base[EDM_MAX_CAT];
-  const ContactStage S{buf, nbuf, L.n_cat > 0 ? kContactSmem / L.n_cat : kContactSmem};
-  if (threadIdx.x < EDM_MAX_CAT) nbuf[threadIdx.x] = 0;
-  __syncthreads();
-  sweep4(st, m, [&](int r, int64_t s) {
-    const EdmDynParams& p = P[r];
-    const Geo g(p);
-    const int sps = fl_species(st.flags[s]);
-    const uint32_t rx = L.sweep_rx[sps], pmask = L.sweep_partners[sps];
-    float2 oi_pre = make_float2(0.f, 0.f), oi_post = make_float2(0.f, 0.f);
-    int cxs = 0, cys = 0;
-    if constexpr (!F64) {
-      oi_pre = ((const float2*)st.pos_pre)[s];
-      oi_post = ((const float2*)st.pos_post)[s];
-      split_cell(st.cell_post[s], g, cxs, cys);
-    }
-    for_neighbour_slots(g, st, st.cell_pre[s], [&](int j, int, int dcx, int dcy) {
-      contact_candidate<F64>(p, g, st, L, s, j, dcx, dcy, rx, pmask, oi_pre, oi_post, cxs, cys,
-                             [&](int c, int e, int sub) { S(st, c, e, sub); });
-    });
-  });
-  flush_contacts(st, L, S, base);
-}
-
-// The per-sweeper work of the column-task contact search: sweeper s, its
-// neighbour column dcx (-1, 0, 1); r0 is a replica at or before s's.
-template <bool F64, typename Stage>
-__device__ __forceinline__ void contact_column_task(const EdmDynParams* __restrict__ P, const DevState& st,
-                                                    const CatLists& L, int64_t s, int dcx, int r0, Stage stage) {
-  int r = r0;
-  while (r + 1 < st.n_rep && st.rep_first[r + 1] <= s) ++r;
-  const EdmDynParams& p = P[r];
-  const Geo g(p);
-  const int sps = fl_species(st.flags[s]);
-  const uint32_t rx = L.sweep_rx[sps], pmask = L.sweep_partners[sps];
-  float2 oi_pre = make_float2(0.f, 0.f), oi_post = make_float2(0.f, 0.f);
-  int cxs = 0, cys = 0;
-  if constexpr (!F64) {
-    oi_pre = ((const float2*)st.pos_pre)[s];
-    oi_post = ((const float2*)st.pos_post)[s];
-    split_cell(st.cell_post[s], g, cxs, cys);
-  }
-  for_neighbour_slots_box(g, st, st.cell_pre[s], dcx, dcx, -1, 1, [&](int j, int, int dcx_, int dcy) {
-    contact_candidate<F64>(p, g, st, L, s, j, dcx_, dcy, rx, pmask, oi_pre, oi_post, cxs, cys, stage);
-  });
-}
-
-// The same contact search with the work spread over (sweeper, neighbour
-// column) tasks: a warp compacts the sweepers of its kSweepChunk slots in
-// shared memory (as sweep4 does), then each lane takes tasks t = lane,
-// lane + 32, ... (sweeper t / 3, column t % 3 - 1) and walks that column's
-// one or two slot runs.  A lane's loop is about three candidates instead of
-// nine, so lanes idle less while the longest run finishes.  Same tests, same
-// contact set (in another order, which the catalytic passes do not depend
-// on).
-template <bool F64, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_contacts_cols(const EdmDynParams* __restrict__ P, DevState st,
-                                                              Match m, CatLists L) {
-  pdl_enter();
-  __shared__ int2 buf[kContactSmem];
-  __shared__ int nbuf[EDM_MAX_CAT], base[EDM_MAX_CAT];
-  __shared__ int32_t list[kBlock / 32][kSweepChunk];
-  const ContactStage S{buf, nbuf, L.n_cat > 0 ? kContactSmem / L.n_cat : kContactSmem};
-  if (threadIdx.x < EDM_MAX_CAT) nbuf[threadIdx.x] = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) * 4;
-  int n = 0, r0 = 0;
-  if (w0 < st.n_slots) {  // whole warps: compact the chunk's sweepers
-    const int64_t s0 = w0 + (int64_t)lane * 4;
-    uchar4 f4 = make_uchar4(0, 0, 0, 0);
-    if (s0 < st.n_slots) f4 = *reinterpret_cast<const uchar4*>(st.flags + s0);
-    const uint8_t fl[4] = {f4.x, f4.y, f4.z, f4.w};
-    const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const bool hit = s0 + k < st.n_slots && matches(fl[k], m);
-      const unsigned bits = __ballot_sync(0xffffffffu, hit);
-      if (hit) list[wid][n + __popc(bits & below)] = (int32_t)(s0 + k);
-      n += __popc(bits);
-    }
-    r0 = st.chunk_rep[w0 / kSweepChunk];
-  }
-  __syncwarp();
-  for (int t = lane; t < 3 * n; t += 32) {
-    const int q = t / 3;
-    contact_column_task<F64>(P, st, L, list[wid][q], t - 3 * q - 1, r0,
-                             [&](int c, int e, int sub) { S(st, c, e, sub); });
-  }
-  flush_contacts(st, L, S, base);
-}
-
-// Block compaction of the slots matching m among the block's kBlock * SPT
-// slots from b0 (SPT per thread, in slot order per thread): writes them to
-// list (kBlock * SPT entries of shared memory) and returns their number.
-// Every thread of the block calls it.
-template <int SPT>
-__device__ __forceinline__ int block_compact(const DevState& st, const Match& m, int64_t b0, int32_t* list,
-                                             int* woff) {
-  static_assert(SPT == 4 || SPT == 16, "4 or 16 slots per thread");
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t s0 = b0 + (int64_t)threadIdx.x * SPT;
-  uint8_t fl[SPT];
-  if (s0 + SPT <= st.n_slots) {  // s0 and SPT are multiples of SPT bytes: aligned
-    if constexpr (SPT == 16) {
-      const uint4 v = *reinterpret_cast<const uint4*>(st.flags + s0);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 16; ++k) fl[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
-    } else {
-      const uchar4 f4 = *reinterpret_cast<const uchar4*>(st.flags + s0);
-      fl[0] = f4.x, fl[1] = f4.y, fl[2] = f4.z, fl[3] = f4.w;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < SPT; ++k) fl[k] = s0 + k < st.n_slots ? st.flags[s0 + k] : (uint8_t)0;
-  }
-  unsigned hits = 0;  // bit k: slot s0 + k matches
-#pragma unroll
-  for (int k = 0; k < SPT; ++k)
-    if (s0 + k < st.n_slots && matches(fl[k], m)) hits |= 1u << k;
-  int wn = 0;
-#pragma unroll
-  for (int k = 0; k < SPT; ++k) wn += __popc(__ballot_sync(0xffffffffu, (hits >> k) & 1u));
-  if (lane == 0) woff[wid + 1] = wn;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    woff[0] = 0;
-    for (int w = 1; w <= kBlock / 32; ++w) woff[w] += woff[w - 1];
-  }
-  __syncthreads();
-  const unsigned below = (1u << lane) - 1u;
-  int at = woff[wid];
+// The alive-or-not species matches among the BLK * SPT slots from s0 (below
+// end), gathered in the block's shared list in any order.
+template <int BLK, int SPT>
+__device__ __forceinline__ void gather_matching(const DevState& st, const Match& m, int64_t s0, int64_t end,
+                                                int32_t* list, int& n_list) {
+  uint8_t f[SPT];
 #pragma unroll
   for (int k = 0; k < SPT; ++k) {
-    const bool hit = (hits >> k) & 1u;
-    const unsigned bits = __ballot_sync(0xffffffffu, hit);
-    if (hit) list[at + __popc(bits & below)] = (int32_t)(s0 + k);
-    at += __popc(bits);
+    const int64_t s = s0 + k * BLK + threadIdx.x;
+    f[k] = s < end ? st.flags[s] : (uint8_t)0;
   }
-  __syncthreads();
-  return woff[kBlock / 32];
+  const int lane = threadIdx.x & 31;
+  unsigned hits = 0;
+#pragma unroll
+  for (int k = 0; k < SPT; ++k)
+    if (s0 + k * BLK + threadIdx.x < end && matches(f[k], m)) hits |= 1u << k;
+  // one shared atomic per warp: lane l's hits go after those of the lanes below
+  const int mine = __popc(hits);
+  int upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, upto, 31);
+  if (total == 0) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(&n_list, total);
+  at = __shfl_sync(0xffffffffu, at, 0) + upto - mine;
+  for (; hits; hits &= hits - 1) list[at++] = (int32_t)(s0 + (__ffs(hits) - 1) * BLK + threadIdx.x);
 }
 
-// The contact search's sweepers as one global list: each block compacts its
-// kBlock * 16 slots and appends them with one atomic (launch with
-// ceil(n_slots / (16 kBlock)) blocks of kBlock).
-__global__ void __launch_bounds__(kBlock) k_sweep_list(DevState st, Match m) {
+// A warp's pairs (sweeper, neighbour, replica) that passed the pre-move test
+// of the sweep.  About one neighbour in six does, so the rest of the work
+// (post-move contact, keyed draw, listing) is done 32 pairs at a time with
+// every lane busy.
+struct ContactQueue {
+  int2 pair[64];
+  int32_t rep[64];
+};
+
+// The first k <= 32 pairs of the queue: the post-move contact radius of each
+// reaction the pair meets, then the reaction's keyed draw; the pairs below
+// the pass's threshold are listed.
+template <bool F64>
+__device__ __forceinline__ void finish_contacts(const EdmDynParams* __restrict__ P, const DevState& st,
+                                                const CatLists& L, const uint8_t* rx_of, const ContactQueue& Q,
+                                                int k) {
+  const int lane = threadIdx.x & 31;
+  if (lane >= k) return;
+  const int2 sj = Q.pair[lane];
+  const int r = Q.rep[lane];
+  const EdmDynParams& p = P[r];
+  const Geo g(p);
+  uint32_t bits = rx_of[fl_species(st.flags[sj.x]) * EDM_MAX_SPECIES + fl_species(st.flags[sj.y])];
+  const int ids = st.ids[sj.x] - g.poff, idj = st.ids[sj.y] - g.poff;
+  // the sweeper first, as the pre-move test (both differences change sign
+  // exactly when the pair is swept from its other side)
+  const double d2 = sep_sq<F64>(st.pos_post, st.cell_post, sj.x, sj.y, g);
+  for (; bits; bits &= bits - 1) {
+    const int c = __ffs(bits) - 1;
+    if (d2 > p.cat[c].contact_sq) continue;
+    if (!cat_draw_passes(p, st, r, c, ids, idj, *st.d_step)) continue;
+    const int q = atomicAdd(&st.contact_count[c], 1);
+    if (q < st.contact_cap)
+      st.contacts[(int64_t)c * st.contact_cap + q] = (L.from_enzyme >> c) & 1u ? sj : make_int2(sj.y, sj.x);
+    else set_status(st.status, EDM_STATUS_CONTACT_CAP);
+  }
+}
+
+// Sweeper s of replica r (one per group of G lanes, `have` false for a group
+// without one) against its neighbour slots: alive, of a species it sweeps
+// for, within the pre-move cutoff.  The pairs go to the warp's queue, `queued`
+// of them wait there.
+template <bool F64, int G>
+__device__ __forceinline__ void contact_sweep(const EdmDynParams* __restrict__ P, const DevState& st,
+                                              const CatLists& L, const uint8_t* rx_of, int r, int s, bool have,
+                                              ContactQueue& Q, int& queued) {
+  const EdmDynParams& p = P[r];
+  const Geo g(p);
+  const int lane = threadIdx.x & 31;
+  const uint32_t pmask = L.partners[fl_species(st.flags[s])];
+  const int c_pre = st.cell_pre[s];
+  float2 oi = make_float2(0.f, 0.f);
+  double2 xi = make_double2(0.0, 0.0);
+  // a float is below the float64 bound exactly when it is below the smallest
+  // float at or above it: the float32 path compares in float32
+  const float cutoff_f = __double2float_ru(p.cutoff_sq);
+  if constexpr (F64) xi = ((const double2*)st.pos_pre)[s];
+  else oi = ((const float2*)st.pos_pre)[s];
+  for_neighbour_slots_grouped<G>(g, st, c_pre, have, [&](int j, bool valid, int column, int base) {
+    bool hit = false;
+    if (valid) {
+      const uint8_t fj = st.flags[j];
+      if constexpr (F64) {
+        const double2 v = ((const double2*)st.pos_pre)[j];
+        double dx, dy;
+        hit = fl_alive(fj) && ((pmask >> fl_species(fj)) & 1u) && j != s &&
+              min_image_sq(xi.x, xi.y, v.x, v.y, g, dx, dy) < g.cutoff_sq();
+      } else {
+        const float2 o = ((const float2*)st.pos_pre)[j];
+        const int dcy = row_offset(st.cell_pre[j] - base, g);
+        // j sits in the neighbour cell at (column - 1, dcy)
+        const float fdx = __fmaf_rn(-(float)(column - 1), g.sxf, oi.x - o.x);
+        const float fdy = __fmaf_rn(-(float)dcy, g.syf, oi.y - o.y);
+        hit = fl_alive(fj) && ((pmask >> fl_species(fj)) & 1u) && j != s &&
+              __fmaf_rn(fdx, fdx, fdy * fdy) < cutoff_f;
+      }
+    }
+    const unsigned who = __ballot_sync(0xffffffffu, hit);
+    if (!who) return;
+    if (hit) {
+      const int at = queued + __popc(who & ((1u << lane) - 1u));
+      Q.pair[at] = make_int2(s, j);
+      Q.rep[at] = r;
+    }
+    queued += __popc(who);
+    __syncwarp();
+    if (queued < 32) return;  // at most 31 + 32 wait here
+    finish_contacts<F64>(P, st, L, rx_of, Q, 32);
+    __syncwarp();
+    queued -= 32;
+    if (lane < queued) {
+      const int2 e = Q.pair[32 + lane];
+      const int32_t k = Q.rep[32 + lane];
+      Q.pair[lane] = e;
+      Q.rep[lane] = k;
+    }
+    __syncwarp();
+  });
+}
+
+// Contact search of the step.  What bounds it is the chain of round trips to
+// L2 (sweeper, bucket bounds, neighbours, their post-move positions) and the
+// instructions per neighbour, not bytes: groups of G lanes take one sweeper
+// each and its neighbour slots G at a time, so a group's chain is a few rounds
+// long whatever the runs' lengths, and the pairs beyond the pre-move test are
+// finished 32 at a time.  A lane per sweeper and column, walking slot by
+// slot, chained three dependent loads per neighbour with 12 of 32 lanes
+// active: 25 us per step for a 5,000-slot system and 56 us for 464,000 slots
+// (float64), against 14 and 26 us here; for 4.7M slots 63 us, against 54 us
+// with the pairs' draws taken too.  64 registers without spills at 4 blocks per
+// SM beat 5, 6 and 8 blocks with spills (42.6 / 48.3 / 50 / 60 us at 1.86M
+// slots).  G follows the neighbours per sweeper, nine cells' occupancy (4
+// lanes at one particle per cell, 54 against 61 us with 8; 8 to 16 at four):
+// the autotuner chooses it.
+//
+// k_contacts: a block takes a tile of BLK * SPT slots of one replica and
+// gathers its sweepers in shared memory.  One launch and one block's chain:
+// the form for systems that do not fill the chip.
+template <bool F64, int BLK, int SPT, int G, int MINB>
+__global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __restrict__ P,
+                                                      const int2* __restrict__ blk, DevState st, Match m,
+                                                      const __grid_constant__ CatLists L) {
   pdl_enter();
-  __shared__ int32_t list[kBlock * 16];
-  __shared__ int woff[kBlock / 32 + 1];
-  __shared__ int at;
-  const int n = block_compact<16>(st, m, (int64_t)blockIdx.x * kBlock * 16, list, woff);
-  if (threadIdx.x == 0) at = n > 0 ? atomicAdd(st.sw_count, n) : 0;
+  __shared__ int32_t list[BLK * SPT];
+  __shared__ ContactQueue queue[BLK / 32];
+  __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
+  __shared__ int n_list;
+  const int2 b = blk[blockIdx.x];
+  const int64_t end = P[b.x].particle_offset + P[b.x].n_particles;
+  if (threadIdx.x == 0) n_list = 0;
+  if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
   __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) st.sw_list[at + k] = list[k];
+  gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)b.y, end, list, n_list);
+  __syncthreads();
+  const int sweepers = n_list, lane = threadIdx.x & 31;
+  ContactQueue& Q = queue[threadIdx.x >> 5];
+  int queued = 0;
+  for (int t0 = (threadIdx.x >> 5) * (32 / G); t0 < sweepers; t0 += BLK / G) {  // whole warps
+    const int t = t0 + lane / G;
+    contact_sweep<F64, G>(P, st, L, (const uint8_t*)rx_of, b.x, list[t < sweepers ? t : t0], t < sweepers, Q, queued);
+  }
+  finish_contacts<F64>(P, st, L, (const uint8_t*)rx_of, Q, queued);
 }
 
-// The column tasks over the global sweeper list, one wave of blocks walking
-// the tasks grid-stride: every lane has a task however the sweepers cluster.
-template <bool F64, int MINB>
+// The sweepers of the step as one global list of (slot, replica), tile by
+// tile, for k_contacts_list.
+constexpr int kSweepSlots = 16;  // per thread
+__global__ void __launch_bounds__(kBlock) k_sweep_list(const EdmDynParams* __restrict__ P,
+                                                       const int2* __restrict__ blk, DevState st, Match m) {
+  pdl_enter();
+  __shared__ int32_t list[kBlock * kSweepSlots];
+  __shared__ int n_list, at;
+  const int2 b = blk[blockIdx.x];
+  if (threadIdx.x == 0) n_list = 0;
+  __syncthreads();
+  gather_matching<kBlock, kSweepSlots>(st, m, (int64_t)(uint32_t)b.y, P[b.x].particle_offset + P[b.x].n_particles, list,
+                                       n_list);
+  __syncthreads();
+  const int n = n_list;
+  if (n == 0) return;
+  if (threadIdx.x == 0) at = atomicAdd(st.sw_count, n);
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += kBlock) st.sw_list[at + k] = make_int2(list[k], b.x);
+}
+
+// The same sweep over the global list, one wave of blocks: no per-tile
+// prologue and every group has a sweeper until the list ends, which pays when
+// the sweepers outnumber the chip's groups several times.
+template <bool F64, int G, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynParams* __restrict__ P, DevState st,
-                                                              CatLists L) {
+                                                              const __grid_constant__ CatLists L) {
   pdl_enter();
-  __shared__ int2 buf[kContactSmem];
-  __shared__ int nbuf[EDM_MAX_CAT], base[EDM_MAX_CAT];
-  const ContactStage S{buf, nbuf, L.n_cat > 0 ? kContactSmem / L.n_cat : kContactSmem};
-  if (threadIdx.x < EDM_MAX_CAT) nbuf[threadIdx.x] = 0;
+  __shared__ ContactQueue queue[kBlock / 32];
+  __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
+  if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
   __syncthreads();
-  const int64_t tasks = 3 * (int64_t)*st.sw_count;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tasks; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t q = t / 3;
-    const int64_t s = st.sw_list[q];
-    contact_column_task<F64>(P, st, L, s, (int)(t - 3 * q) - 1, st.chunk_rep[s / kSweepChunk],
-                             [&](int c, int e, int sub) { S(st, c, e, sub); });
+  const int n = *st.sw_count, lane = threadIdx.x & 31;
+  const int stride = (int)gridDim.x * (kBlock / G);
+  ContactQueue& Q = queue[threadIdx.x >> 5];
+  int queued = 0;
+  int t0 = (int)(blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * (32 / G);
+  if (t0 >= n) return;
+  int2 e = st.sw_list[min(t0 + lane / G, n - 1)];
+  while (t0 < n) {  // whole warps; the next sweeper is read while this one is swept
+    const bool have = t0 + lane / G < n;
+    const int2 cur = e;
+    t0 += stride;
+    if (t0 < n) e = st.sw_list[min(t0 + lane / G, n - 1)];
+    contact_sweep<F64, G>(P, st, L, (const uint8_t*)rx_of, cur.y, cur.x, have, Q, queued);
   }
-  flush_contacts(st, L, S, base);
-}
-
-// The column tasks balanced over the whole block: the block compacts the
-// sweepers of its kBlock * SPT slots (SPT per thread) into one shared list,
-// so a warp whose slots hold a cluster of sweepers shares them with the
-// block's other warps instead of keeping the block waiting.
-template <bool F64, int MINB, int SPT>
-__global__ void __launch_bounds__(kBlock, MINB) k_contacts_block(const EdmDynParams* __restrict__ P, DevState st,
-                                                               Match m, CatLists L) {
-  pdl_enter();
-  __shared__ int2 buf[kContactSmem];
-  __shared__ int nbuf[EDM_MAX_CAT], base[EDM_MAX_CAT];
-  __shared__ int32_t list[kBlock * SPT];
-  __shared__ int woff[kBlock / 32 + 1];
-  const ContactStage S{buf, nbuf, L.n_cat > 0 ? kContactSmem / L.n_cat : kContactSmem};
-  if (threadIdx.x < EDM_MAX_CAT) nbuf[threadIdx.x] = 0;
-  const int64_t b0 = (int64_t)blockIdx.x * blockDim.x * SPT;
-  const int n = block_compact<SPT>(st, m, b0, list, woff);  // its barriers also publish nbuf
-  const int r0 = n > 0 ? st.chunk_rep[b0 / kSweepChunk] : 0;
-  for (int t = threadIdx.x; t < 3 * n; t += blockDim.x) {
-    const int q = t / 3;
-    contact_column_task<F64>(P, st, L, list[q], t - 3 * q - 1, r0,
-                             [&](int c, int e, int sub) { S(st, c, e, sub); });
-  }
-  flush_contacts(st, L, S, base);
+  finish_contacts<F64>(P, st, L, (const uint8_t*)rx_of, Q, queued);
 }
 
 // Late pairs of particle j, which a catalytic pass has just turned into the
@@ -1357,8 +1361,9 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
 
 // Catalytic pass c (dynamics.py:825-983) over its contact list: the set of
 // substrates with at least one accepted (enzyme, substrate) pair converts.
-// Every listed pair is alive, has the pass's enzyme and is within its contact
-// radius; only the partner's current species is left to test.
+// Every listed pair is alive, has the pass's enzyme, is within its contact
+// radius and has its draw below the pass's threshold; the partner's current
+// species and the exact probability are left to test.
 // `late`: the later reactions whose substrate is this pass's product.
 template <bool F64>
 __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __restrict__ P, DevState st, int cidx,

@@ -82,15 +82,21 @@ constexpr LaunchShape kShapes[TK_COUNT][kMaxShapes] = {
     // k_move: the second number bounds its registers (80 at 256 x 3 down to 32
     // at 128 x 16, with spills below 64): occupancy pays more than the spills
     {{256, 3}, {256, 4}, {128, 8}, {128, 10}, {128, 12}, {128, 16}, {256, 6}, {256, 8}},
-    // k_contacts: 0 by sweeper; 1-2 by (sweeper, neighbour column) per warp;
-    // 3-5 the same tasks balanced over the block (16, 16, 4 slots per
-    // thread); 6-7 over a global sweeper list (k_sweep_list), one wave
-    {{256, 6}, {256, 6}, {256, 4}, {256, 6}, {256, 4}, {256, 6}, {256, 6}, {256, 8}},
+    // k_contacts: with kContactSlots slots per thread (0: over the global
+    // sweeper list, one wave of blocks) and kContactLanes lanes per sweeper
+    {{128, 8}, {128, 8}, {256, 4}, {256, 4}, {256, 4}, {256, 5}, {256, 3}, {256, 5}},
 };
+constexpr int kContactSlots[kMaxShapes] = {2, 4, 0, 0, 0, 0, 0, 0};
+constexpr int kContactLanes[kMaxShapes] = {8, 8, 8, 4, 16, 8, 8, 4};
 constexpr int kNumShapes[TK_COUNT] = {5, 8, 8};
 const char* const kTunedNames[TK_COUNT] = {"k_scatter", "k_move", "k_contacts"};
-constexpr int kTileSizes[3] = {128, 256, 512};
-int tile_index(int bs) { return bs == 128 ? 0 : (bs == 256 ? 1 : 2); }
+constexpr int kTileTables = 4;
+constexpr int kTileSizes[kTileTables] = {128, 256, 512, 4096};
+int tile_index(int bs) {
+  int t = 0;
+  while (kTileSizes[t] < bs) ++t;
+  return t;
+}
 
 // Choices of earlier tunings in this process, by (kernel, precision,
 // replicas, log2 of the slot count): later engines of the same kind reuse them.
@@ -114,9 +120,9 @@ struct EdmEngine {
   uint64_t *pass_thr = nullptr, *cat_thr = nullptr;  // draw thresholds ([R][kMaxPP], [R][EDM_MAX_CAT])
   int2 *pblk = nullptr, *eblk = nullptr, *phblk = nullptr, *pxblk = nullptr;
   int npblk = 0, neblk = 0, nphblk = 0, npxblk = 0;
-  // slot tiles of 128, 256 and 512 (the 256 table is pblk) for the tuned kernels
-  int2* pblk_bs[3] = {nullptr, nullptr, nullptr};
-  int npblk_bs[3] = {0, 0, 0};
+  // slot tiles of each of kTileSizes (the 256 table is pblk) for the tuned kernels
+  int2* pblk_bs[kTileTables] = {};
+  int npblk_bs[kTileTables] = {};
   // launch shape of each tuned kernel (index into kShapes), tuning timings
   int shape[TK_COUNT] = {0, 0, 0};
   float tuned_ms[TK_COUNT] = {0, 0, 0}, default_ms[TK_COUNT] = {0, 0, 0};
@@ -177,8 +183,9 @@ struct EdmEngine {
   int32_t *moved = nullptr, *moved_count = nullptr;
   int4* pl = nullptr;  // listed particles of the per-particle passes: (slot, pass bits, replica, id)
   int32_t *pl_count = nullptr, *pl_index = nullptr;
-  int32_t *sw_list = nullptr, *sw_count = nullptr;  // the contact search's sweeper list
   uint32_t sensor_grids[EDM_MAX_SPECIES] = {};  // per species: the grids that sense it in some replica
+  int2* sw_list = nullptr;  // the contact search's sweeper list
+  int32_t* sw_count = nullptr;
   double *adapt_w = nullptr, *local_cdf = nullptr;  // per global grid cell
   std::vector<int32_t> emit_host;  // emitter list last uploaded
   std::vector<uint8_t> has_dye_host;  // has_dye of the last edm_set_state
@@ -382,16 +389,14 @@ struct EdmEngine {
   void set_contact_sides(const int64_t* count, int32_t force_mask = -1) {
     const EdmDynParams& p = hdp[0];
     cat_lists = CatLists{};
-    cat_lists.n_cat = p.n_cat;
     uint32_t sweepers = 0;
     for (int c = 0; c < p.n_cat; ++c) {
       const int e = p.cat[c].enzyme, sub = p.cat[c].substrate;
       const bool from_enzyme = force_mask >= 0 ? ((force_mask >> c) & 1) != 0 : (!count || count[e] <= count[sub]);
       const int sw = from_enzyme ? e : sub, other = from_enzyme ? sub : e;
       if (from_enzyme) cat_lists.from_enzyme |= 1u << c;
-      cat_lists.other[c] = other;
-      cat_lists.sweep_rx[sw] |= 1u << c;
-      cat_lists.sweep_partners[sw] |= 1u << other;
+      cat_lists.partners[sw] |= 1u << other;
+      reinterpret_cast<uint8_t*>(cat_lists.rx_of)[sw * EDM_MAX_SPECIES + other] |= (uint8_t)(1u << c);
       sweepers |= 1u << sw;
     }
     for (Pass& ps : passes)
@@ -625,23 +630,33 @@ struct EdmEngine {
     }
   }
 
+  template <bool F64, int K>  // row K of kShapes[TK_CONTACTS], kContactSlots, kContactLanes
+  void contacts_shape(const DevState& st, const Match& m, cudaStream_t s) {
+    constexpr LaunchShape sh = kShapes[TK_CONTACTS][K];
+    constexpr int slots = kContactSlots[K], lanes = kContactLanes[K];
+    const int t = tile_index(slots > 0 ? sh.block * slots : kBlock * kSweepSlots);
+    if (npblk_bs[t] == 0) return;
+    if constexpr (slots > 0) {
+      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, npblk_bs[t], sh.block, s, dp, pblk_bs[t], st, m,
+         cat_lists);
+    } else {
+      static_assert(sh.block == kBlock, "the list form's blocks");
+      go(k_sweep_list, npblk_bs[t], kBlock, s, dp, pblk_bs[t], st, m);
+      go(k_contacts_list<F64, lanes, sh.min_blocks>, 148 * sh.min_blocks, kBlock, s, dp, st, cat_lists);
+    }
+  }
+
   template <bool F64>
-  void launch_contacts(const DevState& st, const Match& m, int grid, cudaStream_t s) {
-    const int grid16 = (int)((N + 16 * kBlock - 1) / (16 * kBlock));  // 16 slots per thread
-    if (grid16 == 0) return;
-    switch (shape[TK_CONTACTS]) {  // the rows of kShapes[TK_CONTACTS]
-      case 1: go(k_contacts_cols<F64, 6>, grid, kBlock, s, dp, st, m, cat_lists); break;
-      case 2: go(k_contacts_cols<F64, 4>, grid, kBlock, s, dp, st, m, cat_lists); break;
-      case 3: go(k_contacts_block<F64, 6, 16>, grid16, kBlock, s, dp, st, m, cat_lists); break;
-      case 4: go(k_contacts_block<F64, 4, 16>, grid16, kBlock, s, dp, st, m, cat_lists); break;
-      case 5: go(k_contacts_block<F64, 6, 4>, grid, kBlock, s, dp, st, m, cat_lists); break;
-      case 6:
-      case 7:
-        go(k_sweep_list, grid16, kBlock, s, st, m);
-        if (shape[TK_CONTACTS] == 6) go(k_contacts_list<F64, 6>, 148 * 6, kBlock, s, dp, st, cat_lists);
-        else go(k_contacts_list<F64, 8>, 148 * 8, kBlock, s, dp, st, cat_lists);
-        break;
-      default: go(k_contacts<F64, 6>, grid, kBlock, s, dp, st, m, cat_lists); break;
+  void launch_contacts(const DevState& st, const Match& m, cudaStream_t s) {
+    switch (shape[TK_CONTACTS]) {
+      case 1: contacts_shape<F64, 1>(st, m, s); break;
+      case 2: contacts_shape<F64, 2>(st, m, s); break;
+      case 3: contacts_shape<F64, 3>(st, m, s); break;
+      case 4: contacts_shape<F64, 4>(st, m, s); break;
+      case 5: contacts_shape<F64, 5>(st, m, s); break;
+      case 6: contacts_shape<F64, 6>(st, m, s); break;
+      case 7: contacts_shape<F64, 7>(st, m, s); break;
+      default: contacts_shape<F64, 0>(st, m, s); break;
     }
   }
 
@@ -689,7 +704,7 @@ struct EdmEngine {
         case P_DISSOC: go(k_dissociate<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
         case P_CONTACTS:
           tune_mark(TK_CONTACTS, 0, s);
-          launch_contacts<F64>(st, ps.match, sgrid, s);
+          launch_contacts<F64>(st, ps.match, s);
           tune_mark(TK_CONTACTS, 1, s);
           break;
         case P_CAT: go(k_catalytic<F64>, cgrid, kBlock, s, dp, st, ps.index, cat_late[ps.index]); break;
@@ -737,7 +752,7 @@ struct EdmEngine {
   int launches_per_step(bool with_photons) const {
     int n = 3 + 1 + 1 + (int)passes.size() + 1;
     for (const Pass& ps : passes)  // the sweeper-list contact shapes launch two kernels
-      if (ps.kind == P_CONTACTS && shape[TK_CONTACTS] >= 6) ++n;
+      if (ps.kind == P_CONTACTS && kContactSlots[shape[TK_CONTACTS]] == 0) ++n;
     if (with_photons) n += (neblk > 0 ? 3 : 1) + 1 + (nphblk > 0 ? 1 : 0) + 1;
     if (rec_cap > 0) n += 2 + ((has_phot && neblk > 0) ? 1 : 0);
     return n;
@@ -1161,7 +1176,7 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
     ALLOC(E->chunk_rep, cr.size());
     CUDA_TRY(cudaMemcpy(E->chunk_rep, cr.data(), sizeof(int32_t) * cr.size(), cudaMemcpyHostToDevice));
   }
-  for (int t = 0; t < 3; ++t) {
+  for (int t = 0; t < kTileTables; ++t) {
     std::vector<int2> pt = tiles(pfirst, pcount, kTileSizes[t]);
     E->npblk_bs[t] = (int)pt.size();
     ALLOC(E->pblk_bs[t], std::max<size_t>(1, pt.size()));
