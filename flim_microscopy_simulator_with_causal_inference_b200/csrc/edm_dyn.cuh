@@ -75,10 +75,14 @@ struct DevState {
   int32_t* bind_count;   // [R]
   int64_t* bind_key;     // [R][kBindCap]
   int32_t* bind_ab;      // [R][kBindCap][2] local ids (a = reactant A role, b = B role)
-  // catalytic contacts of the step: (enzyme slot, substrate-capable slot)
+  // catalytic contacts of the step: (enzyme slot, substrate-capable slot),
+  // contact_cap per reaction.  With rep_contacts each replica has its own part
+  // of the reaction's array and its own counts (k_react takes a replica per
+  // block), without it one list per reaction serves all replicas.
   int2* contacts;
-  int32_t* contact_count;  // [EDM_MAX_CAT]
+  int32_t* contact_count;  // [EDM_MAX_CAT], or [R][EDM_MAX_CAT]
   int64_t contact_cap;      // per catalytic reaction
+  int rep_contacts;
   const int64_t* rep_first;  // [R + 1] first slot of each replica
   const int32_t* chunk_rep;  // replica of the first slot of each kSweepChunk-slot chunk
   // slots that left their sort bucket's neighbourhood after the sort this step
@@ -86,10 +90,12 @@ struct DevState {
   int32_t* moved;
   int32_t* moved_count;  // [R]
   // particles whose keyed draws pass some per-particle pass's bound this step:
-  // (slot, bit mask of those passes, replica, local id); pl_index[slot] = its entry
+  // (slot, bit mask of those passes, replica, local id); pl_index[slot] = its
+  // entry.  With rep_pl replica r's entries start at its particle_offset.
   int4* pl;
-  int32_t* pl_count;
+  int32_t* pl_count;  // [1], or [R]
   int32_t* pl_index;
+  int rep_pl;
   // per species: the density grids (bit g) that sense it in some replica
   uint32_t sensor_grids[EDM_MAX_SPECIES];
   // the contact search's sweepers (slot, replica) of this step (k_sweep_list)
@@ -412,10 +418,36 @@ __device__ __forceinline__ double adapt_factor(const EdmDynParams& p, const doub
   return 1.0;
 }
 
-// Add d to every grid counting species sp, at (x, y) — into `arr`.
-__device__ __forceinline__ void grid_add(const EdmDynParams& p, int32_t* arr, int sp, double x, double y, int d) {
+// Where a pass's grid changes go until the merge before the next pass that
+// reads the grids: an array of pending changes per cell ...
+struct DeltaArray {
+  int32_t* delta;
+  __device__ __forceinline__ void add(int64_t cell, int d) const { atomicAdd(&delta[cell], d); }
+};
+// ... or, for a block that has the replica to itself, a short list in shared
+// memory (the array takes what finds it full).
+constexpr int kDeltaList = 512;
+struct DeltaList {
+  int64_t* cell;
+  int* d;
+  int* n;
+  int32_t* delta;
+  __device__ __forceinline__ void add(int64_t c, int change) const {
+    const int k = atomicAdd(n, 1);
+    if (k < kDeltaList) {
+      cell[k] = c;
+      d[k] = change;
+    } else {
+      atomicAdd(&delta[c], change);
+    }
+  }
+};
+
+// Add d to every grid counting species sp, at (x, y).
+template <typename Sink>
+__device__ __forceinline__ void grid_add(const EdmDynParams& p, const Sink& sink, int sp, double x, double y, int d) {
   for (int g = 0; g < p.n_grids; ++g) {
-    if (p.grid[g].sensor == sp) atomicAdd(&arr[grid_cell_of(p.grid[g], x, y)], d);
+    if (p.grid[g].sensor == sp) sink.add(grid_cell_of(p.grid[g], x, y), d);
   }
 }
 
@@ -427,10 +459,11 @@ __device__ __forceinline__ double rule_factor(const EdmDynParams& p, int rule, c
 }
 
 // Grid bookkeeping of a particle changing (species, alive) at one position.
-__device__ __forceinline__ void grid_change(const EdmDynParams& p, int32_t* delta, int sp_old, bool alive_old,
+template <typename Sink>
+__device__ __forceinline__ void grid_change(const EdmDynParams& p, const Sink& sink, int sp_old, bool alive_old,
                                             int sp_new, bool alive_new, double x, double y) {
-  if (alive_old) grid_add(p, delta, sp_old, x, y, -1);
-  if (alive_new) grid_add(p, delta, sp_new, x, y, +1);
+  if (alive_old) grid_add(p, sink, sp_old, x, y, -1);
+  if (alive_new) grid_add(p, sink, sp_new, x, y, +1);
 }
 
 // Record a slot placed away from its sort bucket after this step's sort.
@@ -1129,6 +1162,31 @@ __device__ __forceinline__ void gather_matching(const DevState& st, const Match&
   for (; hits; hits &= hits - 1) list[at++] = (int32_t)(s0 + (__ffs(hits) - 1) * BLK + threadIdx.x);
 }
 
+// Where replica r's listed contacts go.
+constexpr int kRepContactsExtra = 4096;  // per replica, beyond 4 per particle
+struct ContactOut {
+  int2* list;      // reaction c's part starts at list + c * stride
+  int64_t stride;
+  int64_t cap;
+  int32_t* count;  // [EDM_MAX_CAT]
+  uint32_t* status;
+  __device__ __forceinline__ void file(int c, int e, int sub) const {
+    const int q = atomicAdd(&count[c], 1);
+    if (q < cap) list[(int64_t)c * stride + q] = make_int2(e, sub);
+    else set_status(status, EDM_STATUS_CONTACT_CAP);
+  }
+};
+__device__ __forceinline__ ContactOut contact_out(const DevState& st, const EdmDynParams& p, int r) {
+  ContactOut o{st.contacts, st.contact_cap, st.contact_cap, st.contact_count, st.status};
+  if (st.rep_contacts) {
+    const int64_t off = 4 * p.particle_offset + (int64_t)kRepContactsExtra * r;
+    o.list += off;
+    o.cap = r + 1 < st.n_rep ? 4 * p.n_particles + kRepContactsExtra : st.contact_cap - off;
+    o.count += (int64_t)r * EDM_MAX_CAT;
+  }
+  return o;
+}
+
 // A warp's pairs (sweeper, neighbour, replica) that passed the pre-move test
 // of the sweep.  About one neighbour in six does, so the rest of the work
 // (post-move contact, keyed draw, listing) is done 32 pairs at a time with
@@ -1160,10 +1218,8 @@ __device__ __forceinline__ void finish_contacts(const EdmDynParams* __restrict__
     const int c = __ffs(bits) - 1;
     if (d2 > p.cat[c].contact_sq) continue;
     if (!cat_draw_passes(p, st, r, c, ids, idj, *st.d_step)) continue;
-    const int q = atomicAdd(&st.contact_count[c], 1);
-    if (q < st.contact_cap)
-      st.contacts[(int64_t)c * st.contact_cap + q] = (L.from_enzyme >> c) & 1u ? sj : make_int2(sj.y, sj.x);
-    else set_status(st.status, EDM_STATUS_CONTACT_CAP);
+    const bool from_enzyme = (L.from_enzyme >> c) & 1u;
+    contact_out(st, p, r).file(c, from_enzyme ? sj.x : sj.y, from_enzyme ? sj.y : sj.x);
   }
 }
 
@@ -1329,7 +1385,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynPara
 // expressions), appended to the reactions' lists.
 template <bool F64>
 __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
-                                           int64_t j, int id_j, int64_t step, uint32_t late) {
+                                           int64_t j, int id_j, int64_t step, uint32_t late,
+                                           const ContactOut& out) {
   uint32_t emask = 0;
   for (uint32_t b = late; b; b &= b - 1) emask |= 1u << p.cat[__ffs(b) - 1].enzyme;
   for_neighbour_slots(g, st, st.cell_pre[j], [&](int e, int, int dcx, int dcy) {
@@ -1352,9 +1409,7 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
       const int c = __ffs(b) - 1;
       if (spe != p.cat[c].enzyme || d2 > p.cat[c].contact_sq) continue;
       if (!cat_draw_passes(p, st, r, c, st.ids[e] - (int)g.poff, id_j, step)) continue;
-      const int q = atomicAdd(&st.contact_count[c], 1);
-      if (q < st.contact_cap) st.contacts[(int64_t)c * st.contact_cap + q] = make_int2(e, (int)j);
-      else set_status(st.status, EDM_STATUS_CONTACT_CAP);
+      out.file(c, e, (int)j);
     }
   });
 }
@@ -1365,6 +1420,31 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
 // radius and has its draw below the pass's threshold; the partner's current
 // species and the exact probability are left to test.
 // `late`: the later reactions whose substrate is this pass's product.
+template <bool F64, typename Sink>
+__device__ __forceinline__ void catalytic_pair(const EdmDynParams& p, const DevState& st, int r, int cidx,
+                                               uint32_t late, int2 es, const Sink& sink, const ContactOut& out) {
+  const uint8_t fs = st.flags[es.y];
+  const EdmCat& C = p.cat[cidx];
+  if (!fl_alive(fs) || fl_species(fs) != C.substrate) return;
+  const Geo g(p);
+  const int ide = st.ids[es.x] - g.poff, ids = st.ids[es.y] - g.poff;
+  const uint32_t lo = ide < ids ? ide : ids, hi = ide < ids ? ids : ide;
+  const uint64_t m = draw_u53(p.seed, *st.d_step, EDM_S_CAT + cidx, lo, hi);
+  if (m >= st.cat_thr[(int64_t)r * EDM_MAX_CAT + cidx]) return;
+  const double u = __dmul_rn(__ull2double_rn(m), 0x1p-53);
+  double xs, ys;
+  abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, es.y, g, xs, ys);
+  double peff = C.prob;
+  if (C.rule >= 0) peff = C.prob * rule_factor(p, C.rule, st, xs, ys);
+  if (C.rule >= 0 && ((p.adapt_cat_mask >> cidx) & 1)) peff = peff * adapt_factor(p, st.adapt_w, C.rule, xs, ys);
+  if (u < peff && cas_u8(&st.flags[es.y], fs, fl_make(C.product, true))) {
+    atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_CATALYTIC], 1);
+    grid_change(p, sink, C.substrate, true, C.product, true, xs, ys);
+    if (late) late_contacts<F64>(p, g, st, r, es.y, ids, *st.d_step, late, out);
+  }
+}
+
+// One pass over one list for all replicas, for systems whose lists are long.
 template <bool F64>
 __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __restrict__ P, DevState st, int cidx,
                                                        uint32_t late) {
@@ -1374,30 +1454,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __r
   const int2* list = st.contacts + (int64_t)cidx * st.contact_cap;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < lim; q += (int64_t)gridDim.x * blockDim.x) {
     const int2 es = list[q];
-    const uint8_t fs = st.flags[es.y];
     int r = st.chunk_rep[es.x / kSweepChunk];
     while (r + 1 < st.n_rep && st.rep_first[r + 1] <= es.x) ++r;
-    const EdmDynParams& p = P[r];
-    const EdmCat& C = p.cat[cidx];
-    if (!fl_alive(fs) || fl_species(fs) != C.substrate) continue;
-    const Geo g(p);
-    const int ide = st.ids[es.x] - (int)g.poff, ids = st.ids[es.y] - (int)g.poff;
-    const uint32_t lo = ide < ids ? ide : ids, hi = ide < ids ? ids : ide;
-    const uint64_t m = draw_u53(p.seed, *st.d_step, EDM_S_CAT + cidx, lo, hi);
-    if (m >= st.cat_thr[(int64_t)r * EDM_MAX_CAT + cidx]) continue;
-    const double u = __dmul_rn(__ull2double_rn(m), 0x1p-53);
-    double xs, ys;
-    abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, es.y, g, xs, ys);
-    double peff = C.prob;
-    if (C.rule >= 0) peff = C.prob * rule_factor(p, C.rule, st, xs, ys);
-    if (C.rule >= 0 && ((p.adapt_cat_mask >> cidx) & 1)) peff = peff * adapt_factor(p, st.adapt_w, C.rule, xs, ys);
-    if (u < peff) {
-      if (cas_u8(&st.flags[es.y], fs, fl_make(C.product, true))) {
-        atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_CATALYTIC], 1);
-        grid_change(p, st.grid_delta, C.substrate, true, C.product, true, xs, ys);
-        if (late) late_contacts<F64>(p, g, st, r, es.y, ids, *st.d_step, late);
-      }
-    }
+    catalytic_pair<F64>(P[r], st, r, cidx, late, es, DeltaArray{st.grid_delta}, contact_out(st, P[r], r));
   }
 }
 
@@ -1449,17 +1508,49 @@ __global__ void __launch_bounds__(kBlock, 8) k_pass_draws(const EdmDynParams* __
     const int id = st.ids[s] - (int)P[r].particle_offset;
     const uint32_t bits = draw_passes(st, D, P[r].seed, r, id, *st.d_step, todo);
     if (bits) {
-      const int q = atomicAdd(st.pl_count, 1);
+      const int q = st.rep_pl ? (int)P[r].particle_offset + atomicAdd(&st.pl_count[r], 1) : atomicAdd(st.pl_count, 1);
       st.pl[q] = make_int4((int)s, (int)bits, r, id);
       st.pl_index[s] = q;
     }
   });
 }
 
-// Apply the first max_recruits accepted candidates in particle order.
-// A recruited particle is alive from here on, so the passes after this one
-// that match it (`after`) get its draws now, in its list entry (the entry
+// Puts particle `id` of replica r, recruited by exchange e, at (x, y).  It is
+// alive from here on, so the passes after this one that match it (`after`) get
+// their draws now, in its list entry (entry(q) = entry q of the list; it
 // exists: the particle was listed for this exchange's candidates).
+template <bool F64, typename Sink, typename Entry>
+__device__ __forceinline__ void place_recruit(const EdmDynParams& p, const Geo& g, const DevState& st, int r, int e,
+                                              int id, double x, double y, const Sink& sink,
+                                              const DrawPlan* __restrict__ D, uint32_t after, Entry entry) {
+  const EdmExch& X = p.exch[e];
+  const int64_t slot = st.slot_of_id[g.poff + id];
+  const int cxn = cell_index(x, g.sx, g.nx), cyn = cell_index(y, g.sy, g.ny);
+  const int newc = cxn * g.ny + cyn;
+  if constexpr (F64) {
+    ((double2*)st.pos_post)[slot] = make_double2(x, y);
+  } else {
+    float2 o;
+    short2 l;
+    split_offset(x - (double)cxn * g.sx, g.sxf, o.x, l.x);
+    split_offset(y - (double)cyn * g.sy, g.syf, o.y, l.y);
+    ((float2*)st.pos_post)[slot] = o;
+    st.lo_post[slot] = l;
+  }
+  st.cell_post[slot] = newc;
+  rebucket(st, g, g.grave, newc);
+  st.flags[slot] = fl_make(X.species, true);
+  note_moved(st, r, p, slot);
+  grid_add(p, sink, X.species, x, y, 1);
+  if (after) {
+    const uint32_t bits = draw_passes(st, D, p.seed, r, id, *st.d_step, after);
+    int4* q = entry(st.pl_index[slot]);
+    if (q && q->x == (int)slot) q->y |= (int)bits;
+    else set_status(st.status, EDM_STATUS_RECRUIT_CAP);  // cannot happen: see above
+  }
+}
+
+// Apply the first max_recruits accepted candidates in particle order.
 template <bool F64>
 __global__ void k_recruit_apply(const EdmDynParams* __restrict__ P, int n_rep, DevState st, int e,
                                 const DrawPlan* __restrict__ D,
@@ -1491,40 +1582,24 @@ __global__ void k_recruit_apply(const EdmDynParams* __restrict__ P, int n_rep, D
   }
   const Geo g(p);
   const int take = n < X.max_recruits ? n : X.max_recruits;
-  for (int a = 0; a < take; ++a) {
-    const int64_t slot = st.slot_of_id[g.poff + ids[a]];
-    const double x = xy[2 * a], y = xy[2 * a + 1];
-    const int cxn = cell_index(x, g.sx, g.nx), cyn = cell_index(y, g.sy, g.ny);
-    const int newc = cxn * g.ny + cyn;
-    if constexpr (F64) {
-      ((double2*)st.pos_post)[slot] = make_double2(x, y);
-    } else {
-      float2 o;
-      short2 l;
-      split_offset(x - (double)cxn * g.sx, g.sxf, o.x, l.x);
-      split_offset(y - (double)cyn * g.sy, g.syf, o.y, l.y);
-      ((float2*)st.pos_post)[slot] = o;
-      st.lo_post[slot] = l;
-    }
-    st.cell_post[slot] = newc;
-    rebucket(st, g, g.grave, newc);
-    st.flags[slot] = fl_make(X.species, true);
-    note_moved(st, r, p, slot);
-    grid_add(p, st.grid_delta, X.species, x, y, 1);
-    if (after) {
-      const uint32_t bits = draw_passes(st, D, p.seed, r, ids[a], *st.d_step, after);
-      const int q = st.pl_index[slot];
-      if (q >= 0 && q < *st.pl_count && st.pl[q].x == (int)slot) st.pl[q].y |= (int)bits;
-      else set_status(st.status, EDM_STATUS_RECRUIT_CAP);  // cannot happen: see above
-    }
-  }
+  for (int a = 0; a < take; ++a)
+    place_recruit<F64>(p, g, st, r, e, ids[a], xy[2 * a], xy[2 * a + 1], DeltaArray{st.grid_delta}, D, after,
+                       [&](int q) { return q >= 0 && q < *st.pl_count ? st.pl + q : (int4*)nullptr; });
   atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_RECRUITED], take);
 }
+
+// Candidates of one replica's recruitment: [kRecCap] ids and positions.
+struct RecruitList {
+  int32_t* count;
+  int32_t* id;
+  double* xy;
+};
 
 // Recruitment candidate of exchange e (dynamics.py:1229-1458): a dormant
 // particle of the species whose keyed draw accepts at the keyed position.
 // The per-particle passes below run on listed particles only.
-__device__ __forceinline__ void recruit_candidate(const EdmDynParams& p, const DevState& st, int r, int id, int e) {
+__device__ __forceinline__ void recruit_candidate(const EdmDynParams& p, const DevState& st, const RecruitList& out,
+                                                  int id, int e) {
   const EdmExch& X = p.exch[e];
   const int64_t step = *st.d_step;
   const double ua = uniform1(p.seed, step, EDM_S_EX_ACCEPT + 4 * e, (uint64_t)id, 0);
@@ -1555,11 +1630,11 @@ __device__ __forceinline__ void recruit_candidate(const EdmDynParams& p, const D
     peff = X.prob_on * rule_factor(p, X.rule_on, st, cx, cy);
   }
   if (ua < peff) {
-    const int k = atomicAdd(&st.rec_count[r], 1);
+    const int k = atomicAdd(out.count, 1);
     if (k < kRecCap) {
-      st.rec_id[(int64_t)r * kRecCap + k] = id;
-      st.rec_xy[((int64_t)r * kRecCap + k) * 2] = cx;
-      st.rec_xy[((int64_t)r * kRecCap + k) * 2 + 1] = cy;
+      out.id[k] = id;
+      out.xy[2 * k] = cx;
+      out.xy[2 * k + 1] = cy;
     } else {
       set_status(st.status, EDM_STATUS_RECRUIT_CAP);
     }
@@ -1579,9 +1654,10 @@ struct LazyPos {
 
 // Detachment of exchange e (dynamics.py:1461-1555) of the alive particle in
 // slot s; returns its flags afterwards.
-template <bool F64>
+template <bool F64, typename Sink>
 __device__ __forceinline__ uint8_t detach_one(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
-                                              int64_t s, int id, LazyPos<F64>& pos, int e, uint8_t f) {
+                                              int64_t s, int id, LazyPos<F64>& pos, int e, uint8_t f,
+                                              const Sink& sink) {
   const EdmExch& X = p.exch[e];
   const double u = uniform1(p.seed, *st.d_step, EDM_S_EX_DETACH + 4 * e, (uint64_t)id, 0);
   pos.get(st, s, g);
@@ -1592,16 +1668,17 @@ __device__ __forceinline__ uint8_t detach_one(const EdmDynParams& p, const Geo& 
     st.flags[s] = f;
     rebucket(st, g, st.cell_post[s], g.grave);
     atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_DETACHED], 1);
-    grid_add(p, st.grid_delta, X.species, pos.x, pos.y, -1);
+    grid_add(p, sink, X.species, pos.x, pos.y, -1);
   }
   return f;
 }
 
 // Unimolecular conversion v (dynamics.py:1565-1657) of the alive particle in
 // slot s; returns its flags afterwards.
-template <bool F64>
+template <bool F64, typename Sink>
 __device__ __forceinline__ uint8_t convert_one(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
-                                               int64_t s, int id, LazyPos<F64>& pos, int v, uint8_t f) {
+                                               int64_t s, int id, LazyPos<F64>& pos, int v, uint8_t f,
+                                               const Sink& sink) {
   const EdmConv& V = p.conv[v];
   const double u = uniform1(p.seed, *st.d_step, EDM_S_CONV + v, (uint64_t)id, 0);
   pos.get(st, s, g);
@@ -1611,7 +1688,7 @@ __device__ __forceinline__ uint8_t convert_one(const EdmDynParams& p, const Geo&
     f = fl_make(V.to, true);
     st.flags[s] = f;
     atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_CONVERTED], 1);
-    grid_change(p, st.grid_delta, V.from, true, V.to, true, pos.x, pos.y);
+    grid_change(p, sink, V.from, true, V.to, true, pos.x, pos.y);
   }
   return f;
 }
@@ -1632,38 +1709,46 @@ struct PassGroup {
   int n;
 };
 
+// Takes the particle of list entry e through the run's passes; returns the
+// entry's pass bits afterwards (a state change adds those of later passes).
+template <bool F64, typename Sink>
+__device__ __forceinline__ uint32_t run_passes(const EdmDynParams& p, const DevState& st, const PassGroup& sg,
+                                               const DrawPlan* __restrict__ D, int4 e, const RecruitList& rec,
+                                               const Sink& sink) {
+  uint32_t bits = (uint32_t)e.y;
+  if (!(bits & sg.bits)) return bits;
+  const int64_t s = e.x;
+  const int r = e.z, id = e.w;
+  const Geo g(p);
+  uint8_t f = st.flags[s];
+  LazyPos<F64> pos;  // these passes move no particle
+  for (int k = 0; k < sg.n; ++k) {
+    const int pk = sg.pp[k];
+    if (!((bits >> pk) & 1u) || !matches(f, sg.m[k])) continue;
+    const int kind = sg.kind[k], idx = sg.index[k];
+    if (kind == kGroupRecruit) {
+      recruit_candidate(p, st, rec, id, idx);
+      continue;
+    }
+    const uint8_t f0 = f;
+    f = kind == kGroupDetach ? detach_one<F64>(p, g, st, r, s, id, pos, idx, f, sink)
+                             : convert_one<F64>(p, g, st, r, s, id, pos, idx, f, sink);
+    if (f != f0) bits |= draw_passes(st, D, p.seed, r, id, *st.d_step, D->after[pk] & ~bits);
+  }
+  return bits;
+}
+
 template <bool F64>
 __global__ void __launch_bounds__(kBlock) k_particle_passes(const EdmDynParams* __restrict__ P, DevState st,
                                                             const PassGroup* __restrict__ G,
                                                             const DrawPlan* __restrict__ D) {
   pdl_enter();
-  const PassGroup& sg = *G;
   const int n = *st.pl_count;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int4 e = st.pl[q];
-    uint32_t bits = (uint32_t)e.y;
-    if (!(bits & sg.bits)) continue;
-    const int64_t s = e.x;
-    const int r = e.z, id = e.w;
-    const EdmDynParams& p = P[r];
-    const Geo g(p);
-    uint8_t f = st.flags[s];
-    const uint32_t bits0 = bits;
-    LazyPos<F64> pos;  // these passes move no particle
-    for (int k = 0; k < sg.n; ++k) {
-      const int pk = sg.pp[k];
-      if (!((bits >> pk) & 1u) || !matches(f, sg.m[k])) continue;
-      const int kind = sg.kind[k], idx = sg.index[k];
-      if (kind == kGroupRecruit) {
-        recruit_candidate(p, st, r, id, idx);
-        continue;
-      }
-      const uint8_t f0 = f;
-      f = kind == kGroupDetach ? detach_one<F64>(p, g, st, r, s, id, pos, idx, f)
-                               : convert_one<F64>(p, g, st, r, s, id, pos, idx, f);
-      if (f != f0) bits |= draw_passes(st, D, p.seed, r, id, *st.d_step, D->after[pk] & ~bits);
-    }
-    if (bits != bits0) st.pl[q].y = (int)bits;
+    const RecruitList rec{st.rec_count + e.z, st.rec_id + (int64_t)e.z * kRecCap, st.rec_xy + (int64_t)e.z * kRecCap * 2};
+    const uint32_t bits = run_passes<F64>(P[e.z], st, *G, D, e, rec, DeltaArray{st.grid_delta});
+    if (bits != (uint32_t)e.y) st.pl[q].y = (int)bits;
   }
 }
 
@@ -1763,8 +1848,8 @@ __global__ void k_bind_apply(const EdmDynParams* __restrict__ P, int n_rep, DevS
     rebucket(st, g, st.cell_post[sb], g.grave);
     st.bond[g.poff + a] = (int32_t)(g.poff + bb);
     st.bond[g.poff + bb] = (int32_t)(g.poff + a);
-    grid_change(p, st.grid_delta, B.ra, true, B.product, true, xa, ya);
-    grid_change(p, st.grid_delta, B.rb, true, B.rb, false, xb, yb);
+    grid_change(p, DeltaArray{st.grid_delta}, B.ra, true, B.product, true, xa, ya);
+    grid_change(p, DeltaArray{st.grid_delta}, B.rb, true, B.rb, false, xb, yb);
     ++nb;
   }
   atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_BINDINGS], nb);
@@ -1802,8 +1887,8 @@ __global__ void __launch_bounds__(kBlock) k_dissociate(const EdmDynParams* __res
     note_moved(st, r, p, sj);
     st.bond[g.poff + id] = -1;
     st.bond[partner] = -1;
-    grid_change(p, st.grid_delta, B.product, true, B.ra, true, x, y);
-    grid_change(p, st.grid_delta, fl_species(fj), fl_alive(fj), B.rb, true, x, y);
+    grid_change(p, DeltaArray{st.grid_delta}, B.product, true, B.ra, true, x, y);
+    grid_change(p, DeltaArray{st.grid_delta}, fl_species(fj), fl_alive(fj), B.rb, true, x, y);
     atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_DISSOC], 1);
   });
 }
@@ -1825,38 +1910,53 @@ __global__ void k_adapt(const EdmDynParams* __restrict__ P, const int32_t* __res
   }
 }
 
-// Local-recruitment CDF of exchange e for each replica (block = replica):
+// Local-recruitment CDF of exchange e of one replica, by one block:
 // cumulative max(density, 0.01) over the feedback grid's cells in (gx, gy)
-// order, sequentially as the reference sums it, then divided by the total
-// (dynamics.py:2356-2371).
-__global__ void k_local_cdf(const EdmDynParams* __restrict__ P, const int32_t* __restrict__ cnt,
-                            double* __restrict__ cdf_all, int e) {
-  pdl_enter();
-  const EdmDynParams& p = P[blockIdx.x];
+// order, summed sequentially as the reference does, then divided by the total
+// (dynamics.py:2356-2371).  One thread adds; the block computes the densities
+// of kCdfTile cells in shared memory before it and writes the sums after it,
+// so the chain is one add per cell (16 us for 900 cells when it went through
+// global memory).
+constexpr int kCdfTile = 512;
+__device__ __forceinline__ void local_cdf_of(const EdmDynParams& p, const int32_t* cnt, double* cdf_all, int e,
+                                             double* tile) {
   const EdmExch& X = p.exch[e];
   if (!X.local_recruit || X.rule_on < 0) return;
   const EdmRule& R = p.rule[X.rule_on];
   const EdmGrid& G = p.grid[R.grid];
   const int n = G.nx * G.ny;
   double* cdf = cdf_all + G.offset;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const double rho = kfold_density(cnt[G.offset + c], R.inv_area);
-    cdf[c] = rho > 0.01 ? rho : 0.01;
-  }
-  __syncthreads();
-  __shared__ double total_s;
-  if (threadIdx.x == 0) {
-    double total = 0.0;
-    for (int c = 0; c < n; ++c) {
-      total = __dadd_rn(total, cdf[c]);
-      cdf[c] = total;
+  double total = 0.0;
+  for (int c0 = 0; c0 < n; c0 += kCdfTile) {
+    const int m = n - c0 < kCdfTile ? n - c0 : kCdfTile;
+    __syncthreads();
+    for (int c = threadIdx.x; c < m; c += blockDim.x) {
+      const double rho = kfold_density(cnt[G.offset + c0 + c], R.inv_area);
+      tile[c] = rho > 0.01 ? rho : 0.01;
     }
-    total_s = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int c = 0; c < m; ++c) {
+        total = __dadd_rn(total, tile[c]);
+        tile[c] = total;
+      }
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < m; c += blockDim.x) cdf[c0 + c] = tile[c];
   }
   __syncthreads();
-  const double total = total_s;
+  if (threadIdx.x == 0) tile[0] = total;
+  __syncthreads();
+  total = tile[0];
   for (int c = threadIdx.x; c < n; c += blockDim.x)
     cdf[c] = total > 0 ? __ddiv_rn(cdf[c], total) : __ddiv_rn((double)c + 1.0, (double)n);
+}
+
+__global__ void k_local_cdf(const EdmDynParams* __restrict__ P, const int32_t* cnt, double* cdf_all, int e) {
+  pdl_enter();
+  __shared__ double tile[kCdfTile];
+  local_cdf_of(P[blockIdx.x], cnt, cdf_all, e, tile);
 }
 
 __global__ void k_grid_merge(int32_t* __restrict__ cnt, int32_t* __restrict__ delta, int64_t n) {
@@ -1866,6 +1966,135 @@ __global__ void k_grid_merge(int32_t* __restrict__ cnt, int32_t* __restrict__ de
     if (d) {
       cnt[i] += d;
       delta[i] = 0;
+    }
+  }
+}
+
+// ---- the passes after the contact search, one block per replica ---------------
+// The catalytic passes, the runs of per-particle passes, the recruitment
+// applies, the local-recruitment CDFs and the grid merges between them touch
+// one replica's data only, and their lists are short (only pairs and
+// particles whose draw lies below the pass's threshold).  So one block takes
+// its replica through all of them with a barrier between two passes instead of
+// a launch: as separate launches each pass cost 2.5 to 7 us however short its
+// list.  The replica's parameters, list entries, counts and grid changes sit in
+// shared memory, which leaves the round trips to the particles themselves.
+constexpr int kReactThreads = 512;
+constexpr int kReactPasses = 48;
+constexpr int kReactGroups = 8;
+constexpr int kReactList = 512;  // list entries held in shared memory
+enum ReactKind : int8_t { kReactCatalytic, kReactGroup, kReactRecruit, kReactCdf, kReactMerge };
+struct ReactPlan {
+  int8_t kind[kReactPasses];
+  int8_t index[kReactPasses];    // reaction, group or exchange
+  uint32_t more[kReactPasses];   // catalytic: later reactions; recruit: later passes
+  int n, n_groups;
+};
+
+template <bool F64>
+__global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __restrict__ P, DevState st,
+                                                       const __grid_constant__ ReactPlan plan,
+                                                       const PassGroup* __restrict__ groups,
+                                                       const DrawPlan* __restrict__ D, int64_t* step,
+                                                       unsigned* ticket) {
+  pdl_enter();
+  static_assert(sizeof(EdmDynParams) % 16 == 0 && sizeof(PassGroup) % 4 == 0, "copied in words");
+  __shared__ __align__(16) uint8_t par[sizeof(EdmDynParams)];
+  __shared__ __align__(16) uint8_t grp[kReactGroups * sizeof(PassGroup)];
+  __shared__ int4 entry[kReactList];
+  __shared__ int64_t delta_cell[kDeltaList];
+  __shared__ int delta_d[kDeltaList];
+  __shared__ double rec_xy[2 * kRecCap];
+  __shared__ double tile[kCdfTile];
+  __shared__ int32_t rec_id[kRecCap], n_contact[EDM_MAX_CAT], n_rec;
+  __shared__ int n_delta;
+  const int r = blockIdx.x, tid = threadIdx.x;
+  for (int k = tid; k < (int)(sizeof(EdmDynParams) / 16); k += blockDim.x)
+    ((uint4*)par)[k] = ((const uint4*)(P + r))[k];
+  for (int k = tid; k < plan.n_groups * (int)(sizeof(PassGroup) / 4); k += blockDim.x)
+    ((uint32_t*)grp)[k] = ((const uint32_t*)groups)[k];
+  if (tid < EDM_MAX_CAT) n_contact[tid] = st.rep_contacts ? st.contact_count[(int64_t)r * EDM_MAX_CAT + tid] : 0;
+  if (tid == 0) n_rec = n_delta = 0;
+  const int n_listed = st.pl_count[r];
+  const int64_t poff = P[r].particle_offset;
+  for (int q = tid; q < n_listed && q < kReactList; q += blockDim.x) entry[q] = st.pl[poff + q];
+  __syncthreads();
+  const EdmDynParams& p = *reinterpret_cast<const EdmDynParams*>(par);
+  const DeltaList sink{delta_cell, delta_d, &n_delta, st.grid_delta};
+  ContactOut out = contact_out(st, p, r);
+  out.count = n_contact;
+  const RecruitList rec{&n_rec, rec_id, rec_xy};
+  auto entry_at = [&](int q) -> int4* {  // entry q of the replica's list
+    return q < kReactList ? entry + q : st.pl + poff + q;
+  };
+  for (int i = 0; i < plan.n; ++i) {
+    const int idx = plan.index[i];
+    switch (plan.kind[i]) {
+      case kReactCatalytic: {
+        const int n = n_contact[idx] < out.cap ? n_contact[idx] : (int)out.cap;
+        for (int q = tid; q < n; q += blockDim.x)
+          catalytic_pair<F64>(p, st, r, idx, plan.more[i], out.list[(int64_t)idx * out.stride + q], sink, out);
+        break;
+      }
+      case kReactGroup: {
+        const PassGroup& sg = reinterpret_cast<const PassGroup*>(grp)[idx];
+        for (int q = tid; q < n_listed; q += blockDim.x) {
+          int4* e = entry_at(q);
+          const int4 v = *e;
+          const uint32_t bits = run_passes<F64>(p, st, sg, D, v, rec, sink);
+          if (bits != (uint32_t)v.y) e->y = (int)bits;
+        }
+        break;
+      }
+      case kReactRecruit: {  // the first max_recruits candidates in particle order
+        const int n = n_rec < kRecCap ? n_rec : kRecCap;
+        if (n == 0) break;
+        const int cap = p.exch[idx].max_recruits, take = n < cap ? n : cap;
+        for (int a = tid; a < n; a += blockDim.x) {
+          const int id = rec_id[a];
+          int rank = 0;
+          for (int b = 0; b < n; ++b) rank += rec_id[b] < id;
+          if (rank < take)
+            place_recruit<F64>(p, Geo(p), st, r, idx, id, rec_xy[2 * a], rec_xy[2 * a + 1], sink, D, plan.more[i],
+                               [&](int q) {
+                                 const int k = q - (int)poff;
+                                 return k >= 0 && k < n_listed ? entry_at(k) : (int4*)nullptr;
+                               });
+        }
+        __syncthreads();
+        if (tid == 0) {
+          n_rec = 0;
+          atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_RECRUITED], take);
+        }
+        break;
+      }
+      case kReactCdf: local_cdf_of(p, st.grid_cnt, st.local_cdf, idx, tile); break;
+      case kReactMerge: {
+        const int n = n_delta;
+        for (int k = tid; k < n && k < kDeltaList; k += blockDim.x) atomicAdd(&st.grid_cnt[delta_cell[k]], delta_d[k]);
+        if (n > kDeltaList && p.n_grids > 0) {  // the changes that found the list full
+          const EdmGrid& last = p.grid[p.n_grids - 1];  // a replica's grids are contiguous
+          for (int64_t at = p.grid[0].offset + tid; at < last.offset + (int64_t)last.nx * last.ny; at += blockDim.x) {
+            const int d = st.grid_delta[at];
+            if (d) {
+              atomicAdd(&st.grid_cnt[at], d);
+              st.grid_delta[at] = 0;
+            }
+          }
+        }
+        __syncthreads();
+        if (tid == 0) n_delta = 0;
+        break;
+      }
+    }
+    __syncthreads();
+  }
+  // the last block to finish moves the step index on
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+      *ticket = 0;
+      *step += 1;
     }
   }
 }

@@ -42,7 +42,7 @@ int fail(int code, const std::string& msg) { return edm::report_error(code, msg)
   } while (0)
 
 enum PassKind { P_BIND_CAND, P_BIND_APPLY, P_DISSOC, P_CONTACTS, P_CAT, P_REC_CAND, P_REC_APPLY, P_DETACH, P_CONV, P_MERGE,
-                P_GROUP, P_DRAWS, P_ADAPT, P_LOCAL_CDF };
+                P_GROUP, P_DRAWS, P_ADAPT, P_LOCAL_CDF, P_REACT };
 struct Pass {
   PassKind kind;
   int index;
@@ -97,6 +97,15 @@ int tile_index(int bs) {
   while (kTileSizes[t] < bs) ++t;
   return t;
 }
+
+// Expected list entries of a replica up to which k_react takes its passes.
+// Per BD step of one replica, k_react against the launches: 41 / 62 us at 1,800
+// expected entries, 64 / 422 at 36,000, 253 / 916 at 573,000, 1,059 / 917 at
+// 2.1 million (5,000 to 430,000 particles with raised rates).
+constexpr double kReactEntries = 1.0e6;
+// With several replicas each has its own part of a reaction's contact list, so
+// the listed share of the contacts is kept small as well.
+constexpr double kReactContactShare = 1.0 / 16.0;
 
 // Choices of earlier tunings in this process, by (kernel, precision,
 // replicas, log2 of the slot count): later engines of the same kind reuse them.
@@ -171,6 +180,11 @@ struct EdmEngine {
   DrawPlan* d_draw = nullptr;     // device copies of the plan and the runs
   PassGroup* d_groups = nullptr;
   uint32_t rec_after[EDM_MAX_EXCH] = {};  // per recruitment apply: later passes matching a recruit
+  std::vector<uint64_t> pass_thr_host, cat_thr_host;
+  ReactPlan react{};  // the passes of P_REACT (k_react)
+  int react_threads = 0;
+  bool rep_contacts = false, rep_pl = false;
+  unsigned* react_ticket = nullptr;
   int2* contacts = nullptr;
   int32_t* contact_count = nullptr;
   int64_t contact_cap = 0;
@@ -233,6 +247,7 @@ struct EdmEngine {
     s.contacts = contacts;
     s.contact_count = contact_count;
     s.contact_cap = contact_cap;
+    s.rep_contacts = rep_contacts;
     s.rep_first = rep_first;
     s.chunk_rep = chunk_rep;
     s.moved = moved;
@@ -240,6 +255,7 @@ struct EdmEngine {
     s.pl = pl;
     s.pl_count = pl_count;
     s.pl_index = pl_index;
+    s.rep_pl = rep_pl;
     for (int sp = 0; sp < EDM_MAX_SPECIES; ++sp) s.sensor_grids[sp] = sensor_grids[sp];
     s.sw_list = sw_list;
     s.sw_count = sw_count;
@@ -540,6 +556,8 @@ struct EdmEngine {
         ct[(size_t)r * EDM_MAX_CAT + c] = thr_of(C.rule >= 0 ? C.prob * rm[C.rule] : C.prob);
       }
     }
+    pass_thr_host = pt;
+    cat_thr_host = ct;
     CUDA_TRY(cudaMemcpy(pass_thr, pt.data(), sizeof(uint64_t) * pt.size(), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(cat_thr, ct.data(), sizeof(uint64_t) * ct.size(), cudaMemcpyHostToDevice));
     int rc;
@@ -549,6 +567,67 @@ struct EdmEngine {
     if (!groups.empty())
       CUDA_TRY(cudaMemcpy(d_groups, groups.data(), sizeof(PassGroup) * groups.size(), cudaMemcpyHostToDevice));
     return EDM_OK;
+  }
+
+  // Hands the passes after the contact search and the draw sweep to k_react,
+  // one block per replica, unless a replica's lists are so long that they want
+  // the whole chip: the bound on its expected entries is its particles times
+  // the passes' largest probabilities, plus four contacts per particle times
+  // the catalytic ones.
+  int plan_react() {
+    size_t start = passes.size();
+    auto fusable = [](PassKind k) {
+      return k == P_CAT || k == P_MERGE || k == P_GROUP || k == P_REC_APPLY || k == P_LOCAL_CDF;
+    };
+    while (start > 0 && fusable(passes[start - 1].kind)) --start;
+    bool pending = hdp[0].n_bind > 0;  // grid changes of passes before the region, in grid_delta
+    for (size_t i = 0; i < start; ++i) pending |= passes[i].kind == P_CAT;
+    if (pending && start < passes.size() && passes[start].kind == P_MERGE) ++start;
+    const size_t n = passes.size() - start;
+    if (n == 0 || n > (size_t)kReactPasses || groups.size() > (size_t)kReactGroups) return EDM_OK;
+    double most = 0.0;
+    for (int r = 0; r < R; ++r) {
+      double e = 0.0;
+      for (int k = 0; k < draw.n; ++k) e += std::ldexp((double)pass_thr_host[(size_t)r * kMaxPP + k], -53);
+      for (int c = 0; c < hdp[r].n_cat; ++c) e += 4.0 * std::ldexp((double)cat_thr_host[(size_t)r * EDM_MAX_CAT + c], -53);
+      most = std::max(most, e * (double)hdp[r].n_particles);
+    }
+    if (most > kReactEntries) return EDM_OK;
+    for (uint64_t t : cat_thr_host)
+      if (R > 1 && std::ldexp((double)t, -53) > kReactContactShare) return EDM_OK;
+    bool merges = false, cats = false;
+    for (size_t i = start; i < passes.size(); ++i) {
+      const Pass& ps = passes[i];
+      const int k = react.n++;
+      react.index[k] = (int8_t)ps.index;
+      react.more[k] = 0;
+      switch (ps.kind) {
+        case P_CAT:
+          react.kind[k] = kReactCatalytic;
+          react.more[k] = cat_late[ps.index];
+          cats = true;
+          break;
+        case P_GROUP: react.kind[k] = kReactGroup; break;
+        case P_REC_APPLY:
+          react.kind[k] = kReactRecruit;
+          react.more[k] = rec_after[ps.index];
+          break;
+        case P_LOCAL_CDF: react.kind[k] = kReactCdf; break;
+        default:
+          react.kind[k] = kReactMerge;
+          merges = true;
+          break;
+      }
+    }
+    react.n_groups = (int)groups.size();
+    rep_contacts = cats;
+    rep_pl = true;
+    react_threads = std::min(kReactThreads, std::max(128, ((int)(2.0 * most) + 31) / 32 * 32));
+    passes.resize(start);
+    // the block merges its own passes' grid changes only
+    if (pending && merges && (start == 0 || passes.back().kind != P_MERGE)) passes.push_back({P_MERGE, 0, Match{}});
+    passes.push_back({P_REACT, 0, Match{}});
+    return alloc(&react_ticket, 1);
   }
 
   // optional CUDA events between kernel groups and between reaction passes (profiling only)
@@ -668,8 +747,8 @@ struct EdmEngine {
     z.p[0] = grid_cnt, z.n[0] = grid_cnt ? n_grid : 0;
     z.p[1] = grid_delta, z.n[1] = grid_delta ? n_grid : 0;
     z.p[2] = moved_count, z.n[2] = R;
-    z.p[3] = contact_count, z.n[3] = contact_count ? EDM_MAX_CAT : 0;
-    z.p[4] = pl_count, z.n[4] = pl_count ? 1 : 0;
+    z.p[3] = contact_count, z.n[3] = contact_count ? (rep_contacts ? R : 1) * EDM_MAX_CAT : 0;
+    z.p[4] = pl_count, z.n[4] = pl_count ? R : 0;
     z.p[5] = sw_count, z.n[5] = sw_count ? 1 : 0;
     k_scan_reduce<<<nbs, kScanThreads, 0, s>>>(cnt, n_cells, bsum, z);  // starts the chain
     pdl_chain = true;
@@ -740,17 +819,25 @@ struct EdmEngine {
         case P_REC_CAND:
         case P_DETACH:
         case P_CONV: break;  // fused into P_GROUP passes
+        case P_REACT:
+          if (!joined) {
+            cudaStreamWaitEvent(s, ev_join, 0);
+            joined = true;
+            pdl_chain = false;
+          }
+          go(k_react<F64>, R, react_threads, s, dp, st, react, d_groups, d_draw, d_step, react_ticket);
+          break;
         case P_MERGE: go(k_grid_merge, gm > 0 ? gm : 1, 256, s, grid_cnt, grid_delta, n_grid); break;
       }
     }
     if (pass_prof) cudaEventRecord(pass_prof[passes.size()], s);
-    go(k_step_inc, 1, 1, s, d_step);
+    if (!react_ticket) go(k_step_inc, 1, 1, s, d_step);  // k_react does it
     cells_valid = true;
     mark(4, s);
   }
 
   int launches_per_step(bool with_photons) const {
-    int n = 3 + 1 + 1 + (int)passes.size() + 1;
+    int n = 3 + 1 + 1 + (int)passes.size() + (react_ticket ? 0 : 1);
     for (const Pass& ps : passes)  // the sweeper-list contact shapes launch two kernels
       if (ps.kind == P_CONTACTS && kContactSlots[shape[TK_CONTACTS]] == 0) ++n;
     if (with_photons) n += (neblk > 0 ? 3 : 1) + 1 + (nphblk > 0 ? 1 : 0) + 1;
@@ -1125,7 +1212,8 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   for (const EdmDynParams& q : E->hdp)
     for (int g = 0; g < q.n_grids && g < EDM_MAX_GRIDS; ++g)
       if (q.grid[g].sensor >= 0 && q.grid[g].sensor < EDM_MAX_SPECIES) E->sensor_grids[q.grid[g].sensor] |= 1u << g;
-  if ((rc = E->build_schedule()) != EDM_OK || (rc = E->upload_thresholds()) != EDM_OK) {
+  if ((rc = E->build_schedule()) != EDM_OK || (rc = E->upload_thresholds()) != EDM_OK ||
+      (rc = E->plan_react()) != EDM_OK) {
     delete E;
     return rc;
   }
@@ -1147,20 +1235,19 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
     CUDA_TRY(cudaEventCreateWithFlags(&E->ev_fork, cudaEventDisableTiming));
     CUDA_TRY(cudaEventCreateWithFlags(&E->ev_join, cudaEventDisableTiming));
   }
-  E->contact_cap = std::max<int64_t>(4 * np, 1 << 20);  // per catalytic reaction
+  E->contact_cap = std::max<int64_t>(4 * np + (int64_t)kRepContactsExtra * n_replicas, 1 << 20);  // per reaction
   ALLOC(E->contacts, (size_t)E->contact_cap * std::max(1, E->hdp[0].n_cat));
-  ALLOC(E->contact_count, EDM_MAX_CAT);
+  ALLOC(E->contact_count, (size_t)n_replicas * EDM_MAX_CAT);
   ALLOC(E->moved, np);
   ALLOC(E->moved_count, (size_t)n_replicas);
   ALLOC(E->pl, (size_t)np);
-  ALLOC(E->pl_count, 1);
+  ALLOC(E->pl_count, (size_t)n_replicas);
   ALLOC(E->pl_index, (size_t)np);
   ALLOC(E->sw_list, (size_t)np);
   ALLOC(E->sw_count, 1);
   ALLOC(E->adapt_w, (size_t)std::max<int64_t>(ng, 1));
   ALLOC(E->local_cdf, (size_t)std::max<int64_t>(ng, 1));
   CUDA_TRY(cudaMemset(E->pl_index, 0xFF, sizeof(int32_t) * np));
-  CUDA_TRY(cudaMemset(E->pl_count, 0, sizeof(int32_t)));
   ALLOC(E->rep_first, (size_t)n_replicas + 1);
   {
     std::vector<int64_t> rf(pfirst);

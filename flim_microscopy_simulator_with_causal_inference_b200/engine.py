@@ -293,7 +293,7 @@ class Engine:
 
     PASS_KINDS = ("bind_candidates", "bind_apply", "dissociation", "contacts", "catalytic", "recruit_candidates",
                   "recruit_apply", "detach", "convert", "grid_merge", "particle_passes", "pass_draws",
-                  "adaptation", "local_cdf")
+                  "adaptation", "local_cdf", "react")
 
     def profile_passes(self, n: int, stream=None) -> list:
         """Mean device ms per dynamics step of each reaction pass, in schedule
