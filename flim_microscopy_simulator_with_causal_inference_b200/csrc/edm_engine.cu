@@ -750,14 +750,14 @@ struct EdmEngine {
     z.p[3] = contact_count, z.n[3] = contact_count ? (rep_contacts ? R : 1) * EDM_MAX_CAT : 0;
     z.p[4] = pl_count, z.n[4] = pl_count ? R : 0;
     z.p[5] = sw_count, z.n[5] = sw_count ? 1 : 0;
+    // with proximity FRET the previous step's photon pass reads the bucket
+    // starts and the list of particles placed after the sort, cleared here
+    if (phot_uses_cells) join_photons(s);
     k_scan_reduce<<<nbs, kScanThreads, 0, s>>>(cnt, n_cells, bsum, z);  // starts the chain
     pdl_chain = true;
     go(k_scan_bsum, 1, 1024, s, bsum, nbs);
-    // the previous step's photon pass reads the slots and positions the sort
-    // rewrites, and with proximity FRET the bucket starts
-    if (phot_uses_cells) join_photons(s);
     go(k_scan_down, nbs, kScanThreads, s, cnt, n_cells, bsum, cell_start, cursor);
-    join_photons(s);
+    join_photons(s);  // it reads the slots and positions the sort rewrites
     mark(1, s);
     cur ^= 1;
     DevState st = dev_state();
