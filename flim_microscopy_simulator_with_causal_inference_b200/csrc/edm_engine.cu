@@ -144,7 +144,8 @@ struct EdmEngine {
   uint8_t* flags[2] = {nullptr, nullptr};
   int32_t* ids[2] = {nullptr, nullptr};
   int cur = 0;
-  int32_t *slot_of_id = nullptr, *bond = nullptr;
+  int32_t* slot_of_id[2] = {nullptr, nullptr};  // of the current step and the one before, as flags and ids
+  int32_t* bond = nullptr;
   uint8_t *has_dye = nullptr, *bleached = nullptr;
   int8_t *dye = nullptr, *ctmc = nullptr;
   int32_t *cell_start = nullptr, *cursor = nullptr, *cnt = nullptr, *bsum = nullptr;
@@ -158,7 +159,8 @@ struct EdmEngine {
   int64_t* bind_key = nullptr;
   int32_t *emit_id = nullptr, *emit_n = nullptr, *emit_nd = nullptr, *emit_acc = nullptr;
   int8_t* emit_cls = nullptr;
-  int64_t* emit_off = nullptr;
+  int64_t* tile_n = nullptr;
+  unsigned* phot_ticket = nullptr;
   int32_t* ph_pid = nullptr;
   double* ph_t = nullptr;
   int8_t* ph_ch = nullptr;
@@ -225,7 +227,7 @@ struct EdmEngine {
     s.flags = flags[cur];
     s.ids_old = ids[cur ^ 1];
     s.ids = ids[cur];
-    s.slot_of_id = slot_of_id;
+    s.slot_of_id = slot_of_id[cur];
     s.bond = bond;
     s.cell_start = cell_start;
     s.cell_cursor = cursor;
@@ -273,7 +275,8 @@ struct EdmEngine {
     p.emit_nd = emit_nd;
     p.emit_acc = emit_acc;
     p.emit_cls = emit_cls;
-    p.emit_off = emit_off;
+    p.tile_n = tile_n;
+    p.ticket = phot_ticket;
     p.has_dye = has_dye;
     p.dye = dye;
     p.ctmc = ctmc;
@@ -658,6 +661,12 @@ struct EdmEngine {
   bool pdl_chain = false;
   template <typename... K, typename... A>
   void go(void (*kernel)(K...), dim3 grid, int block, cudaStream_t s, A&&... args) {
+    launch(kernel, grid, block, s, pdl_chain, std::forward<A>(args)...);
+    pdl_chain = true;
+  }
+  // dependent: the operation before it on the stream is a kernel that opens with pdl_enter()
+  template <typename... K, typename... A>
+  void launch(void (*kernel)(K...), dim3 grid, int block, cudaStream_t s, bool dependent, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
@@ -669,9 +678,8 @@ struct EdmEngine {
     cfg.attrs = at;
     // created streams only (not the legacy or per-thread default stream)
     const bool created = reinterpret_cast<uintptr_t>(s) > 2;
-    cfg.numAttrs = (pdl_on && pdl_chain && created && !prof && !pass_prof && tune_kernel < 0) ? 1 : 0;
+    cfg.numAttrs = (pdl_on && dependent && created && !prof && !pass_prof && tune_kernel < 0) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-    pdl_chain = true;
   }
 
   template <bool F64>
@@ -757,13 +765,15 @@ struct EdmEngine {
     pdl_chain = true;
     go(k_scan_bsum, 1, 1024, s, bsum, nbs);
     go(k_scan_down, nbs, kScanThreads, s, cnt, n_cells, bsum, cell_start, cursor);
-    join_photons(s);  // it reads the slots and positions the sort rewrites
     mark(1, s);
     cur ^= 1;
     DevState st = dev_state();
     tune_mark(TK_SCATTER, 0, s);
     launch_scatter<F64>(st, s);
     tune_mark(TK_SCATTER, 1, s);
+    // it reads the flags and the map from particles to slots, which the sort
+    // writes to their other copies, and the positions the move rewrites
+    join_photons(s);
     mark(2, s);
     tune_mark(TK_MOVE, 0, s);
     launch_move<F64>(st, s);
@@ -840,7 +850,7 @@ struct EdmEngine {
     int n = 3 + 1 + 1 + (int)passes.size() + (react_ticket ? 0 : 1);
     for (const Pass& ps : passes)  // the sweeper-list contact shapes launch two kernels
       if (ps.kind == P_CONTACTS && kContactSlots[shape[TK_CONTACTS]] == 0) ++n;
-    if (with_photons) n += (neblk > 0 ? 3 : 1) + 1 + (nphblk > 0 ? 1 : 0) + 1;
+    if (with_photons) n += (neblk > 0 ? 2 : 1) + (nphblk > 0 ? 1 : 0);
     if (rec_cap > 0) n += 2 + ((has_phot && neblk > 0) ? 1 : 0);
     return n;
   }
@@ -852,12 +862,14 @@ struct EdmEngine {
 
   template <bool F64>
   void enqueue_photons_t(cudaStream_t s) {
-    DevState st = dev_state();
-    PhotState ph = phot_state();
-    if (neblk > 0) k_phot_count<F64><<<neblk, kBlock, 0, s>>>(dp, pp, eblk, st, ph, cells_valid ? 1 : 0);
-    k_phot_scan<<<R, 256, 0, s>>>(pp, ph, counters, status);
-    if (neblk > 0) k_phot_write<F64><<<neblk, kBlock, 0, s>>>(dp, pp, eblk, st, ph, counters);
-    k_phot_advance<<<1, 1, 0, s>>>(d_pstep, d_batch_key);
+    const DevState st = dev_state();
+    const PhotState ph = phot_state();
+    if (neblk == 0) {
+      launch(k_phot_none, 1, 256, s, false, R, ph);
+      return;
+    }
+    launch(k_phot_count<F64>, neblk, kBlock, s, false, dp, pp, eblk, st, ph, cells_valid ? 1 : 0);
+    launch(k_phot_write<F64>, neblk, kBlock, s, true, dp, pp, eblk, st, ph, counters);
   }
 
   void enqueue_photons(cudaStream_t s) {
@@ -865,17 +877,8 @@ struct EdmEngine {
     else enqueue_photons_t<false>(s);
   }
 
-  template <bool F64>
-  void enqueue_scope_t(cudaStream_t s) {
-    DevState st = dev_state();
-    PhotState ph = phot_state();
-    if (nphblk > 0) k_scope<F64><<<nphblk, kBlock, 0, s>>>(dp, pp, sp, phblk, st, ph);
-    k_scope_received<<<(R + 127) / 128, 128, 0, s>>>(pp, R, ph, counters);
-  }
-
   void enqueue_scope(cudaStream_t s) {
-    if (f64) enqueue_scope_t<true>(s);
-    else enqueue_scope_t<false>(s);
+    if (nphblk > 0) launch(k_scope, nphblk, kBlock, s, false, dp, pp, sp, phblk, counters, phot_state());
   }
 
   // The positions of the current photon batch from the current state (a batch
@@ -890,8 +893,9 @@ struct EdmEngine {
 
   // A step's photon pass and detection pass beside the next step, each on a
   // stream of its own.  The photon pass reads the step's final state: the next
-  // step's bucket scan may run beside it, its bucket starts and sort may not
-  // (enqueue_dynamics joins it before them).  The detection pass reads only the
+  // step's bucket scan and sort may run beside it, its move may not
+  // (enqueue_dynamics joins it before the move; with proximity FRET, which
+  // reads the bucket starts, before the scan).  The detection pass reads only the
   // photon records, which carry their positions: the next step's dynamics run
   // beside it, the next photon pass waits for it.  A census and the end of the
   // call wait for both.  Errors surface at the call's cudaGetLastError or at
@@ -1184,7 +1188,8 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   ALLOC(E->flags[1], np + 4);
   ALLOC(E->ids[0], np);
   ALLOC(E->ids[1], np);
-  ALLOC(E->slot_of_id, np);
+  ALLOC(E->slot_of_id[0], np);
+  ALLOC(E->slot_of_id[1], np);
   ALLOC(E->bond, np);
   ALLOC(E->has_dye, np);
   ALLOC(E->bleached, np);
@@ -1286,7 +1291,8 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
     ALLOC(E->emit_nd, np);
     ALLOC(E->emit_acc, np);
     ALLOC(E->emit_cls, np);
-    ALLOC(E->emit_off, np);
+    ALLOC(E->tile_n, np / kBlock + (size_t)n_replicas + 1);  // tiles of kBlock emitters, per replica
+    ALLOC(E->phot_ticket, 1);
     ALLOC(E->ph_pid, nph);
     ALLOC(E->ph_t, nph);
     ALLOC(E->ph_ch, nph);
@@ -1532,11 +1538,11 @@ int edm_set_state(EdmEngine* E, const EdmHostState* st, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_set_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, dpos, E->st_sp, E->st_alive, E->pos_post, E->lo_post,
-                                                    E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id,
+                                                    E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
                                                     E->cnt);
     else
       k_set_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, dpos, E->st_sp, E->st_alive, E->pos_post, E->lo_post,
-                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id,
+                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
                                                      E->cnt);
     k_bond_to_global<<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->bond);
   }
@@ -1604,11 +1610,11 @@ int edm_get_state(EdmEngine* E, EdmHostState* st, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_get_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                    E->slot_of_id, E->bond, E->st_pos, E->st_sp, E->st_alive,
+                                                    E->slot_of_id[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
                                                     E->st_bond);
     else
       k_get_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                     E->slot_of_id, E->bond, E->st_pos, E->st_sp, E->st_alive,
+                                                     E->slot_of_id[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
                                                      E->st_bond);
   }
   CUDA_TRY(cudaGetLastError());
@@ -1669,11 +1675,11 @@ int edm_install_state(EdmEngine* E, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_set_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, in.pos, in.sp, in.alive, E->pos_post, E->lo_post,
-                                                    E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id,
+                                                    E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
                                                     E->cnt);
     else
       k_set_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, in.pos, in.sp, in.alive, E->pos_post, E->lo_post,
-                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id,
+                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
                                                      E->cnt);
     k_bond_to_global<<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->bond);
   }
@@ -1708,10 +1714,10 @@ int edm_get_state_async(EdmEngine* E, EdmHostState* st, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_get_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                    E->slot_of_id, E->bond, out.pos, out.sp, out.alive, out.bond);
+                                                    E->slot_of_id[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
     else
       k_get_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                     E->slot_of_id, E->bond, out.pos, out.sp, out.alive, out.bond);
+                                                     E->slot_of_id[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
   }
   CUDA_TRY(cudaMemcpyAsync(out.ctmc, E->ctmc, N, cudaMemcpyDeviceToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(out.bleached, E->bleached, N, cudaMemcpyDeviceToDevice, s));

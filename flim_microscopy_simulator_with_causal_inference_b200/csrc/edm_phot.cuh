@@ -7,8 +7,8 @@
 // emitting its donor photons then its FRET-acceptor photons, one shared
 // arrival-time cursor.  Here every emitter draws its counts independently
 // (keyed by particle index), an exclusive scan over emitters in particle
-// order gives each photon its stream index k, and every per-photon draw is
-// keyed by k.  Photons beyond the reference's buffer (max_photons) are
+// order (per tile of emitters, and over the tiles' totals) gives each photon
+// its stream index k, and every per-photon draw is keyed by k.  Photons beyond the reference's buffer (max_photons) are
 // dropped exactly as its `break` drops them; arrival draws beyond its
 // est_photons stream fall back to t = tau as it does.
 #pragma once
@@ -31,7 +31,7 @@ struct PhotState {
   int32_t* emit_nd;         // donor photons
   int32_t* emit_acc;        // FRET acceptor (global id) or -1
   int8_t* emit_cls;         // FRET class
-  int64_t* emit_off;        // first photon index within the replica
+  int64_t* tile_n;          // photons of each tile of kBlock emitters
   const uint8_t* has_dye;   // id-indexed
   const int8_t* dye;        // id-indexed
   int8_t* ctmc;             // id-indexed
@@ -46,10 +46,11 @@ struct PhotState {
   uint32_t* touch;          // one bit per 128-bin stretch of flim that a count has landed in
   int64_t* d_pstep;         // photophysics call counter
   int64_t* d_batch_key;     // key of the last batch
+  unsigned* ticket;         // blocks of the write pass that have finished
 };
 
-// Poisson draw of the reference (photophysics.py:486-521): an LCG seeded from
-// one uniform, Knuth's product for mean < 30; exp(-mean) from the host table.
+// Poisson draw of the reference (photophysics.py:486-521; its division by
+// 2^53 is an exact scaling): an LCG seeded from one uniform, Knuth's product for mean < 30; exp(-mean) from the host table.
 __device__ __forceinline__ int64_t poisson_lcg(double mean, double u_seed, double exp_neg_mean, uint32_t* status) {
   if (mean <= 0.0) return 0;
   uint64_t s = (uint64_t)(int64_t)__dmul_rn(u_seed, 9.007199254740992e15);
@@ -58,7 +59,7 @@ __device__ __forceinline__ int64_t poisson_lcg(double mean, double u_seed, doubl
     double pr = 1.0;
     for (;;) {
       s = s * 6364136223846793005ull + 1442695040888963407ull;
-      const double u = __ddiv_rn(__ull2double_rn(s >> 11), 9.007199254740992e15);
+      const double u = __dmul_rn(__ull2double_rn(s >> 11), 0x1p-53);
       pr = __dmul_rn(pr, u);
       if (pr <= exp_neg_mean) break;
       k += 1;
@@ -68,9 +69,9 @@ __device__ __forceinline__ int64_t poisson_lcg(double mean, double u_seed, doubl
   }
   set_status(status, EDM_STATUS_POISSON_NORMAL);
   s = s * 6364136223846793005ull + 1442695040888963407ull;
-  double u1 = __ddiv_rn(__ull2double_rn(s >> 11), 9.007199254740992e15);
+  double u1 = __dmul_rn(__ull2double_rn(s >> 11), 0x1p-53);
   s = s * 6364136223846793005ull + 1442695040888963407ull;
-  const double u2 = __ddiv_rn(__ull2double_rn(s >> 11), 9.007199254740992e15);
+  const double u2 = __dmul_rn(__ull2double_rn(s >> 11), 0x1p-53);
   if (u1 < 1e-30) u1 = 1e-30;
   const double z = sqrt(-2.0 * log(u1)) * cos(6.283185307179586 * u2);
   const int64_t n = (int64_t)(mean + sqrt(mean) * z + 0.5);
@@ -169,38 +170,29 @@ __device__ int fret_class(const EdmDynParams& p, const EdmPhotParams& pp, const 
   return cls;
 }
 
-// Per emitter: FRET class, photon counts, photophysical transition.
+// FRET class, photon count and photophysical transition of emitter e; returns
+// its number of photons.
 template <bool F64>
-__global__ void __launch_bounds__(kBlock) k_phot_count(const EdmDynParams* __restrict__ DP,
-                                                       const EdmPhotParams* __restrict__ PP,
-                                                       const int2* __restrict__ eblk, DevState st, PhotState ph,
-                                                       int cells_valid) {
-  const Tile t = tile_of(eblk);
-  const EdmPhotParams& pp = PP[t.r];
-  const EdmDynParams& p = DP[t.r];
-  const int64_t e = t.s;
-  if (e >= pp.emitter_offset + pp.n_emitters) return;
+__device__ __forceinline__ int count_photons(const EdmDynParams& p, const EdmPhotParams& pp, const DevState& st,
+                                             const PhotState& ph, int r, int64_t e, int cells_valid) {
   const int gid = ph.emit_id[e];
   const int lid = gid - (int)p.particle_offset;
-  ph.emit_n[e] = 0;
-  ph.emit_nd[e] = 0;
-  ph.emit_acc[e] = -1;
   const int64_t slot = st.slot_of_id[gid];
   const uint8_t f = st.flags[slot];
-  if (!ph.has_dye[gid] || !fl_alive(f) || ph.bleached[gid]) return;
-  const int dt = ph.dye[gid];
-  if (dt < 0 || dt >= pp.n_fluoro) return;
+  const uint8_t dyed = ph.has_dye[gid], bleached = ph.bleached[gid];
+  const int dt = ph.dye[gid], cur = ph.ctmc[gid];
+  if (!dyed || !fl_alive(f) || bleached) return 0;
+  if (dt < 0 || dt >= pp.n_fluoro) return 0;
   const int s0 = pp.ground[dt], s1 = pp.excited[dt], t1 = pp.t1[dt], bl = pp.bl[dt];
-  const int cur = ph.ctmc[gid];
   int pss;
   if (cur == s0 || cur == s1) pss = 0;
   else if (t1 >= 0 && cur == t1) pss = 1;
   else if (bl >= 0 && cur == bl) {
     ph.bleached[gid] = 1;
-    return;
+    return 0;
   } else pss = 0;
   int acc = -1;
-  const int cls = fret_class<F64>(p, pp, st, ph, t.r, gid, slot, dt, true, cells_valid, acc);
+  const int cls = fret_class<F64>(p, pp, st, ph, r, gid, slot, dt, true, cells_valid, acc);
   const int64_t key = *ph.d_pstep;
   const double up = uniform1(p.seed, key, EDM_S_PH_POISSON, (uint64_t)lid, 0);
   const double ut = uniform1(p.seed, key, EDM_S_PH_TRANS, (uint64_t)lid, 0);
@@ -211,7 +203,6 @@ __global__ void __launch_bounds__(kBlock) k_phot_count(const EdmDynParams* __res
     nf = poisson_lcg(mf, __dadd_rn(__dmul_rn(up, 0.5), 0.25), pp.exp_neg_f[dt][pss][cls], st.status);
   const int64_t ntot = nd + ((nf > 0 && acc >= 0) ? nf : 0);
   ph.emit_nd[e] = (int32_t)nd;
-  ph.emit_n[e] = (int32_t)ntot;
   ph.emit_acc[e] = acc;
   ph.emit_cls[e] = (int8_t)cls;
   // transition (photophysics.py:474-481)
@@ -221,54 +212,44 @@ __global__ void __launch_bounds__(kBlock) k_phot_count(const EdmDynParams* __res
     ph.ctmc[gid] = (int8_t)(bl >= 0 ? bl : s0);
     ph.bleached[gid] = 1;
   }
+  return (int)ntot;
 }
 
-// Exclusive scan of emitter photon counts, one block per replica.
-__global__ void k_phot_scan(const EdmPhotParams* __restrict__ PP, PhotState ph, int64_t* counters, uint32_t* status) {
-  const int r = blockIdx.x;
-  const EdmPhotParams& pp = PP[r];
-  int64_t carry = 0;
-  __shared__ long long sh[32];
-  for (int64_t off = 0; off < pp.n_emitters; off += blockDim.x) {
-    const int64_t e = pp.emitter_offset + off + threadIdx.x;
-    const long long v = (off + threadIdx.x < pp.n_emitters) ? ph.emit_n[e] : 0;
-    // block scan (64-bit)
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    long long x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) sh[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      const int nw = blockDim.x >> 5;
-      long long w = lane < nw ? sh[lane] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        const long long y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      if (lane < nw) sh[lane] = w;
-    }
-    __syncthreads();
-    const long long base = wid > 0 ? sh[wid - 1] : 0;
-    const long long total = sh[(blockDim.x >> 5) - 1];
-    if (off + threadIdx.x < pp.n_emitters) ph.emit_off[e] = carry + base + x - v;
-    carry += total;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    int64_t n = carry;
-    if (n > pp.max_photons) {
-      n = pp.max_photons;
-      set_status(status, EDM_STATUS_PHOTON_CAP);
-    }
-    ph.ph_count[r] = n;
-    counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_PHOTONS] += n;
-  }
+// Sum of a 64-bit value over the block (all threads call it).
+__device__ __forceinline__ int64_t block_sum(int64_t v) {
+  __shared__ long long sums[32];
+  long long x = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = x;
+  __syncthreads();
+  x = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += sums[w];
+  __syncthreads();
+  return x;
 }
 
-// Write the photons of each emitter (photophysics.py:433-472).
+// Per tile of kBlock emitters: counts and their total.
+template <bool F64>
+__global__ void __launch_bounds__(kBlock) k_phot_count(const EdmDynParams* __restrict__ DP,
+                                                       const EdmPhotParams* __restrict__ PP,
+                                                       const int2* __restrict__ eblk, DevState st, PhotState ph,
+                                                       int cells_valid) {
+  pdl_enter();
+  const Tile t = tile_of(eblk);
+  const EdmPhotParams& pp = PP[t.r];
+  const int64_t e = t.s;
+  int n = 0;
+  if (e < pp.emitter_offset + pp.n_emitters) {
+    ph.emit_nd[e] = 0;
+    ph.emit_acc[e] = -1;
+    n = count_photons<F64>(DP[t.r], pp, st, ph, t.r, e, cells_valid);
+    ph.emit_n[e] = n;
+  }
+  const int64_t total = block_sum(n);
+  if (threadIdx.x == 0) ph.tile_n[blockIdx.x] = total;
+}
+
 // Absolute position of the particle with replica-local index pid.
 template <bool F64>
 __device__ __forceinline__ double2 particle_pos(const DevState& st, const Geo& g, int pid) {
@@ -277,61 +258,75 @@ __device__ __forceinline__ double2 particle_pos(const DevState& st, const Geo& g
   return make_double2(x, y);
 }
 
-// The photon records, each with the position of the particle it leaves
-// (the donor, or the acceptor of a FRET photon), so the detection pass reads
-// no particle state and can run beside the next step.
+// End of a photon batch: its key, and the next call's.
+__device__ __forceinline__ void advance_batch(const PhotState& ph) {
+  *ph.d_batch_key = *ph.d_pstep;
+  *ph.d_pstep += 1;
+}
+
+// The photon records of each tile of emitters (photophysics.py:433-472), each
+// with the position of the particle it leaves (the donor, or the acceptor of a
+// FRET photon), so the detection pass reads no particle state and can run
+// beside the next step.  A tile's first stream index is the total of the
+// replica's tiles before it, summed by the block itself (a scan by one block
+// per replica took 140 us for 46,000 emitters); within the tile each thread
+// takes a photon, not an emitter, and the block adds its counts to the
+// replica's counters once.  The replica's last tile sets the batch's size, the
+// last block the batch's key.
 template <bool F64>
 __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __restrict__ DP,
                                                        const EdmPhotParams* __restrict__ PP,
                                                        const int2* __restrict__ eblk, DevState st, PhotState ph,
                                                        int64_t* counters) {
+  pdl_enter();
+  __shared__ int first[kBlock];  // first photon of each emitter within the tile
   const Tile t = tile_of(eblk);
   const EdmPhotParams& pp = PP[t.r];
-  const int64_t e = t.s;
-  if (e >= pp.emitter_offset + pp.n_emitters) return;
-  const int ntot = ph.emit_n[e];
-  if (ntot == 0) return;
   const EdmDynParams& p = DP[t.r];
-  const int gid = ph.emit_id[e];
-  const int lid = gid - (int)p.particle_offset;
-  const int nd = ph.emit_nd[e];
-  const int dt = ph.dye[gid];
-  const int cls = ph.emit_cls[e];
-  const double tau = pp.tau[dt][cls];
-  const int64_t off = ph.emit_off[e];
+  const int64_t e0 = t.s - threadIdx.x, e_end = pp.emitter_offset + pp.n_emitters;
+  const int ordinal = (int)((e0 - pp.emitter_offset) / kBlock);
+  int64_t before = 0;
+  for (int k = threadIdx.x; k < ordinal; k += kBlock) before += ph.tile_n[blockIdx.x - ordinal + k];
+  const int64_t base = block_sum(before);
+  int total;
+  const int n_mine = t.s < e_end ? ph.emit_n[t.s] : 0;
+  first[threadIdx.x] = block_exclusive_scan(n_mine, total);
+  __syncthreads();
   const int64_t key = *ph.d_pstep;
   const Geo g(p);
-  const double2 xy_donor = particle_pos<F64>(st, g, lid);
-  double2 xy_acc = xy_donor;
-  bool have_acc = false;
   int n_donor_ch = 0, n_acc_ch = 0, n_fret = 0;
-  for (int j = 0; j < ntot; ++j) {
-    const int64_t k = off + j;
+  for (int i = threadIdx.x; i < total; i += kBlock) {
+    const int64_t k = base + i;
     if (k >= pp.max_photons) break;
-    const bool fret = j >= nd;
-    int ch = dt, pid = lid;
-    double ta = tau;
+    int lo = 0, hi = kBlock - 1;  // the last emitter whose first photon is at or before i
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (first[mid] <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    const int64_t e = e0 + lo;
+    const int gid = ph.emit_id[e];
+    const int dt = ph.dye[gid], cls = ph.emit_cls[e];
+    const bool fret = i - first[lo] >= ph.emit_nd[e];
+    int ch = dt, pid = gid - (int)p.particle_offset;
+    double ta = pp.tau[dt][cls];
     if (fret) {
       const int acc = ph.emit_acc[e];
       const int at = ph.dye[acc];
-      ta = (at >= 0 && at < pp.n_fluoro) ? pp.tau_all[at] : tau;
+      if (at >= 0 && at < pp.n_fluoro) ta = pp.tau_all[at];
       ch = at;
       pid = acc - (int)p.particle_offset;
     }
-    double tt;
+    double tt = ta;
     if (k < pp.est_photons) {
       double u = uniform1(p.seed, key, EDM_S_PH_ARRIVAL, (uint64_t)k, 0);
       if (u < 1e-30) u = 1e-30;
       tt = -ta * log(u);
-    } else {
-      tt = ta;
     }
     const int64_t o = pp.photon_offset + k;
-    if (fret && !have_acc && pid >= 0 && pid < p.n_particles) {
-      xy_acc = particle_pos<F64>(st, g, pid);
-      have_acc = true;
-    }
-    ph.ph_xy[o] = fret ? xy_acc : xy_donor;
+    // a FRET photon whose acceptor lies outside the replica keeps the donor's position
+    const int at = fret && !(pid >= 0 && pid < p.n_particles) ? gid - (int)p.particle_offset : pid;
+    ph.ph_xy[o] = particle_pos<F64>(st, g, at);
     ph.ph_pid[o] = pid;
     ph.ph_t[o] = tt;
     ph.ph_ch[o] = (int8_t)ch;
@@ -340,34 +335,51 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
     n_acc_ch += ch == pp.acceptor_channel;
     n_fret += fret;
   }
-  int64_t* c = counters + (int64_t)t.r * EDM_NCOUNTERS;
-  if (n_donor_ch) atomic_add_i64(c + EDM_C_DONOR_PH, n_donor_ch);
-  if (n_acc_ch) atomic_add_i64(c + EDM_C_ACCEPTOR_PH, n_acc_ch);
-  if (n_fret) atomic_add_i64(c + EDM_C_FRET_PH, n_fret);
+  if (total > 0) {
+    int64_t* c = counters + (int64_t)t.r * EDM_NCOUNTERS;
+    const int64_t nd = block_sum(n_donor_ch), na = block_sum(n_acc_ch), nf = block_sum(n_fret);
+    if (threadIdx.x == 0) {
+      if (nd) atomic_add_i64(c + EDM_C_DONOR_PH, nd);
+      if (na) atomic_add_i64(c + EDM_C_ACCEPTOR_PH, na);
+      if (nf) atomic_add_i64(c + EDM_C_FRET_PH, nf);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (e0 + kBlock >= e_end) {  // the replica's last tile
+    int64_t n = base + total;
+    if (n > pp.max_photons) {
+      n = pp.max_photons;
+      set_status(st.status, EDM_STATUS_PHOTON_CAP);
+    }
+    ph.ph_count[t.r] = n;
+    counters[(int64_t)t.r * EDM_NCOUNTERS + EDM_C_PHOTONS] += n;
+  }
+  if (blockIdx.x == 0)  // replicas without emitters have no tile
+    for (int r = 0; r < st.n_rep; ++r)
+      if (PP[r].n_emitters == 0) ph.ph_count[r] = 0;
+  __threadfence();
+  if (atomicAdd(ph.ticket, 1u) == gridDim.x - 1) {
+    *ph.ticket = 0;
+    advance_batch(ph);
+  }
 }
 
-__global__ void k_phot_advance(int64_t* d_pstep, int64_t* d_batch_key) {
-  *d_batch_key = *d_pstep;
-  *d_pstep += 1;
+// The photon pass of a system without emitters.
+__global__ void k_phot_none(int n_rep, PhotState ph) {
+  pdl_enter();
+  for (int r = threadIdx.x; r < n_rep; r += blockDim.x) ph.ph_count[r] = 0;
+  if (threadIdx.x == 0) advance_batch(ph);
 }
 
-// Per photon: detection efficiency, PSF pixel draw, IRF jitter, TCSPC bin.
-template <bool F64>
-__global__ void __launch_bounds__(kBlock) k_scope(const EdmDynParams* __restrict__ DP,
-                                                  const EdmPhotParams* __restrict__ PP,
-                                                  const EdmScopeParams* __restrict__ SP,
-                                                  const int2* __restrict__ phblk, DevState st, PhotState ph) {
-  const Tile t = tile_of(phblk);
-  const EdmPhotParams& pp = PP[t.r];
-  const int64_t k = t.s - pp.photon_offset;
-  if (k >= ph.ph_count[t.r]) return;
-  const EdmDynParams& p = DP[t.r];
-  const EdmScopeParams& sp = SP[t.r];
+// Photon o (stream index k): detection efficiency, PSF pixel draw, IRF jitter,
+// TCSPC bin; whether it is detected (a pixel drawn; its time may still be lost).
+__device__ __forceinline__ bool detect_photon(const EdmDynParams& p, const EdmScopeParams& sp, const PhotState& ph,
+                                              int64_t o, int64_t k) {
   const int64_t key = *ph.d_batch_key;
-  const int64_t o = t.s;
-  if (!(uniform1(p.seed, key, EDM_S_SC_QE, (uint64_t)k, 0) < sp.qe)) return;
+  if (!(uniform1(p.seed, key, EDM_S_SC_QE, (uint64_t)k, 0) < sp.qe)) return false;
   const int pid = ph.ph_pid[o];
-  if (pid < 0 || pid >= p.n_particles) return;
+  if (pid < 0 || pid >= p.n_particles) return false;
   const double2 xy = ph.ph_xy[o];
   const double x = xy.x, y = xy.y;
   int ch = ph.ph_ch[o];
@@ -379,8 +391,8 @@ __global__ void __launch_bounds__(kBlock) k_scope(const EdmDynParams* __restrict
   const double fy = (y - sp.offset_y) / sp.pixel_size - 0.5;
   const int i0 = (int)floor(fx + 0.5), j0 = (int)floor(fy + 0.5);
   const int R = sp.psf_range_px;
-  if (i0 < -R || i0 >= sp.nx + R) return;
-  if (j0 < -R || j0 >= sp.ny + R) return;
+  if (i0 < -R || i0 >= sp.nx + R) return false;
+  if (j0 < -R || j0 >= sp.ny + R) return false;
   // Pixel weights exp(-(dx^2 + dy^2) / 2 sigma^2) over the in-FOV pixels of
   // the (2R+1)^2 window, summed and searched in the reference's order (di
   // outer, dj inner): the Gaussian factors into exp(-dx^2 / 2 sigma^2)
@@ -406,7 +418,7 @@ __global__ void __launch_bounds__(kBlock) k_scope(const EdmDynParams* __restrict
       ++n;
     }
   }
-  if (n == 0 || total <= 0.0) return;
+  if (n == 0 || total <= 0.0) return false;
   const double u = uniform1(p.seed, key, EDM_S_SC_ASSIGN, (uint64_t)k, 0) * total;
   int si = -1, sj = -1, fi = -1, fj = -1;
   double cum = 0.0;
@@ -434,17 +446,36 @@ __global__ void __launch_bounds__(kBlock) k_scope(const EdmDynParams* __restrict
     si = fi;
     sj = fj;
   }
-  int64_t* cnt = st.counters + (int64_t)t.r * EDM_NCOUNTERS;
-  atomic_add_i64(cnt + EDM_C_DETECTED, 1);
   const double z = normal2(p.seed, key, EDM_S_SC_JITTER, (uint64_t)k).u0;
   double tt = __dadd_rn(ph.ph_t[o], __dmul_rn(sp.sigma_irf, z));
-  if (ch < 0 || ch >= sp.n_channels) return;
+  if (ch < 0 || ch >= sp.n_channels) return true;
   if (tt < 0.0) tt = 0.0;
   const int64_t b = (int64_t)__ddiv_rn(tt, sp.bin_width);
-  if (b >= sp.n_bins) return;
+  if (b >= sp.n_bins) return true;
   const int64_t e = sp.flim_offset + (((int64_t)ch * sp.nx + si) * sp.ny + sj) * sp.n_bins + b;
   atomicAdd(&ph.flim[e], 1u);
   touch_stretch(ph.touch, e);
+  return true;
+}
+
+// A tile of a replica's photon buffer; the block adds its detections to the
+// replica's counter once, the replica's first tile the photons received
+// (microscope.py:1093).
+__global__ void __launch_bounds__(kBlock) k_scope(const EdmDynParams* __restrict__ DP,
+                                                  const EdmPhotParams* __restrict__ PP,
+                                                  const EdmScopeParams* __restrict__ SP,
+                                                  const int2* __restrict__ phblk, int64_t* counters, PhotState ph) {
+  pdl_enter();
+  const Tile t = tile_of(phblk);
+  const int64_t k0 = t.s - threadIdx.x - PP[t.r].photon_offset, n = ph.ph_count[t.r];
+  if (k0 >= n) return;
+  const int64_t k = k0 + threadIdx.x;
+  const bool hit = k < n && detect_photon(DP[t.r], SP[t.r], ph, t.s, k);
+  const int hits = __syncthreads_count(hit);
+  if (threadIdx.x != 0) return;
+  int64_t* c = counters + (int64_t)t.r * EDM_NCOUNTERS;
+  if (hits) atomic_add_i64(c + EDM_C_DETECTED, hits);
+  if (k0 == 0) atomic_add_i64(c + EDM_C_RECEIVED, n);
 }
 
 // The positions of a photon batch set from the host (edm_set_photons) or left
@@ -463,12 +494,6 @@ __global__ void __launch_bounds__(kBlock) k_photon_positions(const EdmDynParams*
   if (pid < 0 || pid >= p.n_particles) return;
   const Geo g(p);
   ph.ph_xy[t.s] = particle_pos<F64>(st, g, pid);
-}
-
-// Photons received per replica (microscope.py:1093).
-__global__ void k_scope_received(const EdmPhotParams* __restrict__ PP, int n_rep, PhotState ph, int64_t* counters) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < n_rep) counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_RECEIVED] += ph.ph_count[r];
 }
 
 // Dark counts (microscope.py:850-887) — one thread per (channel, pixel).
