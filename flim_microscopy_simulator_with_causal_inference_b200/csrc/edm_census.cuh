@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kBlock) k_census_particles(const EdmDynParams*
     const uint8_t f = st.flags[t.s];
     alive = fl_alive(f);
     sp = fl_species(f);
-    const int id = st.ids[t.s];
+    const int id = slot_id(st, t.s);
     bonded = st.bond[id] >= 0;
     bl = bleached != nullptr && bleached[id] != 0;
   }

@@ -51,8 +51,8 @@ struct DevState {
   const uint8_t* flags_old;
   uint8_t* flags;     // slot flags of the current step
   const int32_t* ids_old;
-  int32_t* ids;       // global particle id of each slot
-  int32_t* slot_of_id;
+  int32_t* ids;       // global particle id of each slot, the top bit set in a tracked one
+  int32_t* slot_of_id;  // slot of each tracked particle (a dye carrier; with binding, every one)
   int32_t* bond;      // id-indexed, global id or -1
   int32_t* cell_start;   // sort-bucket starts [n_buckets + 1]
   int32_t* cell_cursor;
@@ -71,6 +71,7 @@ struct DevState {
   // candidate buffers
   int32_t* rec_count;    // [R]
   int32_t* rec_id;       // [R][kRecCap] local id
+  int32_t* rec_slot;     // [R][kRecCap]
   double* rec_xy;        // [R][kRecCap][2]
   int32_t* bind_count;   // [R]
   int64_t* bind_key;     // [R][kBindCap]
@@ -108,6 +109,12 @@ struct DevState {
   int n_rep;
   int64_t n_slots;
 };
+
+// Tracked particles keep their entry of slot_of_id current through every sort.
+// Nothing reads the others' entries, and their scattered 4-byte writes over the
+// whole map were a fifth of the sort's time.
+constexpr int32_t kTracked = (int32_t)0x80000000;
+__device__ __forceinline__ int slot_id(const DevState& st, int64_t s) { return st.ids[s] & ~kTracked; }
 
 __device__ __forceinline__ int replica_of(const int64_t* __restrict__ rep_first, int R, int64_t s) {
   int lo = 0, hi = R - 1;
@@ -583,53 +590,63 @@ __global__ void k_scan_down(int32_t* __restrict__ cnt, int64_t n, const int32_t*
   if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) start[0] = 0;
 }
 
+// A tile of one replica's slots: [first, end), the replica's first bucket and
+// its last one (non-alive particles).  A kernel that takes these from the tile
+// reads the slots' data one round trip earlier than through the replica's
+// parameter block.
+struct SlotTile {
+  int32_t first, end, bucket0, grave;
+};
+
+// The counting sort's permutation.  Its time is the chain of round trips a
+// warp makes (tile, slot, bucket cursor, stores) and its scattered stores, not
+// the cursor atomics: ranks taken in the move instead of cursors measured the
+// same.  So every load of a slot is issued before its cursor atomic (78 to 68
+// us for 4.7M slots) and only tracked particles update slot_of_id (68 to 53).
+// SPT tiles per block put SPT slots' loads and atomics in flight per thread.
 template <bool F64, int BS, int SPT>
-__global__ void __launch_bounds__(BS) k_scatter(const EdmDynParams* __restrict__ P, const int2* __restrict__ blk,
-                                                    int ntiles, DevState st) {
+__global__ void __launch_bounds__(BS) k_scatter(const SlotTile* __restrict__ tiles, int ntiles, DevState st) {
   pdl_enter();
-  // SPT tiles per block (blockIdx.x * SPT + k): each thread reads its slots'
-  // buckets and takes all their cursor positions before the first dependent
-  // store, so SPT atomics are in flight per thread
-  int64_t src[SPT], bkt[SPT];
+  using Pos = typename std::conditional<F64, double2, float2>::type;
+  int src[SPT], cl[SPT], id[SPT], dst[SPT], grave[SPT], bucket0[SPT];
   uint8_t fl[SPT];
-  int cl[SPT], dst[SPT];
+  Pos pos[SPT];
+  short2 lo[SPT];
 #pragma unroll
   for (int k = 0; k < SPT; ++k) {
     src[k] = -1;
     const int tile = (int)blockIdx.x * SPT + k;
     if (tile >= ntiles) continue;
-    const int2 b = blk[tile];
-    const EdmDynParams& p = P[b.x];
-    const int64_t s = (int64_t)(uint32_t)b.y + threadIdx.x;
-    if (s >= p.particle_offset + p.n_particles) continue;
+    const SlotTile t = tiles[tile];
+    const int s = t.first + (int)threadIdx.x;
+    if (s >= t.end) continue;
     src[k] = s;
+    bucket0[k] = t.bucket0;
+    grave[k] = t.grave;
     cl[k] = st.cell_post[s];
     fl[k] = st.flags_old[s];
-    bkt[k] = p.cell_offset + (fl_alive(fl[k]) ? cl[k] : p.nx * p.ny);
+    id[k] = st.ids_old[s];
+    pos[k] = ((const Pos*)st.pos_post)[s];
+    if constexpr (!F64) lo[k] = st.lo_post[s];
   }
 #pragma unroll
   for (int k = 0; k < SPT; ++k) {
     if (src[k] < 0) continue;
     // alive particles mostly have a cell to themselves: a plain atomic; the
     // non-alive ones all share their replica's last bucket: aggregated per warp
-    dst[k] = fl_alive(fl[k]) ? atomicAdd(&st.cell_cursor[bkt[k]], 1) : atomic_inc_aggregated(&st.cell_cursor[bkt[k]]);
+    dst[k] = fl_alive(fl[k]) ? atomicAdd(&st.cell_cursor[bucket0[k] + cl[k]], 1)
+                             : atomic_inc_aggregated(&st.cell_cursor[grave[k]]);
   }
 #pragma unroll
   for (int k = 0; k < SPT; ++k) {
     if (src[k] < 0) continue;
-    const int64_t s = src[k];
     const int d = dst[k];
-    if constexpr (F64) {
-      ((double2*)st.pos_pre)[d] = ((const double2*)st.pos_post)[s];
-    } else {
-      ((float2*)st.pos_pre)[d] = ((const float2*)st.pos_post)[s];
-      st.lo_pre[d] = st.lo_post[s];
-    }
+    ((Pos*)st.pos_pre)[d] = pos[k];
+    if constexpr (!F64) st.lo_pre[d] = lo[k];
     st.cell_pre[d] = cl[k];
     st.flags[d] = fl[k];
-    const int id = st.ids_old[s];
-    st.ids[d] = id;
-    st.slot_of_id[id] = d;
+    st.ids[d] = id[k];
+    if (id[k] & kTracked) st.slot_of_id[id[k] & ~kTracked] = d;
   }
 }
 
@@ -705,7 +722,7 @@ __device__ __forceinline__ void for_each_force_term(const EdmDynParams& p, const
       const int spj = fl_species(fj);
       const double sig = p.sigma[sp * EDM_MAX_SPECIES + spj];
       if (!(sig > 0.0)) return;
-      const int idj = st.ids[j] - (int)g.poff;
+      const int idj = slot_id(st, j) - (int)g.poff;
       const uint64_t order = idj < id ? (uint64_t)idj
                                       : ((1ull << 60) | ((uint64_t)ordinal << 32) | (uint64_t)(0xFFFFFFFFu - (uint32_t)idj));
       // The pair force itself is float64 on both paths: a pair inside force
@@ -856,7 +873,7 @@ __global__ void __launch_bounds__(BS, MINB) k_move(const EdmDynParams* __restric
   int id = 0;
   int64_t step = 0;
   if constexpr (F64) {
-    id = st.ids[s] - (int)g.poff;
+    id = slot_id(st, s) - (int)g.poff;
     step = *st.d_step;
   }
 
@@ -946,7 +963,7 @@ __global__ void __launch_bounds__(BS, MINB) k_move(const EdmDynParams* __restric
     ((double2*)st.pos_post)[s] = make_double2(x, y);
     newc = cell_index(x, g.sx, g.nx) * g.ny + cell_index(y, g.sy, g.ny);
   } else {
-    id = st.ids[s] - (int)g.poff;
+    id = slot_id(st, s) - (int)g.poff;
     step = *st.d_step;
     float z0, z1;
     normal2_f32(p.seed, step, EDM_S_BD_NORMAL, (uint64_t)id, z0, z1);
@@ -1210,7 +1227,7 @@ __device__ __forceinline__ void finish_contacts(const EdmDynParams* __restrict__
   const EdmDynParams& p = P[r];
   const Geo g(p);
   uint32_t bits = rx_of[fl_species(st.flags[sj.x]) * EDM_MAX_SPECIES + fl_species(st.flags[sj.y])];
-  const int ids = st.ids[sj.x] - g.poff, idj = st.ids[sj.y] - g.poff;
+  const int ids = slot_id(st, sj.x) - g.poff, idj = slot_id(st, sj.y) - g.poff;
   // the sweeper first, as the pre-move test (both differences change sign
   // exactly when the pair is swept from its other side)
   const double d2 = sep_sq<F64>(st.pos_post, st.cell_post, sj.x, sj.y, g);
@@ -1408,7 +1425,7 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
     for (uint32_t b = late; b; b &= b - 1) {
       const int c = __ffs(b) - 1;
       if (spe != p.cat[c].enzyme || d2 > p.cat[c].contact_sq) continue;
-      if (!cat_draw_passes(p, st, r, c, st.ids[e] - (int)g.poff, id_j, step)) continue;
+      if (!cat_draw_passes(p, st, r, c, slot_id(st, e) - (int)g.poff, id_j, step)) continue;
       out.file(c, e, (int)j);
     }
   });
@@ -1427,7 +1444,7 @@ __device__ __forceinline__ void catalytic_pair(const EdmDynParams& p, const DevS
   const EdmCat& C = p.cat[cidx];
   if (!fl_alive(fs) || fl_species(fs) != C.substrate) return;
   const Geo g(p);
-  const int ide = st.ids[es.x] - g.poff, ids = st.ids[es.y] - g.poff;
+  const int ide = slot_id(st, es.x) - g.poff, ids = slot_id(st, es.y) - g.poff;
   const uint32_t lo = ide < ids ? ide : ids, hi = ide < ids ? ids : ide;
   const uint64_t m = draw_u53(p.seed, *st.d_step, EDM_S_CAT + cidx, lo, hi);
   if (m >= st.cat_thr[(int64_t)r * EDM_MAX_CAT + cidx]) return;
@@ -1505,7 +1522,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_pass_draws(const EdmDynParams* __
     const uint8_t f = st.flags[s];
     const int sp = fl_species(f);
     const uint32_t todo = sp < EDM_MAX_SPECIES ? D->reach[fl_alive(f) ? 1 : 0][sp] : 0u;
-    const int id = st.ids[s] - (int)P[r].particle_offset;
+    const int id = slot_id(st, s) - (int)P[r].particle_offset;
     const uint32_t bits = draw_passes(st, D, P[r].seed, r, id, *st.d_step, todo);
     if (bits) {
       const int q = st.rep_pl ? (int)P[r].particle_offset + atomicAdd(&st.pl_count[r], 1) : atomicAdd(st.pl_count, 1);
@@ -1515,16 +1532,15 @@ __global__ void __launch_bounds__(kBlock, 8) k_pass_draws(const EdmDynParams* __
   });
 }
 
-// Puts particle `id` of replica r, recruited by exchange e, at (x, y).  It is
+// Puts particle `id` of replica r (in `slot`), recruited by exchange e, at (x, y).  It is
 // alive from here on, so the passes after this one that match it (`after`) get
 // their draws now, in its list entry (entry(q) = entry q of the list; it
 // exists: the particle was listed for this exchange's candidates).
 template <bool F64, typename Sink, typename Entry>
 __device__ __forceinline__ void place_recruit(const EdmDynParams& p, const Geo& g, const DevState& st, int r, int e,
-                                              int id, double x, double y, const Sink& sink,
+                                              int id, int64_t slot, double x, double y, const Sink& sink,
                                               const DrawPlan* __restrict__ D, uint32_t after, Entry entry) {
   const EdmExch& X = p.exch[e];
-  const int64_t slot = st.slot_of_id[g.poff + id];
   const int cxn = cell_index(x, g.sx, g.nx), cyn = cell_index(y, g.sy, g.ny);
   const int newc = cxn * g.ny + cyn;
   if constexpr (F64) {
@@ -1565,33 +1581,37 @@ __global__ void k_recruit_apply(const EdmDynParams* __restrict__ P, int n_rep, D
   st.rec_count[r] = 0;
   if (n == 0) return;
   int32_t* ids = st.rec_id + (int64_t)r * kRecCap;
+  int32_t* slots = st.rec_slot + (int64_t)r * kRecCap;
   double* xy = st.rec_xy + (int64_t)r * kRecCap * 2;
   for (int a = 1; a < n; ++a) {  // insertion sort by particle index
-    const int id = ids[a];
+    const int id = ids[a], slot = slots[a];
     const double x = xy[2 * a], y = xy[2 * a + 1];
     int b = a - 1;
     while (b >= 0 && ids[b] > id) {
       ids[b + 1] = ids[b];
+      slots[b + 1] = slots[b];
       xy[2 * (b + 1)] = xy[2 * b];
       xy[2 * (b + 1) + 1] = xy[2 * b + 1];
       --b;
     }
     ids[b + 1] = id;
+    slots[b + 1] = slot;
     xy[2 * (b + 1)] = x;
     xy[2 * (b + 1) + 1] = y;
   }
   const Geo g(p);
   const int take = n < X.max_recruits ? n : X.max_recruits;
   for (int a = 0; a < take; ++a)
-    place_recruit<F64>(p, g, st, r, e, ids[a], xy[2 * a], xy[2 * a + 1], DeltaArray{st.grid_delta}, D, after,
+    place_recruit<F64>(p, g, st, r, e, ids[a], slots[a], xy[2 * a], xy[2 * a + 1], DeltaArray{st.grid_delta}, D, after,
                        [&](int q) { return q >= 0 && q < *st.pl_count ? st.pl + q : (int4*)nullptr; });
   atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_RECRUITED], take);
 }
 
-// Candidates of one replica's recruitment: [kRecCap] ids and positions.
+// Candidates of one replica's recruitment: [kRecCap] ids, slots and positions.
 struct RecruitList {
   int32_t* count;
   int32_t* id;
+  int32_t* slot;
   double* xy;
 };
 
@@ -1599,7 +1619,7 @@ struct RecruitList {
 // particle of the species whose keyed draw accepts at the keyed position.
 // The per-particle passes below run on listed particles only.
 __device__ __forceinline__ void recruit_candidate(const EdmDynParams& p, const DevState& st, const RecruitList& out,
-                                                  int id, int e) {
+                                                  int id, int64_t slot, int e) {
   const EdmExch& X = p.exch[e];
   const int64_t step = *st.d_step;
   const double ua = uniform1(p.seed, step, EDM_S_EX_ACCEPT + 4 * e, (uint64_t)id, 0);
@@ -1633,6 +1653,7 @@ __device__ __forceinline__ void recruit_candidate(const EdmDynParams& p, const D
     const int k = atomicAdd(out.count, 1);
     if (k < kRecCap) {
       out.id[k] = id;
+      out.slot[k] = (int32_t)slot;
       out.xy[2 * k] = cx;
       out.xy[2 * k + 1] = cy;
     } else {
@@ -1727,7 +1748,7 @@ __device__ __forceinline__ uint32_t run_passes(const EdmDynParams& p, const DevS
     if (!((bits >> pk) & 1u) || !matches(f, sg.m[k])) continue;
     const int kind = sg.kind[k], idx = sg.index[k];
     if (kind == kGroupRecruit) {
-      recruit_candidate(p, st, rec, id, idx);
+      recruit_candidate(p, st, rec, id, s, idx);
       continue;
     }
     const uint8_t f0 = f;
@@ -1746,7 +1767,8 @@ __global__ void __launch_bounds__(kBlock) k_particle_passes(const EdmDynParams* 
   const int n = *st.pl_count;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int4 e = st.pl[q];
-    const RecruitList rec{st.rec_count + e.z, st.rec_id + (int64_t)e.z * kRecCap, st.rec_xy + (int64_t)e.z * kRecCap * 2};
+    const int64_t at = (int64_t)e.z * kRecCap;
+    const RecruitList rec{st.rec_count + e.z, st.rec_id + at, st.rec_slot + at, st.rec_xy + 2 * at};
     const uint32_t bits = run_passes<F64>(P[e.z], st, *G, D, e, rec, DeltaArray{st.grid_delta});
     if (bits != (uint32_t)e.y) st.pl[q].y = (int)bits;
   }
@@ -1764,12 +1786,12 @@ __global__ void __launch_bounds__(kBlock) k_bind_candidates(const EdmDynParams* 
     const EdmBind& B = p.bind[b];
     const int spi = fl_species(st.flags[s]);
     const Geo g(p);
-    const int id = st.ids[s] - (int)g.poff;
+    const int id = slot_id(st, s) - (int)g.poff;
     if (st.bond[g.poff + id] >= 0) return;
     const int64_t step = *st.d_step;
     for_neighbour_slots(g, st, st.cell_pre[s], [&](int j, int ordinal, int, int) {
       {
-        const int idj = st.ids[j] - (int)g.poff;
+        const int idj = slot_id(st, j) - (int)g.poff;
         if (idj <= id) return;
         const uint8_t fj = st.flags[j];
         if (!fl_alive(fj)) return;
@@ -1864,7 +1886,7 @@ __global__ void __launch_bounds__(kBlock) k_dissociate(const EdmDynParams* __res
     const EdmDynParams& p = P[r];
     const EdmBind& B = p.bind[b];
     const Geo g(p);
-    const int id = st.ids[s] - (int)g.poff;
+    const int id = slot_id(st, s) - (int)g.poff;
     const int partner = st.bond[g.poff + id];
     if (partner < 0) return;
     const double u = uniform1(p.seed, *st.d_step, EDM_S_DISSOC + 2 * b, (uint64_t)id, 0);
@@ -2006,7 +2028,7 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
   __shared__ int delta_d[kDeltaList];
   __shared__ double rec_xy[2 * kRecCap];
   __shared__ double tile[kCdfTile];
-  __shared__ int32_t rec_id[kRecCap], n_contact[EDM_MAX_CAT], n_rec;
+  __shared__ int32_t rec_id[kRecCap], rec_slot[kRecCap], n_contact[EDM_MAX_CAT], n_rec;
   __shared__ int n_delta;
   const int r = blockIdx.x, tid = threadIdx.x;
   for (int k = tid; k < (int)(sizeof(EdmDynParams) / 16); k += blockDim.x)
@@ -2023,7 +2045,7 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
   const DeltaList sink{delta_cell, delta_d, &n_delta, st.grid_delta};
   ContactOut out = contact_out(st, p, r);
   out.count = n_contact;
-  const RecruitList rec{&n_rec, rec_id, rec_xy};
+  const RecruitList rec{&n_rec, rec_id, rec_slot, rec_xy};
   auto entry_at = [&](int q) -> int4* {  // entry q of the replica's list
     return q < kReactList ? entry + q : st.pl + poff + q;
   };
@@ -2055,7 +2077,8 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
           int rank = 0;
           for (int b = 0; b < n; ++b) rank += rec_id[b] < id;
           if (rank < take)
-            place_recruit<F64>(p, Geo(p), st, r, idx, id, rec_xy[2 * a], rec_xy[2 * a + 1], sink, D, plan.more[i],
+            place_recruit<F64>(p, Geo(p), st, r, idx, id, rec_slot[a], rec_xy[2 * a], rec_xy[2 * a + 1], sink, D,
+                               plan.more[i],
                                [&](int q) {
                                  const int k = q - (int)poff;
                                  return k >= 0 && k < n_listed ? entry_at(k) : (int4*)nullptr;

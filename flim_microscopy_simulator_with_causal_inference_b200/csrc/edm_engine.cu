@@ -77,8 +77,8 @@ struct LaunchShape {
 enum TunedKernel { TK_SCATTER = 0, TK_MOVE = 1, TK_CONTACTS = 2, TK_COUNT = 3 };
 constexpr int kMaxShapes = 8;
 constexpr LaunchShape kShapes[TK_COUNT][kMaxShapes] = {
-    // k_scatter: one slot per thread, then (3-4) two
-    {{256, 1}, {128, 1}, {512, 1}, {128, 1}, {256, 1}},
+    // k_scatter: one slot per thread, then (3) two and (4) four
+    {{256, 1}, {128, 1}, {512, 1}, {128, 1}, {128, 1}},
     // k_move: the second number bounds its registers (80 at 256 x 3 down to 32
     // at 128 x 16, with spills below 64): occupancy pays more than the spills
     {{256, 3}, {256, 4}, {128, 8}, {128, 10}, {128, 12}, {128, 16}, {256, 6}, {256, 8}},
@@ -131,6 +131,7 @@ struct EdmEngine {
   int npblk = 0, neblk = 0, nphblk = 0, npxblk = 0;
   // slot tiles of each of kTileSizes (the 256 table is pblk) for the tuned kernels
   int2* pblk_bs[kTileTables] = {};
+  SlotTile* ptile_bs[kTileTables] = {};
   int npblk_bs[kTileTables] = {};
   // launch shape of each tuned kernel (index into kShapes), tuning timings
   int shape[TK_COUNT] = {0, 0, 0};
@@ -154,7 +155,7 @@ struct EdmEngine {
   int64_t* counters = nullptr;
   uint32_t* status = nullptr;
   int64_t *d_step = nullptr, *d_pstep = nullptr, *d_batch_key = nullptr;
-  int32_t *rec_count = nullptr, *rec_id = nullptr, *bind_count = nullptr, *bind_ab = nullptr;
+  int32_t *rec_count = nullptr, *rec_id = nullptr, *rec_slot = nullptr, *bind_count = nullptr, *bind_ab = nullptr;
   double* rec_xy = nullptr;
   int64_t* bind_key = nullptr;
   int32_t *emit_id = nullptr, *emit_n = nullptr, *emit_nd = nullptr, *emit_acc = nullptr;
@@ -242,6 +243,7 @@ struct EdmEngine {
     s.d_step = d_step;
     s.rec_count = rec_count;
     s.rec_id = rec_id;
+    s.rec_slot = rec_slot;
     s.rec_xy = rec_xy;
     s.bind_count = bind_count;
     s.bind_key = bind_key;
@@ -688,13 +690,13 @@ struct EdmEngine {
     const int t = tile_index(sh.block);
     if (npblk_bs[t] == 0) return;
     const int nt = npblk_bs[t];
-    const int2* b = pblk_bs[t];
+    const SlotTile* b = ptile_bs[t];
     switch (shape[TK_SCATTER]) {  // the rows of kShapes[TK_SCATTER]
-      case 1: go(k_scatter<F64, 128, 1>, nt, 128, s, dp, b, nt, st); break;
-      case 2: go(k_scatter<F64, 512, 1>, nt, 512, s, dp, b, nt, st); break;
-      case 3: go(k_scatter<F64, 128, 2>, (nt + 1) / 2, 128, s, dp, b, nt, st); break;
-      case 4: go(k_scatter<F64, 256, 2>, (nt + 1) / 2, 256, s, dp, b, nt, st); break;
-      default: go(k_scatter<F64, 256, 1>, nt, 256, s, dp, b, nt, st); break;
+      case 1: go(k_scatter<F64, 128, 1>, nt, 128, s, b, nt, st); break;
+      case 2: go(k_scatter<F64, 512, 1>, nt, 512, s, b, nt, st); break;
+      case 3: go(k_scatter<F64, 128, 2>, (nt + 1) / 2, 128, s, b, nt, st); break;
+      case 4: go(k_scatter<F64, 128, 4>, (nt + 3) / 4, 128, s, b, nt, st); break;
+      default: go(k_scatter<F64, 256, 1>, nt, 256, s, b, nt, st); break;
     }
   }
 
@@ -901,6 +903,9 @@ struct EdmEngine {
   // call wait for both.  Errors surface at the call's cudaGetLastError or at
   // the capture's end.
   cudaStream_t phot_stream = nullptr, scope_stream = nullptr;
+  // the current photon batch may name particles whose slots the sorts do not
+  // track (edm_set_photons, or a state set after the batch was made)
+  bool host_batch = false;
   bool phot_uses_cells = true;  // some replica's FRET is by proximity (a cell-list search)
   cudaEvent_t ev_phot_fork = nullptr, ev_phot_join = nullptr, ev_scope_join = nullptr;
   bool phot_pending = false, scope_pending = false;
@@ -1210,6 +1215,7 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   ALLOC(E->d_batch_key, 1);
   ALLOC(E->rec_count, n_replicas);
   ALLOC(E->rec_id, (size_t)n_replicas * kRecCap);
+  ALLOC(E->rec_slot, (size_t)n_replicas * kRecCap);
   ALLOC(E->rec_xy, (size_t)n_replicas * kRecCap * 2);
   ALLOC(E->bind_count, n_replicas);
   ALLOC(E->bind_key, (size_t)n_replicas * kBindCap);
@@ -1272,8 +1278,17 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
     std::vector<int2> pt = tiles(pfirst, pcount, kTileSizes[t]);
     E->npblk_bs[t] = (int)pt.size();
     ALLOC(E->pblk_bs[t], std::max<size_t>(1, pt.size()));
-    if (!pt.empty())
+    std::vector<SlotTile> st;
+    for (const int2& b : pt) {
+      const EdmDynParams& p = E->hdp[b.x];
+      st.push_back({b.y, (int32_t)(p.particle_offset + p.n_particles), (int32_t)p.cell_offset,
+                    (int32_t)(p.cell_offset + (int64_t)p.nx * p.ny)});
+    }
+    ALLOC(E->ptile_bs[t], std::max<size_t>(1, pt.size()));
+    if (!pt.empty()) {
       CUDA_TRY(cudaMemcpy(E->pblk_bs[t], pt.data(), sizeof(int2) * pt.size(), cudaMemcpyHostToDevice));
+      CUDA_TRY(cudaMemcpy(E->ptile_bs[t], st.data(), sizeof(SlotTile) * st.size(), cudaMemcpyHostToDevice));
+    }
   }
   E->pblk = E->pblk_bs[1];
   E->npblk = E->npblk_bs[1];
@@ -1441,7 +1456,8 @@ __global__ void __launch_bounds__(kSpThreads) k_sp_write(uint32_t* __restrict__ 
 template <bool F64>
 __global__ void k_set_state(const EdmDynParams* __restrict__ P, const int2* __restrict__ blk, const double* pos,
                             const int32_t* species, const uint8_t* alive, void* pos_post, short2* lo_post,
-                            int32_t* cell_post, uint8_t* flags, int32_t* ids, int32_t* slot_of_id, int32_t* cnt) {
+                            int32_t* cell_post, uint8_t* flags, int32_t* ids, int32_t* slot_of_id, int32_t* cnt,
+                            const uint8_t* has_dye, int track_all) {
   const Tile t = tile_of(blk);
   const EdmDynParams& p = P[t.r];
   const int64_t s = t.s;
@@ -1462,30 +1478,37 @@ __global__ void k_set_state(const EdmDynParams* __restrict__ P, const int2* __re
   const int c = cx * g.ny + cy;
   cell_post[s] = c;
   flags[s] = fl_make(species[s], alive[s] != 0);
-  ids[s] = (int32_t)s;
+  ids[s] = (int32_t)s | (track_all || (has_dye && has_dye[s]) ? kTracked : 0);
   slot_of_id[s] = (int32_t)s;
   atomicAdd(&cnt[g.cbase + (alive[s] ? c : g.grave)], 1);
 }
 
+// By slot: the slot's particle gets its position and flags, the particle with
+// the slot's own number its bond.
 template <bool F64>
 __global__ void k_get_state(const EdmDynParams* __restrict__ P, const int2* __restrict__ blk, const void* pos_post,
-                            const short2* lo_post, const int32_t* cell_post, const uint8_t* flags, const int32_t* slot_of_id,
+                            const short2* lo_post, const int32_t* cell_post, const uint8_t* flags, const int32_t* ids,
                             const int32_t* bond, double* pos, int32_t* species, uint8_t* alive, int32_t* bond_local) {
   const Tile t = tile_of(blk);
   const EdmDynParams& p = P[t.r];
-  const int64_t id = t.s;
-  if (id >= p.particle_offset + p.n_particles) return;
+  const int64_t s = t.s;
+  if (s >= p.particle_offset + p.n_particles) return;
   const Geo g(p);
-  const int64_t s = slot_of_id[id];
+  const int64_t id = ids[s] & ~kTracked;
   double x, y;
   abs_pos<F64>(pos_post, lo_post, cell_post, s, g, x, y);
-  pos[2 * id] = x;
-  pos[2 * id + 1] = y;
+  reinterpret_cast<double2*>(pos)[id] = make_double2(x, y);
   const uint8_t f = flags[s];
   species[id] = fl_species(f);
   alive[id] = fl_alive(f) ? 1 : 0;
-  const int b = bond[id];
-  bond_local[id] = b >= 0 ? (int32_t)(b - p.particle_offset) : -1;
+  const int b = bond[s];
+  bond_local[s] = b >= 0 ? (int32_t)(b - p.particle_offset) : -1;
+}
+
+// The whole map from particles to slots (the sorts keep the tracked part only).
+__global__ void k_slot_map(const int32_t* __restrict__ ids, int32_t* __restrict__ slot_of_id, int64_t n) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x)
+    slot_of_id[ids[s] & ~kTracked] = (int32_t)s;
 }
 
 __global__ void k_narrow_i8(const int32_t* __restrict__ in, int8_t* __restrict__ out, int64_t n) {
@@ -1509,6 +1532,7 @@ extern "C" {
 int edm_set_state(EdmEngine* E, const EdmHostState* st, void* stream) {
   if (!E || !st || st->n != E->N) return fail(EDM_EINVAL, "edm_set_state: size mismatch");
   E->cells_valid = false;
+  E->host_batch = true;
   cudaStream_t s = (cudaStream_t)stream;
   CUDA_TRY(cudaSetDevice(E->device));
   const int64_t N = E->N;
@@ -1539,11 +1563,11 @@ int edm_set_state(EdmEngine* E, const EdmHostState* st, void* stream) {
     if (E->f64)
       k_set_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, dpos, E->st_sp, E->st_alive, E->pos_post, E->lo_post,
                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
-                                                    E->cnt);
+                                                    E->cnt, E->has_phot ? E->has_dye : nullptr, E->hdp[0].n_bind > 0);
     else
       k_set_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, dpos, E->st_sp, E->st_alive, E->pos_post, E->lo_post,
                                                      E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
-                                                     E->cnt);
+                                                     E->cnt, E->has_phot ? E->has_dye : nullptr, E->hdp[0].n_bind > 0);
     k_bond_to_global<<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->bond);
   }
   // emitters: particles carrying a dye, in particle order per replica.  When
@@ -1610,11 +1634,11 @@ int edm_get_state(EdmEngine* E, EdmHostState* st, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_get_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                    E->slot_of_id[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
+                                                    E->ids[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
                                                     E->st_bond);
     else
       k_get_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                     E->slot_of_id[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
+                                                     E->ids[E->cur], E->bond, E->st_pos, E->st_sp, E->st_alive,
                                                      E->st_bond);
   }
   CUDA_TRY(cudaGetLastError());
@@ -1664,6 +1688,7 @@ int edm_install_state(EdmEngine* E, void* stream) {
   const int64_t N = E->N;
   const EdmEngine::Xfer& in = E->in;
   E->cells_valid = false;
+  E->host_batch = true;
   // in order on `stream`: as edm_set_state, from the staging
   CUDA_TRY(cudaStreamWaitEvent(s, E->ev_staged, 0));
   CUDA_TRY(cudaMemcpyAsync(E->bond, in.bond, sizeof(int32_t) * N, cudaMemcpyDeviceToDevice, s));
@@ -1676,11 +1701,11 @@ int edm_install_state(EdmEngine* E, void* stream) {
     if (E->f64)
       k_set_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, in.pos, in.sp, in.alive, E->pos_post, E->lo_post,
                                                     E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
-                                                    E->cnt);
+                                                    E->cnt, E->has_phot ? E->has_dye : nullptr, E->hdp[0].n_bind > 0);
     else
       k_set_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, in.pos, in.sp, in.alive, E->pos_post, E->lo_post,
                                                      E->cell_post, E->flags[E->cur], E->ids[E->cur], E->slot_of_id[E->cur],
-                                                     E->cnt);
+                                                     E->cnt, E->has_phot ? E->has_dye : nullptr, E->hdp[0].n_bind > 0);
     k_bond_to_global<<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->bond);
   }
   CUDA_TRY(cudaEventRecord(E->ev_in_free, s));
@@ -1714,10 +1739,10 @@ int edm_get_state_async(EdmEngine* E, EdmHostState* st, void* stream) {
   if (E->npblk > 0) {
     if (E->f64)
       k_get_state<true><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                    E->slot_of_id[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
+                                                    E->ids[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
     else
       k_get_state<false><<<E->npblk, kBlock, 0, s>>>(E->dp, E->pblk, E->pos_post, E->lo_post, E->cell_post, E->flags[E->cur],
-                                                     E->slot_of_id[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
+                                                     E->ids[E->cur], E->bond, out.pos, out.sp, out.alive, out.bond);
   }
   CUDA_TRY(cudaMemcpyAsync(out.ctmc, E->ctmc, N, cudaMemcpyDeviceToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(out.bleached, E->bleached, N, cudaMemcpyDeviceToDevice, s));
@@ -1775,6 +1800,7 @@ int edm_photon_step(EdmEngine* E, void* stream) {
   if (!E || !E->has_phot) return fail(EDM_EINVAL, "edm_photon_step: engine has no photophysics");
   CUDA_TRY(cudaSetDevice(E->device));
   E->enqueue_photons((cudaStream_t)stream);
+  E->host_batch = false;
   CUDA_TRY(cudaGetLastError());
   return EDM_OK;
 }
@@ -1809,7 +1835,9 @@ int edm_get_photons(EdmEngine* E, int32_t replica, int32_t* particle_idx, double
 int edm_scope_process(EdmEngine* E, void* stream) {
   if (!E || !E->has_scope) return fail(EDM_EINVAL, "edm_scope_process: engine has no microscope");
   CUDA_TRY(cudaSetDevice(E->device));
-  E->enqueue_photon_positions((cudaStream_t)stream);  // the batch may come from the host
+  if (E->host_batch && E->N > 0)
+    k_slot_map<<<148 * 8, 256, 0, (cudaStream_t)stream>>>(E->ids[E->cur], E->slot_of_id[E->cur], E->N);
+  E->enqueue_photon_positions((cudaStream_t)stream);
   E->enqueue_scope((cudaStream_t)stream);
   CUDA_TRY(cudaGetLastError());
   return EDM_OK;
@@ -1828,6 +1856,7 @@ int edm_set_photons(EdmEngine* E, int32_t replica, const int32_t* particle_idx, 
     CUDA_TRY(cudaMemcpyAsync(E->ph_ch + o, channel, n, cudaMemcpyHostToDevice, s));
     if (is_fret) CUDA_TRY(cudaMemcpyAsync(E->ph_fret + o, is_fret, n, cudaMemcpyHostToDevice, s));
   }
+  E->host_batch = true;
   std::vector<int64_t> counts(E->R, 0);
   counts[replica] = n;
   CUDA_TRY(cudaMemcpyAsync(E->ph_count, counts.data(), sizeof(int64_t) * E->R, cudaMemcpyHostToDevice, s));
@@ -1841,6 +1870,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
   if (with_photons && !E->has_scope) return fail(EDM_EINVAL, "edm_pipeline_steps: no photophysics/microscope");
   CUDA_TRY(cudaSetDevice(E->device));
   cudaStream_t s = (cudaStream_t)stream;
+  if (with_photons && n_steps > 0) E->host_batch = false;
   auto body = [&](cudaStream_t st) {
     E->enqueue_dynamics(st);  // beside the previous step's photon and detection passes
     if (with_photons) E->enqueue_photons_beside(st);
@@ -2314,7 +2344,8 @@ int edm_get_cells(EdmEngine* E, int32_t replica, int32_t* cell_start, int32_t* m
   for (int64_t i = 0; i < p.n_particles; ++i) cell_start[cells[i] + 1] += 1;
   for (int64_t c = 0; c < nc; ++c) cell_start[c + 1] += cell_start[c];
   std::vector<int32_t> fill(cell_start, cell_start + nc);
-  for (int64_t i = 0; i < p.n_particles; ++i) members[fill[cells[i]]++] = ids[i] - (int32_t)p.particle_offset;
+  for (int64_t i = 0; i < p.n_particles; ++i)
+    members[fill[cells[i]]++] = (ids[i] & ~kTracked) - (int32_t)p.particle_offset;
   return EDM_OK;
 }
 

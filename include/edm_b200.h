@@ -430,7 +430,7 @@ int edm_ground_truth(EdmEngine* eng, double* fret_E, double* tau_DA,
 int edm_autotune(EdmEngine* eng, int32_t steps_per_shape, int32_t retune, void* stream);
 /* The launch shape in use per tuned kernel: shapes[k][4] = (threads per block,
  * minimum blocks per SM, candidates, chosen candidate; k_scatter candidates
- * 3-4 give a thread two slots, the others one; k_contacts candidates 0-1
+ * 3 and 4 give a thread two and four slots, the others one; k_contacts candidates 0-1
  * gather a tile's sweepers per block, 2-7 sweep a global sweeper list, each
  * with 4, 8 or 16 lanes per sweeper), ms[k][2] = (time of the default shape, time of the chosen shape) from
  * the last tuning (0 if not tuned).  Either pointer may be NULL.  Returns the

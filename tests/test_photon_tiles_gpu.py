@@ -61,3 +61,23 @@ def test_proximity_fret_in_graph_chunks():
         P.orc.bd_step()
     assert np.array_equal(P.eng.flim(0), P.orc.flim)
     compare_state(P.gpu_state(), P.orc, F64_TOL)
+
+
+@pytest.mark.gpu
+def test_host_batch_of_particles_without_dye():
+    """A batch from the host may name any particle, the sorts keep the slots of
+    dye carriers only: detection after 9 steps equals detection by an engine
+    that was given the state at that point."""
+    P, Q = Pair(_system(200), precision=64), Pair(_system(200), precision=64)
+    P.eng.dynamics_step(9)
+    g = P.gpu_state()
+    st = P.state
+    Q.eng.set_state(g["positions"], g["species"], g["alive"], g["bond"], g["has_dye"], st.dye_type_id, g["ctmc"],
+                    g["bleached"])
+    pid = np.flatnonzero(~st.has_dye)[:300].astype(np.int32)
+    for X in (P, Q):
+        X.eng.set_photons(0, pid, np.linspace(0.0, 2.0e-8, pid.size), np.zeros(pid.size, np.int8),
+                          np.zeros(pid.size, np.uint8), batch_key=5)
+        X.eng.scope_process()
+    a, b = P.eng.flim(0), Q.eng.flim(0)
+    assert a.sum() > 0 and np.array_equal(a, b)
