@@ -773,9 +773,11 @@ struct EdmEngine {
     tune_mark(TK_SCATTER, 0, s);
     launch_scatter<F64>(st, s);
     tune_mark(TK_SCATTER, 1, s);
-    // it reads the flags and the map from particles to slots, which the sort
-    // writes to their other copies, and the positions the move rewrites
-    join_photons(s);
+    // a photon pass begun after the previous step reads the flags and the map
+    // from particles to slots, which the sort writes to their other copies, and
+    // the positions the move rewrites
+    if (photons_due) enqueue_photons_beside(s, true);
+    else join_photons(s);
     mark(2, s);
     tune_mark(TK_MOVE, 0, s);
     launch_move<F64>(st, s);
@@ -789,6 +791,9 @@ struct EdmEngine {
     for (size_t i = 0; i < passes.size(); ++i) {
       const Pass& ps = passes[i];
       if (pass_prof) cudaEventRecord(pass_prof[i], s);
+      // the photon pass reads the flags and bonds that the reactions change
+      if (photons_late && ps.kind != P_CONTACTS && ps.kind != P_DRAWS && ps.kind != P_ADAPT && ps.kind != P_MERGE)
+        join_photons(s);
       switch (ps.kind) {
         case P_BIND_CAND: go(k_bind_candidates<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
         case P_BIND_APPLY: go(k_bind_apply<F64>, rb, 128, s, dp, R, st, ps.index); break;
@@ -842,6 +847,7 @@ struct EdmEngine {
         case P_MERGE: go(k_grid_merge, gm > 0 ? gm : 1, 256, s, grid_cnt, grid_delta, n_grid); break;
       }
     }
+    if (photons_late) join_photons(s);  // before the next sort rewrites what it reads
     if (pass_prof) cudaEventRecord(pass_prof[passes.size()], s);
     if (!react_ticket) go(k_step_inc, 1, 1, s, d_step);  // k_react does it
     cells_valid = true;
@@ -863,8 +869,13 @@ struct EdmEngine {
   }
 
   template <bool F64>
-  void enqueue_photons_t(cudaStream_t s) {
-    const DevState st = dev_state();
+  void enqueue_photons_t(cudaStream_t s, bool sorted) {
+    DevState st = dev_state();
+    if (sorted) {  // the step's final positions as the next step's sort has laid them out
+      st.pos_post = pos_pre;
+      st.lo_post = lo_pre;
+      st.cell_post = cell_pre;
+    }
     const PhotState ph = phot_state();
     if (neblk == 0) {
       launch(k_phot_none, 1, 256, s, false, R, ph);
@@ -874,9 +885,9 @@ struct EdmEngine {
     launch(k_phot_write<F64>, neblk, kBlock, s, true, dp, pp, eblk, st, ph, counters);
   }
 
-  void enqueue_photons(cudaStream_t s) {
-    if (f64) enqueue_photons_t<true>(s);
-    else enqueue_photons_t<false>(s);
+  void enqueue_photons(cudaStream_t s, bool sorted = false) {
+    if (f64) enqueue_photons_t<true>(s, sorted);
+    else enqueue_photons_t<false>(s, sorted);
   }
 
   void enqueue_scope(cudaStream_t s) {
@@ -894,14 +905,22 @@ struct EdmEngine {
   }
 
   // A step's photon pass and detection pass beside the next step, each on a
-  // stream of its own.  The photon pass reads the step's final state: the next
-  // step's bucket scan and sort may run beside it, its move may not
-  // (enqueue_dynamics joins it before the move; with proximity FRET, which
-  // reads the bucket starts, before the scan).  The detection pass reads only the
-  // photon records, which carry their positions: the next step's dynamics run
-  // beside it, the next photon pass waits for it.  A census and the end of the
-  // call wait for both.  Errors surface at the call's cudaGetLastError or at
-  // the capture's end.
+  // stream of its own.  The photon pass reads the step's final state.  It starts
+  // after the step and runs beside the next one's scan and sort, joined before
+  // the move; or (photons_late) it waits until the next step's sort has copied
+  // that state and runs beside the move and the contact search, joined before
+  // the first pass that changes flags or bonds.  Two launches of latency, it
+  // takes 12 us: the first window is 5 us in a small system, the second 14, and
+  // a step of 5,000 slots falls from 31.3 to 28.5 us, of 207,000 from 46.4 to
+  // 42.6; in a large system it competes with the move instead (1.9M slots 202
+  // against 206 us, 4.7M slots 324 against 332).  The last step of a call, a
+  // recorded step (its census reads the photon state) and proximity FRET (a
+  // search over the step's own cell list) run it right after the step.  The
+  // detection pass reads only the photon records, which carry their positions:
+  // the next step's dynamics run beside it, the next photon pass waits for it.
+  // A census and the end of the call wait for both.  Errors surface at the
+  // call's cudaGetLastError or at the capture's end.
+  bool photons_late = false;
   cudaStream_t phot_stream = nullptr, scope_stream = nullptr;
   // the current photon batch may name particles whose slots the sorts do not
   // track (edm_set_photons, or a state set after the batch was made)
@@ -909,11 +928,13 @@ struct EdmEngine {
   bool phot_uses_cells = true;  // some replica's FRET is by proximity (a cell-list search)
   cudaEvent_t ev_phot_fork = nullptr, ev_phot_join = nullptr, ev_scope_join = nullptr;
   bool phot_pending = false, scope_pending = false;
-  void enqueue_photons_beside(cudaStream_t s) {
+  bool photons_due = false;
+  void enqueue_photons_beside(cudaStream_t s, bool sorted) {
+    photons_due = false;
     cudaEventRecord(ev_phot_fork, s);
     cudaStreamWaitEvent(phot_stream, ev_phot_fork, 0);
     if (scope_pending) cudaStreamWaitEvent(phot_stream, ev_scope_join, 0);  // the records are free again
-    enqueue_photons(phot_stream);
+    enqueue_photons(phot_stream, sorted);
     cudaEventRecord(ev_phot_join, phot_stream);
     cudaStreamWaitEvent(scope_stream, ev_phot_join, 0);
     enqueue_scope(scope_stream);
@@ -927,6 +948,7 @@ struct EdmEngine {
     pdl_chain = false;
   }
   void join_beside(cudaStream_t s) {
+    if (photons_due) enqueue_photons_beside(s, false);
     join_photons(s);
     if (!scope_pending) return;
     cudaStreamWaitEvent(s, ev_scope_join, 0);
@@ -1234,6 +1256,7 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
       for (int f = 0; f < q.n_fret && f < EDM_MAX_FRET; ++f)
         if (q.fret[f].mode != 0) E->phot_uses_cells = true;
   }
+  E->photons_late = !E->phot_uses_cells && np <= (1 << 20);
   if (E->has_scope) {
     CUDA_TRY(cudaStreamCreateWithFlags(&E->phot_stream, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&E->scope_stream, cudaStreamNonBlocking));
@@ -1873,7 +1896,10 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
   if (with_photons && n_steps > 0) E->host_batch = false;
   auto body = [&](cudaStream_t st) {
     E->enqueue_dynamics(st);  // beside the previous step's photon and detection passes
-    if (with_photons) E->enqueue_photons_beside(st);
+    if (with_photons) {
+      if (E->photons_late) E->photons_due = true;
+      else E->enqueue_photons_beside(st, false);
+    }
     if (E->rec_cap > 0) {
       E->join_beside(st);  // the census reads the photon state and the detection counters
       E->enqueue_census(st, E->rec_ring, E->rec_cap, with_photons != 0);
