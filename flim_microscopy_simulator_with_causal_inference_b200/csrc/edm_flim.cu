@@ -400,9 +400,13 @@ struct LaneRng {
     s2 = (uint32_t)b;
     s3 = (uint32_t)(b >> 32) | ((a | b) == 0ull ? 1u : 0u);  // the all-zero state is the one fixed point
   }
-  __device__ __forceinline__ uint32_t next() {
-    const uint32_t sum = s0 + s3;
-    const uint32_t out = __funnelshift_l(sum, sum, 7) + s0;
+  // The generator's two additions go through a multiply-add by `one` (1, from a
+  // kernel argument, so that it stays one): the photon loop is bound by the
+  // integer ALU, whose rotations and exclusive ors have no other home, while
+  // the multiply-add pipe has room.
+  __device__ __forceinline__ uint32_t next(uint32_t one = 1u) {
+    const uint32_t sum = s0 * one + s3;
+    const uint32_t out = __funnelshift_l(sum, sum, 7) * one + s0;
     const uint32_t t = s1 << 9;
     s2 ^= s0;
     s3 ^= s1;
@@ -462,6 +466,32 @@ __device__ __forceinline__ uint32_t poisson(float mu, Rng& rng) {
   return mu < 10.0f ? poisson_small(mu, rng.uniform()) : poisson_ptrs(mu, rng);
 }
 
+// A photon's random word w: its top bits pick the alias cell, its low 24 bits
+// are compared with the cell's threshold.  w * 256 + 255 holds the top byte in
+// its high word and the low 24 bits over a full byte in its low word, in one
+// wide multiply-add: below a table entry (threshold << 8 | alias) exactly when
+// the 24 bits are below the threshold.
+__device__ __forceinline__ uint64_t split_word(uint32_t w) { return (uint64_t)w * 256u + 255u; }
+template <int NB>
+__device__ __forceinline__ uint32_t cell_of(uint64_t w) {
+  return (uint32_t)(w >> 32) >> (NB == 256 ? 0 : 1);
+}
+template <int NB>
+__device__ __forceinline__ uint32_t bin_of(uint64_t w, uint32_t e) {
+  return (uint32_t)w < e ? cell_of<NB>(w) : e & 0xFFu;
+}
+
+// Word i of the shared table at `base`, and one more count in word i: the byte
+// address by a multiply-add with `four` (a kernel argument), as above.
+__device__ __forceinline__ uint32_t load_word(uint32_t base, uint32_t i, uint32_t four) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(i * four + base));
+  return v;
+}
+__device__ __forceinline__ void count_word(uint32_t base, uint32_t i, uint32_t four) {
+  asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(i * four + base) : "memory");
+}
+
 // A warp takes 32 consecutive pixels at a time (grid-stride).  The counts
 // n_b ~ Poisson(mu_b), mu_b = A h_free[b] y_free + B h_bound[b] y_bound, are
 // drawn through the identity "Poisson total, then independent categorical
@@ -475,26 +505,41 @@ __device__ __forceinline__ uint32_t poisson(float mu, Rng& rng) {
 //      group's pixels), four per lane per round so table loads and
 //      shared-memory atomics overlap, and the pixel's histogram leaves in
 //      512-byte coalesced stores.
-__global__ void __launch_bounds__(256, 4) k_hist(EdmFlimParams p, const float* __restrict__ I /*[R][2][256*256]*/,
+// Bound: the integer ALU and the shared-memory wavefronts of a photon (xoshiro
+// word, table word, histogram add), not the 1 KB a pixel writes.  A table entry
+// is one 32-bit word (two made 6.6 wavefronts of bank conflicts per 32 photons,
+// one 4.7), its test one wide multiply-add, additions and addresses go through
+// the multiply-add pipe, and blocks of two warps spread one field of view's
+// 2,048 warps evenly: 256 fields of 256 bins in 11.0 ms against 12.8, the same
+// counts bit for bit.
+constexpr int kHistWarps = 2;
+template <int NB>
+__global__ void __launch_bounds__(32 * kHistWarps, 40 / kHistWarps) k_hist(EdmFlimParams p, const float* __restrict__ I /*[R][2][256*256]*/,
                                                  const int2* __restrict__ alias, const double* __restrict__ sums,
-                                                 uint32_t* __restrict__ hist, double* __restrict__ tau_expected) {
-  __shared__ int2 tab[2][256];
-  __shared__ __align__(16) uint32_t wh[8][256];
-  const int nb = p.n_bins;
-  for (int i = threadIdx.x; i < 2 * nb; i += blockDim.x) tab[i / nb][i % nb] = alias[i];
+                                                 uint32_t* __restrict__ hist, double* __restrict__ tau_expected,
+                                                 uint32_t one, uint32_t four) {
+  __shared__ uint32_t tab[2][NB];
+  __shared__ __align__(16) uint32_t wh[kHistWarps][NB];
+  constexpr int nb = NB;
+  for (int i = threadIdx.x; i < 2 * nb; i += blockDim.x) {
+    const int2 a = alias[i];
+    // a cell that always keeps its bin names it as its alias too
+    tab[i / nb][i % nb] = a.x >= 1 << 24 ? (uint32_t)(i % nb) : ((uint32_t)a.x << 8) | (uint32_t)a.y;
+  }
   __syncthreads();
   const double Tf = sums[0], Sf = sums[1], Tb = sums[2], Sb = sums[3];
   const unsigned FULL = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int shift = nb == 256 ? 24 : 25;  // top bits of a word pick the cell
   uint32_t* h = wh[warp];
+  const uint32_t hb = smem_u32(h);
   const uint32_t npx = (uint32_t)kDim * kDim;
   const uint32_t total = npx * (uint32_t)p.n_replicas;
   // pixel index over all replicas: at most 4096 x 2^16 = 2^28, so 32 bits
   // hold it and the replica / pixel split is a shift and a mask; a group of
   // 32 aligned pixels never straddles two replicas
   static_assert(kDim * kDim == 1 << 16, "pixel split assumes 2^16 pixels per replica");
-  for (uint32_t g0 = (blockIdx.x * 8u + (uint32_t)warp) * 32u; g0 < total; g0 += gridDim.x * 8u * 32u) {
+  for (uint32_t g0 = (blockIdx.x * kHistWarps + (uint32_t)warp) * 32u; g0 < total;
+       g0 += gridDim.x * kHistWarps * 32u) {
     const uint32_t r = g0 >> 16;
     const uint64_t seed = edm_flim_replica_seed(p.seed, (int32_t)r);
     // ---- 1. this lane's pixel of the group: totals and expected lifetime
@@ -530,25 +575,25 @@ __global__ void __launch_bounds__(256, 4) k_hist(EdmFlimParams p, const float* _
       // the free component's photons, then the bound component's, each
       // from its own alias table
       for (int c = 0; c < 2; ++c) {
-        const int2* tc = tab[c];
+        const uint32_t tc = smem_u32(tab[c]);
         const int n = c == 0 ? nf : na - nf;
         int i = lane;
         for (; i + 96 < n; i += 128) {
-          uint32_t w[4];
-          int2 e[4];
+          uint64_t w[4];
+          uint32_t e[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) w[k] = rng.next();
+          for (int k = 0; k < 4; ++k) w[k] = split_word(rng.next(one));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) e[k] = tc[w[k] >> shift];
+          for (int k = 0; k < 4; ++k) e[k] = load_word(tc, cell_of<NB>(w[k]), four);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            atomicAdd(&h[(int)(w[k] & 0xFFFFFFu) < e[k].x ? (int)(w[k] >> shift) : e[k].y], 1u);
+          for (int k = 0; k < 4; ++k) count_word(hb, bin_of<NB>(w[k], e[k]), four);
         }
-        for (; i < n; i += 32) {
-          const uint32_t w = rng.next();
-          const int2 e = tc[w >> shift];
-          atomicAdd(&h[(int)(w & 0xFFFFFFu) < e.x ? (int)(w >> shift) : e.y], 1u);
-        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)  // at most three are left to a lane
+          if (i + 32 * k < n) {
+            const uint64_t w = split_word(rng.next(one));
+            count_word(hb, bin_of<NB>(w, load_word(tc, cell_of<NB>(w), four)), four);
+          }
       }
       __syncwarp();
       uint4* out = (uint4*)(hist + (size_t)gpx * (size_t)nb);
@@ -705,7 +750,9 @@ int edm_flim_create(const EdmFlimParams* params, int32_t device, EdmFlim** out) 
   if (e == cudaSuccess) {
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hist, 256, 0);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, params->n_bins == 256 ? k_hist<256> : k_hist<128>,
+                                                        32 * kHistWarps, 0);
     if (e == cudaSuccess) F->hist_blocks = std::max(1, sms * std::max(1, per_sm));
   }
   if (e == cudaSuccess) {
@@ -771,8 +818,10 @@ int edm_flim_histograms(EdmFlim* F, int32_t with_tau, void* stream) {
   FL_TRY(cudaSetDevice(F->device));
   const EdmFlimParams& p = F->p;
   const size_t total_px = (size_t)p.n_replicas * kDim * kDim;
-  const unsigned blocks = (unsigned)std::min<size_t>((total_px + 7) / 8, (size_t)F->hist_blocks);
-  k_hist<<<blocks, 256, 0, (cudaStream_t)stream>>>(p, F->I, F->alias, F->sums, F->hist, with_tau ? F->tau : nullptr);
+  const unsigned blocks = (unsigned)std::min<size_t>((total_px / 32 + kHistWarps - 1) / kHistWarps, (size_t)F->hist_blocks);
+  const auto kernel = p.n_bins == 256 ? k_hist<256> : k_hist<128>;
+  kernel<<<blocks, 32 * kHistWarps, 0, (cudaStream_t)stream>>>(p, F->I, F->alias, F->sums, F->hist, with_tau ? F->tau : nullptr, 1u,
+                                                  4u);
   FL_TRY(cudaGetLastError());
   return EDM_OK;
 }
