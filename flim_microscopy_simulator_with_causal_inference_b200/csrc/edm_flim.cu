@@ -51,9 +51,11 @@ constexpr int kDim = 256;                  // pixels per side; the GEMM tiles as
 constexpr int kBM = 128;                   // UMMA M per CTA
 constexpr int kBK = 64;                    // K per stage: one 128-byte swizzle atom of bf16
 constexpr int kStageA = kBM * kBK * 2;     // 16 KB
-constexpr int kStageB = kDim * kBK * 2;    // 32 KB
+constexpr int kBN = 64;                    // UMMA N per CTA
+constexpr int kStageB = kBN * kBK * 2;     // 8 KB
 constexpr int kStage = kStageA + kStageB;  // multiple of 1024: every tile stays swizzle-aligned
-constexpr int kGemmSmem = 2 * kStage + 1024 + 256;
+constexpr int kGemmStages = 4;
+constexpr int kGemmSmem = kGemmStages * kStage + 1024 + 256;
 constexpr uint32_t kWaitLimit = 1u << 22;  // bounded mbarrier polls before reporting an error
 constexpr int kK1 = 512, kK2 = 768;        // K of the two GEMMs (hi/lo concatenations)
 
@@ -104,7 +106,7 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
 // kind::f16 instruction descriptor: FP32 D (bits 4-5 = 1), BF16 A (7-9 = 1)
 // and B (10-12 = 1), both K-major, N/8 in bits 17-22, M/16 in bits 24-28.
 constexpr uint32_t kIdesc =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kDim >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc) {
   asm volatile(
@@ -129,9 +131,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 }
 
 struct GemmArgs {
-  int k_chunks;            // K / 64
+  int sections;            // 256-wide parts of K (the hi/lo concatenations)
   int a_kwrap;             // A's K coordinate taken modulo this (0: no wrap)
   int a_batched, b_batched;
+  int band_a;              // the operand that is the PSF band: 1 A (its rows are this tile's), 0 B
+  int taps;                // the band's half-width
   int split_transpose;     // 0: FP32 out[batch][row][col]; 1: bf16 [hi|lo|hi] transposed into b2
   float* out;
   __nv_bfloat16* b2;
@@ -139,27 +143,35 @@ struct GemmArgs {
 };
 
 // D[batch] = A[batch] (256 x K) . B[batch]^T (256 x K), both operands
-// K-major bf16.  One CTA per 128-row M tile and batch, 128 threads: thread 0
-// streams K in 64-wide stages by TMA (double-buffered, mbarrier-tracked) and
-// issues the MMAs; then each warp reads its 32 accumulator lanes (rows) from
-// tensor memory and writes them out.
+// K-major bf16.  One CTA per 128 x 64 tile and batch, 128 threads: thread 0
+// streams K in 64-wide stages by TMA (a ring of kGemmStages, mbarrier-tracked)
+// and issues the MMAs; then each warp reads its 32 accumulator lanes (rows)
+// from tensor memory and writes them out.
+//
+// These products are small (256 x 256 per map), so a CTA's time is the latency
+// of its loads.  One operand is the PSF band, zero farther than `taps` from the
+// diagonal: the 64-wide chunks of each section that hold no nonzero of this
+// tile's band rows are left out (a sum of exact zeros), and the stages in
+// flight cover the rest.  Eight CTAs per map instead of two with 256 columns
+// each and two stages: 15.8 to 7 and 8 us for the two products of one field of view.
 __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUtensorMap tmA,
                                                    const __grid_constant__ CUtensorMap tmB, GemmArgs args) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = (uint64_t*)(smem + 2 * kStage);  // full[2], empty[2], done
-  uint32_t* tmem_slot = (uint32_t*)(bars + 6);
-  const int m_tile = blockIdx.x, batch = blockIdx.y;
+  uint64_t* bars = (uint64_t*)(smem + kGemmStages * kStage);  // full[stages], empty[stages], done
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * kGemmStages + 1);
+  const int m_tile = blockIdx.x & 1, n_tile = blockIdx.x >> 1, batch = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[2]), done = smem_u32(&bars[4]);
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kGemmStages]),
+                 done = smem_u32(&bars[2 * kGemmStages]);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 5; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    for (int i = 0; i < 2 * kGemmStages + 1; ++i) mbar_init(smem_u32(&bars[i]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {  // 256 columns x 128 lanes of FP32 accumulator
+  if (warp == 0) {  // kBN columns x 128 lanes of FP32 accumulator
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kDim)
+                 "r"(kBN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -167,24 +179,26 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  edm::pdl_enter();  // the operands come from the kernel before
 
   if (threadIdx.x == 0) {
-    const int KC = args.k_chunks;
+    const int row0 = args.band_a ? m_tile * kBM : n_tile * kBN, rows = args.band_a ? kBM : kBN;
+    const int c_lo = max(0, row0 - args.taps) / kBK, c_hi = min(kDim - 1, row0 + rows - 1 + args.taps) / kBK;
+    const int per = c_hi - c_lo + 1, n = args.sections * per;
     bool ok = true;
-    auto load = [&](int kc) {
-      const int s = kc & 1;
+    auto load = [&](int t) {
+      const int s = t % kGemmStages;
       const uint32_t a_dst = smem_u32(smem + s * kStage), b_dst = a_dst + kStageA;
       const uint32_t bar = full0 + 8 * s;
+      const int k = (t / per) * kDim + (c_lo + t % per) * kBK;
       mbar_expect_tx(bar, kStage);
-      const int ka = args.a_kwrap > 0 ? (kc * kBK) % args.a_kwrap : kc * kBK;
-      tma_load_3d(a_dst, &tmA, ka, m_tile * kBM, args.a_batched ? batch : 0, bar);
-      tma_load_3d(b_dst, &tmB, kc * kBK, 0, args.b_batched ? batch : 0, bar);
+      tma_load_3d(a_dst, &tmA, args.a_kwrap > 0 ? k % args.a_kwrap : k, m_tile * kBM, args.a_batched ? batch : 0, bar);
+      tma_load_3d(b_dst, &tmB, k, n_tile * kBN, args.b_batched ? batch : 0, bar);
     };
-    load(0);
-    if (KC > 1) load(1);
-    for (int kc = 0; kc < KC; ++kc) {
-      const int s = kc & 1;
-      if (!mbar_wait(full0 + 8 * s, (kc >> 1) & 1)) {
+    for (int t = 0; t < n && t < kGemmStages; ++t) load(t);
+    for (int t = 0; t < n; ++t) {
+      const int s = t % kGemmStages;
+      if (!mbar_wait(full0 + 8 * s, (t / kGemmStages) & 1)) {
         ok = false;
         break;
       }
@@ -193,14 +207,14 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
       const uint64_t db = sw128_desc(smem_u32(smem + s * kStage + kStageA));
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j)  // K = 16 per MMA: +32 bytes = +2 in the start-address field
-        umma_bf16(tmem, da + 2 * j, db + 2 * j, (kc > 0 || j > 0) ? 1u : 0u);
+        umma_bf16(tmem, da + 2 * j, db + 2 * j, (t > 0 || j > 0) ? 1u : 0u);
       umma_commit(empty0 + 8 * s);  // stage s is free once these MMAs have read it
-      if (kc + 2 < KC) {
-        if (!mbar_wait(empty0 + 8 * s, (kc >> 1) & 1)) {
+      if (t + kGemmStages < n) {
+        if (!mbar_wait(empty0 + 8 * s, (t / kGemmStages) & 1)) {
           ok = false;
           break;
         }
-        load(kc + 2);
+        load(t + kGemmStages);
       }
     }
     umma_commit(done);
@@ -214,11 +228,12 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int row = m_tile * kBM + warp * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    for (int c0 = 0; c0 < kDim; c0 += 32) {
+    for (int c0 = 0; c0 < kBN; c0 += 32) {
       uint32_t v[32];
       tmem_ld32(lane_base + (uint32_t)c0, v);
+      const int col0 = n_tile * kBN + c0;
       if (!args.split_transpose) {
-        float4* out = (float4*)(args.out + ((size_t)batch * kDim + row) * kDim + c0);
+        float4* out = (float4*)(args.out + ((size_t)batch * kDim + row) * kDim + col0);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           out[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
@@ -230,7 +245,7 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
           const float x = __uint_as_float(v[i]);
           const __nv_bfloat16 hi = __float2bfloat16_rn(x);
           const __nv_bfloat16 lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-          __nv_bfloat16* col = base + (size_t)(c0 + i) * kK2;
+          __nv_bfloat16* col = base + (size_t)(col0 + i) * kK2;
           col[0] = hi;
           col[kDim] = lo;
           col[2 * kDim] = hi;
@@ -241,7 +256,7 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kDim) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kBN) : "memory");
 }
 
 // ----------------------------------------------------------------------------
@@ -338,6 +353,7 @@ __global__ void k_emitters(EdmFlimParams p, const double* bound_fraction, int32_
 
 // Counts to bf16, exact up to 256 per pixel; larger counts set an error bit.
 __global__ void k_counts_to_bf16(const int32_t* counts, __nv_bfloat16* maps, size_t n, uint32_t* err) {
+  edm::pdl_enter();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int32_t c = counts[i];
     if (c > 256) atomicOr(err, EDM_FLIM_ERR_COUNT);
@@ -527,6 +543,7 @@ __global__ void __launch_bounds__(32 * kHistWarps, 40 / kHistWarps) k_hist(EdmFl
     tab[i / nb][i % nb] = a.x >= 1 << 24 ? (uint32_t)(i % nb) : ((uint32_t)a.x << 8) | (uint32_t)a.y;
   }
   __syncthreads();
+  edm::pdl_enter();  // the intensities come from the kernel before
   const double Tf = sums[0], Sf = sums[1], Tb = sums[2], Sb = sums[3];
   const unsigned FULL = 0xffffffffu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -695,6 +712,25 @@ int falloc(EdmFlim* F, T** ptr, size_t n) {
   return EDM_OK;
 }
 
+// A kernel of the acquisition, queued as a programmatic dependent of the kernel
+// before it on a created stream: its prologue overlaps that kernel's tail, and
+// edm::pdl_enter() holds it until that kernel's writes are visible.  Behind
+// anything but a kernel the attribute changes nothing.
+template <typename... K, typename... A>
+void launch_after(void (*kernel)(K...), dim3 grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = reinterpret_cast<uintptr_t>(s) > 2 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int check_params(const EdmFlimParams& p) {
   if (p.nx != kDim || p.ny != kDim) return fail(EDM_EUNSUP, "FLIM acquisition: the GEMM path needs 256 x 256 pixels");
   if (p.n_replicas <= 0 || p.n_replicas > 4096) return fail(EDM_EINVAL, "FLIM acquisition: n_replicas out of 1..4096");
@@ -740,9 +776,9 @@ int edm_flim_create(const EdmFlimParams* params, int32_t device, EdmFlim** out) 
   FA(F->err, 1);
 #undef FA
   if ((rc = make_map(&F->mA1, F->maps, kDim, kDim, 2 * R, kBM)) != EDM_OK ||
-      (rc = make_map(&F->mB1, F->g1, kK1, kDim, 1, kDim)) != EDM_OK ||
+      (rc = make_map(&F->mB1, F->g1, kK1, kDim, 1, kBN)) != EDM_OK ||
       (rc = make_map(&F->mA2, F->a2, kK2, kDim, 1, kBM)) != EDM_OK ||
-      (rc = make_map(&F->mB2, F->b2, kK2, kDim, 2 * R, kDim)) != EDM_OK) {
+      (rc = make_map(&F->mB2, F->b2, kK2, kDim, 2 * R, kBN)) != EDM_OK) {
     delete F;
     return rc;
   }
@@ -794,21 +830,25 @@ int edm_flim_project(EdmFlim* F, void* stream) {
   const size_t R = (size_t)p.n_replicas, npx = (size_t)kDim * kDim;
   FL_TRY(cudaMemsetAsync(F->counts, 0, sizeof(int32_t) * R * 2 * npx, s));
   k_emitters<<<dim3(64, (unsigned)R), 256, 0, s>>>(p, F->bound_fraction, F->counts);
-  k_counts_to_bf16<<<148 * 8, 256, 0, s>>>(F->counts, F->maps, R * 2 * npx, F->err);
+  launch_after(k_counts_to_bf16, dim3(148 * 8), 256, 0, s, (const int32_t*)F->counts, F->maps, R * 2 * npx, F->err);
+  const dim3 tiles((kDim / kBM) * (kDim / kBN), (unsigned)(2 * R));
   GemmArgs a1{};
-  a1.k_chunks = kK1 / kBK;
+  a1.sections = kK1 / kDim;
   a1.a_kwrap = kDim;  // A = [M | M]: the count map twice along K
   a1.a_batched = 1;
+  a1.taps = p.half_taps;
   a1.split_transpose = 1;
   a1.b2 = F->b2;
   a1.err = F->err;
-  k_umma_gemm<<<dim3(kDim / kBM, (unsigned)(2 * R)), 128, kGemmSmem, s>>>(F->mA1, F->mB1, a1);
+  launch_after(k_umma_gemm, tiles, 128, kGemmSmem, s, F->mA1, F->mB1, a1);
   GemmArgs a2{};
-  a2.k_chunks = kK2 / kBK;
+  a2.sections = kK2 / kDim;
   a2.b_batched = 1;
+  a2.band_a = 1;
+  a2.taps = p.half_taps;
   a2.out = F->I;
   a2.err = F->err;
-  k_umma_gemm<<<dim3(kDim / kBM, (unsigned)(2 * R)), 128, kGemmSmem, s>>>(F->mA2, F->mB2, a2);
+  launch_after(k_umma_gemm, tiles, 128, kGemmSmem, s, F->mA2, F->mB2, a2);
   FL_TRY(cudaGetLastError());
   return EDM_OK;
 }
@@ -820,8 +860,8 @@ int edm_flim_histograms(EdmFlim* F, int32_t with_tau, void* stream) {
   const size_t total_px = (size_t)p.n_replicas * kDim * kDim;
   const unsigned blocks = (unsigned)std::min<size_t>((total_px / 32 + kHistWarps - 1) / kHistWarps, (size_t)F->hist_blocks);
   const auto kernel = p.n_bins == 256 ? k_hist<256> : k_hist<128>;
-  kernel<<<blocks, 32 * kHistWarps, 0, (cudaStream_t)stream>>>(p, F->I, F->alias, F->sums, F->hist, with_tau ? F->tau : nullptr, 1u,
-                                                  4u);
+  launch_after(kernel, dim3(blocks), 32 * kHistWarps, 0, (cudaStream_t)stream, p, (const float*)F->I,
+               (const int2*)F->alias, (const double*)F->sums, F->hist, with_tau ? F->tau : (double*)nullptr, 1u, 4u);
   FL_TRY(cudaGetLastError());
   return EDM_OK;
 }
