@@ -1776,53 +1776,61 @@ __global__ void __launch_bounds__(kBlock) k_particle_passes(const EdmDynParams* 
 
 // Binding candidates of reaction b (dynamics.py:528-606): pairs (i < j)
 // passing every test of the pass-start state, keyed by the reference's pair
-// order (i, neighbour-cell ordinal, descending j).
-template <bool F64>
-__global__ void __launch_bounds__(kBlock) k_bind_candidates(const EdmDynParams* __restrict__ P, DevState st,
-                                                            Match m, int b) {
+// order (i, neighbour-cell ordinal seen from i, descending j).  Swept from one
+// of the two species (both distance tests are symmetric in the particles), a
+// tile of BLK * SPT slots per block, G lanes per sweeper, as the contact search;
+// with both species swept slot by slot in a lane each the pass was 36 us for a
+// 13,900-slot sensor membrane.
+template <bool F64, int BLK, int SPT, int G>
+__global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __restrict__ P,
+                                                         const int2* __restrict__ blk, DevState st, Match m, int b) {
   pdl_enter();
-  sweep4(st, m, [&](int r, int64_t s) {
-    const EdmDynParams& p = P[r];
-    const EdmBind& B = p.bind[b];
-    const int spi = fl_species(st.flags[s]);
-    const Geo g(p);
-    const int id = slot_id(st, s) - (int)g.poff;
-    if (st.bond[g.poff + id] >= 0) return;
-    const int64_t step = *st.d_step;
-    for_neighbour_slots(g, st, st.cell_pre[s], [&](int j, int ordinal, int, int) {
-      {
-        const int idj = slot_id(st, j) - (int)g.poff;
-        if (idj <= id) return;
-        const uint8_t fj = st.flags[j];
-        if (!fl_alive(fj)) return;
-        if (st.bond[g.poff + idj] >= 0) return;
-        const int spj = fl_species(fj);
-        int a, bb;
-        if (spi == B.ra && spj == B.rb) {
-          a = id;
-          bb = idj;
-        } else if (spi == B.rb && spj == B.ra) {
-          a = idj;
-          bb = id;
-        } else {
-          return;
-        }
-        if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, s, j, g) < g.cutoff_sq())) return;
-        if (sep_sq<F64>(st.pos_post, st.cell_post, s, j, g) > B.contact_sq) return;
-        const double u = uniform1(p.seed, step, EDM_S_BIND + 2 * b, (uint64_t)id, (uint64_t)idj);
-        if (!(u < B.prob_bind)) return;
-        const int k = atomicAdd(&st.bind_count[r], 1);
-        if (k < kBindCap) {
-          st.bind_key[(int64_t)r * kBindCap + k] =
-              ((int64_t)id << 36) | ((int64_t)ordinal << 32) | (int64_t)(0xFFFFFFFFu - (uint32_t)idj);
-          st.bind_ab[((int64_t)r * kBindCap + k) * 2] = a;
-          st.bind_ab[((int64_t)r * kBindCap + k) * 2 + 1] = bb;
-        } else {
-          set_status(st.status, EDM_STATUS_BIND_CAP);
-        }
+  __shared__ int32_t list[BLK * SPT];
+  __shared__ int n_list;
+  const int2 tile = blk[blockIdx.x];
+  const int r = tile.x;
+  const EdmDynParams& p = P[r];
+  if (threadIdx.x == 0) n_list = 0;
+  __syncthreads();
+  gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)tile.y, p.particle_offset + p.n_particles, list, n_list);
+  __syncthreads();
+  const int sweepers = n_list, lane = threadIdx.x & 31;
+  if (sweepers == 0) return;
+  const EdmBind& B = p.bind[b];
+  const Geo g(p);
+  for (int t0 = (threadIdx.x >> 5) * (32 / G); t0 < sweepers; t0 += BLK / G) {  // whole warps
+    const int t = t0 + lane / G;
+    const int s = list[t < sweepers ? t : t0];
+    const int other = fl_species(st.flags[s]) == B.ra ? B.rb : B.ra;
+    const int id = slot_id(st, s) - g.poff;
+    const bool have = t < sweepers && st.bond[g.poff + id] < 0;
+    for_neighbour_slots_grouped<G>(g, st, st.cell_pre[s], have, [&](int j, bool valid, int column, int base) {
+      if (!valid || j == s) return;
+      const uint8_t fj = st.flags[j];
+      if (!fl_alive(fj) || fl_species(fj) != other) return;
+      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, s, j, g) < g.cutoff_sq())) return;
+      if (sep_sq<F64>(st.pos_post, st.cell_post, s, j, g) > B.contact_sq) return;
+      const int idj = slot_id(st, j) - g.poff;
+      if (B.ra == B.rb && idj < id) return;  // seen from the other particle
+      if (st.bond[g.poff + idj] >= 0) return;
+      const int lo = id < idj ? id : idj, hi = id < idj ? idj : id;
+      const double u = uniform1(p.seed, *st.d_step, EDM_S_BIND + 2 * b, (uint64_t)lo, (uint64_t)hi);
+      if (!(u < B.prob_bind)) return;
+      int dcx = column - 1, dcy = row_offset(st.cell_pre[j] - base, g);
+      if (lo != id) dcx = -dcx, dcy = -dcy;
+      const int ordinal = (dcx + 1) * 3 + dcy + 1;
+      const bool swept_ra = other == B.rb;
+      const int k = atomicAdd(&st.bind_count[r], 1);
+      if (k < kBindCap) {
+        st.bind_key[(int64_t)r * kBindCap + k] =
+            ((int64_t)lo << 36) | ((int64_t)ordinal << 32) | (int64_t)(0xFFFFFFFFu - (uint32_t)hi);
+        st.bind_ab[((int64_t)r * kBindCap + k) * 2] = swept_ra ? id : idj;
+        st.bind_ab[((int64_t)r * kBindCap + k) * 2 + 1] = swept_ra ? idj : id;
+      } else {
+        set_status(st.status, EDM_STATUS_BIND_CAP);
       }
     });
-  });
+  }
 }
 
 // Sequential greedy application in pair order, re-checking the live state.

@@ -336,7 +336,7 @@ struct EdmEngine {
     };
     for (int b = 0; b < p.n_bind; ++b) {
       const EdmBind& B = p.bind[b];
-      passes.push_back({P_BIND_CAND, b, match({B.ra, B.rb}, 1)});
+      passes.push_back({P_BIND_CAND, b, match({B.ra}, 1)});
       passes.push_back({P_BIND_APPLY, b, none});
       passes.push_back({P_DISSOC, b, match({B.product}, 1)});
       writes({B.ra, B.rb, B.product});
@@ -420,8 +420,13 @@ struct EdmEngine {
       reinterpret_cast<uint8_t*>(cat_lists.rx_of)[sw * EDM_MAX_SPECIES + other] |= (uint8_t)(1u << c);
       sweepers |= 1u << sw;
     }
-    for (Pass& ps : passes)
+    for (Pass& ps : passes) {
       if (ps.kind == P_CONTACTS) ps.match = Match{{0u, sweepers}};
+      if (ps.kind == P_BIND_CAND) {  // likewise the rarer of a binding's two species
+        const int ra = p.bind[ps.index].ra, rb = p.bind[ps.index].rb;
+        ps.match = Match{{0u, 1u << (count && count[rb] < count[ra] ? rb : ra)}};
+      }
+    }
   }
 
   // The per-particle passes (recruitment candidates, detachments,
@@ -795,7 +800,12 @@ struct EdmEngine {
       if (photons_late && ps.kind != P_CONTACTS && ps.kind != P_DRAWS && ps.kind != P_ADAPT && ps.kind != P_MERGE)
         join_photons(s);
       switch (ps.kind) {
-        case P_BIND_CAND: go(k_bind_candidates<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
+        case P_BIND_CAND: {
+          const int t = tile_index(kBlock);
+          if (npblk_bs[t] > 0)
+            go(k_bind_candidates<F64, 128, 2, 8>, npblk_bs[t], 128, s, dp, pblk_bs[t], st, ps.match, ps.index);
+          break;
+        }
         case P_BIND_APPLY: go(k_bind_apply<F64>, rb, 128, s, dp, R, st, ps.index); break;
         case P_DISSOC: go(k_dissociate<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
         case P_CONTACTS:
@@ -1571,8 +1581,8 @@ int edm_set_state(EdmEngine* E, const EdmHostState* st, void* stream) {
   CUDA_TRY(cudaMemcpyAsync(E->ctmc, st->ctmc_state, N, cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(E->bleached, st->is_bleached, N, cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemsetAsync(E->cnt, 0, sizeof(int32_t) * (E->n_cells > 0 ? E->n_cells : 1), s));
-  if (!E->contact_sides_counted && E->hdp[0].n_cat > 0) {
-    // the contact sweep's sides from the first state's alive species counts
+  if (!E->contact_sides_counted && (E->hdp[0].n_cat > 0 || E->hdp[0].n_bind > 0)) {
+    // the contact and binding sweeps' sides from the first state's alive species counts
     int64_t count[EDM_MAX_SPECIES] = {};
     for (int64_t i = 0; i < N; ++i) {
       const int32_t sp = st->species_id[i];
@@ -1744,7 +1754,7 @@ int edm_set_state_async(EdmEngine* E, const EdmHostState* st, void* stream) {
   if (E->has_phot && !(E->has_dye_host.size() == (size_t)E->N &&
                        std::memcmp(E->has_dye_host.data(), st->has_dye, (size_t)E->N) == 0))
     return edm_set_state(E, st, stream);
-  if (!E->contact_sides_counted && E->hdp[0].n_cat > 0) return edm_set_state(E, st, stream);
+  if (!E->contact_sides_counted && (E->hdp[0].n_cat > 0 || E->hdp[0].n_bind > 0)) return edm_set_state(E, st, stream);
   const int rc = edm_stage_state_async(E, st);
   return rc != EDM_OK ? rc : edm_install_state(E, stream);
 }
