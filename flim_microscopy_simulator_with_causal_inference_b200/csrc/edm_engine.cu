@@ -70,7 +70,7 @@ std::vector<int2> tiles(const std::vector<int64_t>& first, const std::vector<int
 
 // ---- launch shapes of the tuned kernels -------------------------------------
 // Candidate (threads per block, minimum resident blocks per SM) of each kernel
-// the autotuner times; candidate 0 is the fixed shape used without tuning.
+// the autotuner times.
 struct LaunchShape {
   int block, min_blocks;
 };
@@ -133,8 +133,9 @@ struct EdmEngine {
   int2* pblk_bs[kTileTables] = {};
   SlotTile* ptile_bs[kTileTables] = {};
   int npblk_bs[kTileTables] = {};
-  // launch shape of each tuned kernel (index into kShapes), tuning timings
-  int shape[TK_COUNT] = {0, 0, 0};
+  // launch shape of each tuned kernel (index into kShapes): in use, and without
+  // tuning; tuning timings
+  int shape[TK_COUNT] = {0, 0, 0}, untuned[TK_COUNT] = {0, 0, 0};
   float tuned_ms[TK_COUNT] = {0, 0, 0}, default_ms[TK_COUNT] = {0, 0, 0};
   int tune_kernel = -1;  // the kernel the autotuner is timing, with its event pair
   cudaEvent_t tune_ev[2] = {nullptr, nullptr};
@@ -1325,6 +1326,15 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   }
   E->pblk = E->pblk_bs[1];
   E->npblk = E->npblk_bs[1];
+  // Without tuning: candidate 0, the shapes for systems that do not fill the
+  // chip, and for larger ones what was fastest over dense and sparse membranes
+  // on both paths.  k_move with more resident warps from 2^18 slots (430,000
+  // slots 36.8 to 30.8 us float64, 25.2 to 22.6 float32; at 140,000 15.4 against
+  // 16.7), the contact search over the global list from 2^20 (1.4M slots 45 to
+  // 41 us float64, 28 to 26 float32; at 430,000 15.3 against 19.5).
+  if (np >= (1 << 18)) E->untuned[TK_MOVE] = 3;
+  if (np >= (1 << 20)) E->untuned[TK_CONTACTS] = 2;
+  for (int k = 0; k < TK_COUNT; ++k) E->shape[k] = E->untuned[k];
   {  // launch shapes chosen by an earlier tuning of an engine of this kind
     std::lock_guard<std::mutex> lock(g_tune_mu);
     for (int k = 0; k < TK_COUNT; ++k) {
@@ -2158,7 +2168,7 @@ int edm_autotune(EdmEngine* E, int32_t steps_per_shape, int32_t retune, void* st
         acc += t;
       }
       const double ms = acc / steps_per_shape;
-      if (v == 0) E->default_ms[k] = (float)ms;
+      if (v == E->untuned[k]) E->default_ms[k] = (float)ms;
       if (ms < best) {
         best = ms;
         best_v = v;
