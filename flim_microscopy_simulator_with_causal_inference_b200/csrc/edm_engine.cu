@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -222,6 +223,9 @@ struct EdmEngine {
   bool cells_valid = false;  // the cell list matches the state (a dynamics step ran since set_state)
   // captured pipeline chunks, keyed by (steps, with photons, slot parity, recording)
   std::map<std::tuple<int, int, int, int>, cudaGraphExec_t> graphs;
+  // chunks launched once without a graph: capturing and instantiating 100 steps
+  // (1,100 launches) takes 10 ms, a run of one frame of 3 ms never earns it back
+  std::set<std::tuple<int, int, int, int>> launched_once;
   // sub-frame recorder ring [rec_cap][R][EDM_CENSUS_FIELDS] and ground-truth buffers
   int rec_cap = 0;
   int64_t* rec_ring = nullptr;
@@ -1973,6 +1977,15 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
       const auto key = std::make_tuple(graph_chunk, with_photons ? 1 : 0, E->cur, E->rec_cap > 0 ? 1 : 0);
       auto it = E->graphs.find(key);
       if (it == E->graphs.end()) {
+        cudaStreamCaptureStatus capturing;
+        CUDA_TRY(cudaStreamIsCapturing(s, &capturing));
+        if (capturing == cudaStreamCaptureStatusNone && E->launched_once.insert(key).second) {
+          for (int i = 0; i < graph_chunk; ++i) body(s);
+          E->join_beside(s);
+          CUDA_TRY(cudaGetLastError());
+          done += graph_chunk;
+          continue;
+        }
         const int cur0 = E->cur;
         cudaGraph_t g;
         CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
