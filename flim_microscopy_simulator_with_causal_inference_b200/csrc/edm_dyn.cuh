@@ -208,6 +208,17 @@ struct Geo {
   }
 };
 
+// Asks for the lines of a replica's parameters that a step's kernels read
+// whatever they do (its head, its grids, its key), by the block's first
+// threads, before pdl_enter().
+__device__ __forceinline__ void prefetch_params(const EdmDynParams& p) {
+  const int t = threadIdx.x;
+  if (t < 4) prefetch_l1(reinterpret_cast<const char*>(&p) + 128 * t);
+  else if (t == 4) prefetch_l1(&p.seed);
+  else if (t == 5) prefetch_l1(&p.grid[0]);
+  else if (t == 6) prefetch_l1(&p.n_bind);
+}
+
 // Cell key c = cx * ny + cy -> (cx, cy) without an integer division: the
 // float quotient (c + 0.5) / ny is within one of cx for any c < 2^24 and the
 // remainder check corrects it, so the result is exact.
@@ -606,7 +617,6 @@ struct SlotTile {
 // SPT tiles per block put SPT slots' loads and atomics in flight per thread.
 template <bool F64, int BS, int SPT>
 __global__ void __launch_bounds__(BS) k_scatter(const SlotTile* __restrict__ tiles, int ntiles, DevState st) {
-  pdl_enter();
   using Pos = typename std::conditional<F64, double2, float2>::type;
   int src[SPT], cl[SPT], id[SPT], dst[SPT], grave[SPT], bucket0[SPT];
   uint8_t fl[SPT];
@@ -623,6 +633,12 @@ __global__ void __launch_bounds__(BS) k_scatter(const SlotTile* __restrict__ til
     src[k] = s;
     bucket0[k] = t.bucket0;
     grave[k] = t.grave;
+  }
+  pdl_enter();
+#pragma unroll
+  for (int k = 0; k < SPT; ++k) {
+    const int s = src[k];
+    if (s < 0) continue;
     cl[k] = st.cell_post[s];
     fl[k] = st.flags_old[s];
     id[k] = st.ids_old[s];
@@ -848,12 +864,14 @@ __device__ __noinline__ void dfield_call(const EdmDynParams& p, int sp, double x
 template <bool F64, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_move(const EdmDynParams* __restrict__ P, const int2* __restrict__ blk,
                                                  DevState st) {
-  pdl_enter();
   const Tile t = tile_of(blk);
   const EdmDynParams& p = P[t.r];
   const int64_t s = t.s;
-  if (s >= p.particle_offset + p.n_particles) return;
+  prefetch_params(p);
   const Geo g(p);
+  const bool in = s < p.particle_offset + p.n_particles;
+  pdl_enter();
+  if (!in) return;
   const uint8_t f = st.flags[s];
   const int c = st.cell_pre[s];
   if (!fl_alive(f)) {  // dead / dormant particles do not move (dynamics.py:360)
@@ -1302,6 +1320,60 @@ __device__ __forceinline__ void contact_sweep(const EdmDynParams* __restrict__ P
   });
 }
 
+// ---- per-particle passes: recruitment candidates, detachments, conversions ----
+// Each decides for one particle from its flags, its keyed draw u, and (only
+// when u is below the pass's threshold, pass_thr) its position and the grid
+// counts.  One sweep before the first of these passes (k_pass_draws) draws,
+// for every particle, the passes whose match holds its state; the few
+// particles with some draw below its threshold go to a list, and the passes
+// visit only that list.  A pass that changes a listed particle's state
+// (detachment, conversion, recruitment) draws at once the later passes that
+// match the new state.  A particle left off the list for a pass would be
+// rejected by it, so skipping it changes nothing.
+enum GroupPass : int8_t { kGroupRecruit = 0, kGroupDetach = 1, kGroupConvert = 2 };
+struct DrawPlan {
+  Match any;                           // states that some pass matches
+  uint32_t reach[2][EDM_MAX_SPECIES];  // passes matching (alive, species), from the sweep on
+  uint32_t after[kMaxPP];              // passes after pass k matching the state pass k leaves
+  int8_t kind[kMaxPP];                 // GroupPass of each per-particle pass
+  int8_t index[kMaxPP];                // its exchange or conversion
+  int n;
+};
+
+__device__ __forceinline__ int pass_stream(int kind, int idx) {
+  return kind == kGroupRecruit ? EDM_S_EX_ACCEPT + 4 * idx
+                               : (kind == kGroupDetach ? EDM_S_EX_DETACH + 4 * idx : EDM_S_CONV + idx);
+}
+
+// Bits of the passes in `todo` whose keyed draw for local id `id` lies below
+// the pass's threshold (the others reject the particle).
+__device__ __forceinline__ uint32_t draw_passes(const DevState& st, const DrawPlan* __restrict__ D, uint64_t seed,
+                                                int r, int id, int64_t step, uint32_t todo) {
+  uint32_t bits = 0;
+  for (; todo; todo &= todo - 1) {
+    const int k = __ffs(todo) - 1;
+    const uint64_t m = draw_u53(seed, step, pass_stream(D->kind[k], D->index[k]), (uint64_t)id, 0);
+    if (m < st.pass_thr[(int64_t)r * kMaxPP + k]) bits |= 1u << k;
+  }
+  return bits;
+}
+
+// The draw sweep's work for one slot of replica r: its passes' draws, and its
+// list entry when one lies below its threshold.
+__device__ __forceinline__ void draw_slot(const EdmDynParams& p, const DevState& st, const DrawPlan* __restrict__ D,
+                                          int r, int64_t s) {
+  const uint8_t f = st.flags[s];
+  const int sp = fl_species(f);
+  const uint32_t todo = sp < EDM_MAX_SPECIES ? D->reach[fl_alive(f) ? 1 : 0][sp] : 0u;
+  const int id = slot_id(st, s) - (int)p.particle_offset;
+  const uint32_t bits = draw_passes(st, D, p.seed, r, id, *st.d_step, todo);
+  if (bits) {
+    const int q = st.rep_pl ? (int)p.particle_offset + atomicAdd(&st.pl_count[r], 1) : atomicAdd(st.pl_count, 1);
+    st.pl[q] = make_int4((int)s, (int)bits, r, id);
+    st.pl_index[s] = q;
+  }
+}
+
 // Contact search of the step.  What bounds it is the chain of round trips to
 // L2 (sweeper, bucket bounds, neighbours, their post-move positions) and the
 // instructions per neighbour, not bytes: groups of G lanes take one sweeper
@@ -1319,23 +1391,32 @@ __device__ __forceinline__ void contact_sweep(const EdmDynParams* __restrict__ P
 //
 // k_contacts: a block takes a tile of BLK * SPT slots of one replica and
 // gathers its sweepers in shared memory.  One launch and one block's chain:
-// the form for systems that do not fill the chip.
+// the form for systems that do not fill the chip.  With a draw plan D as many
+// blocks again take the tiles' draws (the draw sweep, k_pass_draws, beside the
+// search without a stream of its own).
 template <bool F64, int BLK, int SPT, int G, int MINB>
 __global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __restrict__ P,
-                                                      const int2* __restrict__ blk, DevState st, Match m,
-                                                      const __grid_constant__ CatLists L) {
-  pdl_enter();
+                                                      const int2* __restrict__ blk, int ntiles, DevState st, Match m,
+                                                      const __grid_constant__ CatLists L,
+                                                      const DrawPlan* __restrict__ D, Match any) {
   __shared__ int32_t list[BLK * SPT];
   __shared__ ContactQueue queue[BLK / 32];
   __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   __shared__ int n_list;
-  const int2 b = blk[blockIdx.x];
+  const bool draws = (int)blockIdx.x >= ntiles;
+  const int2 b = blk[draws ? (int)blockIdx.x - ntiles : (int)blockIdx.x];
   const int64_t end = P[b.x].particle_offset + P[b.x].n_particles;
+  prefetch_params(P[b.x]);
+  pdl_enter();
   if (threadIdx.x == 0) n_list = 0;
   if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
   __syncthreads();
-  gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)b.y, end, list, n_list);
+  gather_matching<BLK, SPT>(st, draws ? any : m, (int64_t)(uint32_t)b.y, end, list, n_list);
   __syncthreads();
+  if (draws) {
+    for (int t = threadIdx.x; t < n_list; t += BLK) draw_slot(P[b.x], st, D, b.x, list[t]);
+    return;
+  }
   const int sweepers = n_list, lane = threadIdx.x & 31;
   ContactQueue& Q = queue[threadIdx.x >> 5];
   int queued = 0;
@@ -1351,14 +1432,14 @@ __global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __re
 constexpr int kSweepSlots = 16;  // per thread
 __global__ void __launch_bounds__(kBlock) k_sweep_list(const EdmDynParams* __restrict__ P,
                                                        const int2* __restrict__ blk, DevState st, Match m) {
-  pdl_enter();
   __shared__ int32_t list[kBlock * kSweepSlots];
   __shared__ int n_list, at;
   const int2 b = blk[blockIdx.x];
+  const int64_t end = P[b.x].particle_offset + P[b.x].n_particles;
   if (threadIdx.x == 0) n_list = 0;
+  pdl_enter();
   __syncthreads();
-  gather_matching<kBlock, kSweepSlots>(st, m, (int64_t)(uint32_t)b.y, P[b.x].particle_offset + P[b.x].n_particles, list,
-                                       n_list);
+  gather_matching<kBlock, kSweepSlots>(st, m, (int64_t)(uint32_t)b.y, end, list, n_list);
   __syncthreads();
   const int n = n_list;
   if (n == 0) return;
@@ -1373,10 +1454,10 @@ __global__ void __launch_bounds__(kBlock) k_sweep_list(const EdmDynParams* __res
 template <bool F64, int G, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynParams* __restrict__ P, DevState st,
                                                               const __grid_constant__ CatLists L) {
-  pdl_enter();
   __shared__ ContactQueue queue[kBlock / 32];
   __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
+  pdl_enter();
   __syncthreads();
   const int n = *st.sw_count, lane = threadIdx.x & 31;
   const int stride = (int)gridDim.x * (kBlock / G);
@@ -1477,59 +1558,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __r
   }
 }
 
-// ---- per-particle passes: recruitment candidates, detachments, conversions ----
-// Each decides for one particle from its flags, its keyed draw u, and (only
-// when u is below the pass's threshold, pass_thr) its position and the grid
-// counts.  One sweep before the first of these passes (k_pass_draws) draws,
-// for every particle, the passes whose match holds its state; the few
-// particles with some draw below its threshold go to a list, and the passes
-// visit only that list.  A pass that changes a listed particle's state
-// (detachment, conversion, recruitment) draws at once the later passes that
-// match the new state.  A particle left off the list for a pass would be
-// rejected by it, so skipping it changes nothing.
-enum GroupPass : int8_t { kGroupRecruit = 0, kGroupDetach = 1, kGroupConvert = 2 };
-struct DrawPlan {
-  Match any;                           // states that some pass matches
-  uint32_t reach[2][EDM_MAX_SPECIES];  // passes matching (alive, species), from the sweep on
-  uint32_t after[kMaxPP];              // passes after pass k matching the state pass k leaves
-  int8_t kind[kMaxPP];                 // GroupPass of each per-particle pass
-  int8_t index[kMaxPP];                // its exchange or conversion
-  int n;
-};
-
-__device__ __forceinline__ int pass_stream(int kind, int idx) {
-  return kind == kGroupRecruit ? EDM_S_EX_ACCEPT + 4 * idx
-                               : (kind == kGroupDetach ? EDM_S_EX_DETACH + 4 * idx : EDM_S_CONV + idx);
-}
-
-// Bits of the passes in `todo` whose keyed draw for local id `id` lies below
-// the pass's threshold (the others reject the particle).
-__device__ __forceinline__ uint32_t draw_passes(const DevState& st, const DrawPlan* __restrict__ D, uint64_t seed,
-                                                int r, int id, int64_t step, uint32_t todo) {
-  uint32_t bits = 0;
-  for (; todo; todo &= todo - 1) {
-    const int k = __ffs(todo) - 1;
-    const uint64_t m = draw_u53(seed, step, pass_stream(D->kind[k], D->index[k]), (uint64_t)id, 0);
-    if (m < st.pass_thr[(int64_t)r * kMaxPP + k]) bits |= 1u << k;
-  }
-  return bits;
-}
-
 __global__ void __launch_bounds__(kBlock, 8) k_pass_draws(const EdmDynParams* __restrict__ P, DevState st,
                                                        const DrawPlan* __restrict__ D, Match any) {
   pdl_enter();
-  sweep4(st, any, [&](int r, int64_t s) {
-    const uint8_t f = st.flags[s];
-    const int sp = fl_species(f);
-    const uint32_t todo = sp < EDM_MAX_SPECIES ? D->reach[fl_alive(f) ? 1 : 0][sp] : 0u;
-    const int id = slot_id(st, s) - (int)P[r].particle_offset;
-    const uint32_t bits = draw_passes(st, D, P[r].seed, r, id, *st.d_step, todo);
-    if (bits) {
-      const int q = st.rep_pl ? (int)P[r].particle_offset + atomicAdd(&st.pl_count[r], 1) : atomicAdd(st.pl_count, 1);
-      st.pl[q] = make_int4((int)s, (int)bits, r, id);
-      st.pl_index[s] = q;
-    }
-  });
+  sweep4(st, any, [&](int r, int64_t s) { draw_slot(P[r], st, D, r, s); });
 }
 
 // Puts particle `id` of replica r (in `slot`), recruited by exchange e, at (x, y).  It is
@@ -1784,15 +1816,17 @@ __global__ void __launch_bounds__(kBlock) k_particle_passes(const EdmDynParams* 
 template <bool F64, int BLK, int SPT, int G>
 __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __restrict__ P,
                                                          const int2* __restrict__ blk, DevState st, Match m, int b) {
-  pdl_enter();
   __shared__ int32_t list[BLK * SPT];
   __shared__ int n_list;
   const int2 tile = blk[blockIdx.x];
   const int r = tile.x;
   const EdmDynParams& p = P[r];
+  const int64_t end = p.particle_offset + p.n_particles;
+  prefetch_params(p);
   if (threadIdx.x == 0) n_list = 0;
+  pdl_enter();
   __syncthreads();
-  gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)tile.y, p.particle_offset + p.n_particles, list, n_list);
+  gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)tile.y, end, list, n_list);
   __syncthreads();
   const int sweepers = n_list, lane = threadIdx.x & 31;
   if (sweepers == 0) return;
@@ -2027,7 +2061,6 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
                                                        const PassGroup* __restrict__ groups,
                                                        const DrawPlan* __restrict__ D, int64_t* step,
                                                        unsigned* ticket) {
-  pdl_enter();
   static_assert(sizeof(EdmDynParams) % 16 == 0 && sizeof(PassGroup) % 4 == 0, "copied in words");
   __shared__ __align__(16) uint8_t par[sizeof(EdmDynParams)];
   __shared__ __align__(16) uint8_t grp[kReactGroups * sizeof(PassGroup)];
@@ -2043,10 +2076,11 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
     ((uint4*)par)[k] = ((const uint4*)(P + r))[k];
   for (int k = tid; k < plan.n_groups * (int)(sizeof(PassGroup) / 4); k += blockDim.x)
     ((uint32_t*)grp)[k] = ((const uint32_t*)groups)[k];
+  const int64_t poff = P[r].particle_offset;
+  pdl_enter();
   if (tid < EDM_MAX_CAT) n_contact[tid] = st.rep_contacts ? st.contact_count[(int64_t)r * EDM_MAX_CAT + tid] : 0;
   if (tid == 0) n_rec = n_delta = 0;
   const int n_listed = st.pl_count[r];
-  const int64_t poff = P[r].particle_offset;
   for (int q = tid; q < n_listed && q < kReactList; q += blockDim.x) entry[q] = st.pl[poff + q];
   __syncthreads();
   const EdmDynParams& p = *reinterpret_cast<const EdmDynParams*>(par);

@@ -742,14 +742,15 @@ struct EdmEngine {
   }
 
   template <bool F64, int K>  // row K of kShapes[TK_CONTACTS], kContactSlots, kContactLanes
-  void contacts_shape(const DevState& st, const Match& m, cudaStream_t s) {
+  void contacts_shape(const DevState& st, const Match& m, bool with_draws, cudaStream_t s) {
     constexpr LaunchShape sh = kShapes[TK_CONTACTS][K];
     constexpr int slots = kContactSlots[K], lanes = kContactLanes[K];
     const int t = tile_index(slots > 0 ? sh.block * slots : kBlock * kSweepSlots);
     if (npblk_bs[t] == 0) return;
     if constexpr (slots > 0) {
-      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, npblk_bs[t], sh.block, s, dp, pblk_bs[t], st, m,
-         cat_lists);
+      const int nt = npblk_bs[t];
+      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, with_draws ? 2 * nt : nt, sh.block, s, dp, pblk_bs[t], nt,
+         st, m, cat_lists, with_draws ? d_draw : nullptr, draw.any);
     } else {
       static_assert(sh.block == kBlock, "the list form's blocks");
       go(k_sweep_list, npblk_bs[t], kBlock, s, dp, pblk_bs[t], st, m);
@@ -758,16 +759,16 @@ struct EdmEngine {
   }
 
   template <bool F64>
-  void launch_contacts(const DevState& st, const Match& m, cudaStream_t s) {
+  void launch_contacts(const DevState& st, const Match& m, bool with_draws, cudaStream_t s) {
     switch (shape[TK_CONTACTS]) {
-      case 1: contacts_shape<F64, 1>(st, m, s); break;
-      case 2: contacts_shape<F64, 2>(st, m, s); break;
-      case 3: contacts_shape<F64, 3>(st, m, s); break;
-      case 4: contacts_shape<F64, 4>(st, m, s); break;
-      case 5: contacts_shape<F64, 5>(st, m, s); break;
-      case 6: contacts_shape<F64, 6>(st, m, s); break;
-      case 7: contacts_shape<F64, 7>(st, m, s); break;
-      default: contacts_shape<F64, 0>(st, m, s); break;
+      case 1: contacts_shape<F64, 1>(st, m, with_draws, s); break;
+      case 2: contacts_shape<F64, 2>(st, m, with_draws, s); break;
+      case 3: contacts_shape<F64, 3>(st, m, with_draws, s); break;
+      case 4: contacts_shape<F64, 4>(st, m, with_draws, s); break;
+      case 5: contacts_shape<F64, 5>(st, m, with_draws, s); break;
+      case 6: contacts_shape<F64, 6>(st, m, with_draws, s); break;
+      case 7: contacts_shape<F64, 7>(st, m, with_draws, s); break;
+      default: contacts_shape<F64, 0>(st, m, with_draws, s); break;
     }
   }
 
@@ -810,6 +811,7 @@ struct EdmEngine {
     const int cgrid = 148 * 8;
     const int gm = (int)std::min<int64_t>((n_grid + 255) / 256, 4096);
     bool joined = true;  // the side stream's draw sweep has been waited for
+    const bool draws_beside = draws_join_contacts() && !pass_prof && tune_kernel < 0;
     for (size_t i = 0; i < passes.size(); ++i) {
       const Pass& ps = passes[i];
       if (pass_prof) cudaEventRecord(pass_prof[i], s);
@@ -827,13 +829,14 @@ struct EdmEngine {
         case P_DISSOC: go(k_dissociate<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
         case P_CONTACTS:
           tune_mark(TK_CONTACTS, 0, s);
-          launch_contacts<F64>(st, ps.match, s);
+          launch_contacts<F64>(st, ps.match, draws_beside, s);
           tune_mark(TK_CONTACTS, 1, s);
           break;
         case P_CAT: go(k_catalytic<F64>, cgrid, kBlock, s, dp, st, ps.index, cat_late[ps.index]); break;
         case P_REC_APPLY: go(k_recruit_apply<F64>, rb, 128, s, dp, R, st, ps.index, d_draw, rec_after[ps.index]); break;
         case P_DRAWS: {
           // beside the following passes on the side stream (not while timing passes one by one)
+          if (draws_beside) break;
           const bool fork = draws_early && !pass_prof && side_stream;
           cudaStream_t ds = s;
           if (fork) {
@@ -881,8 +884,17 @@ struct EdmEngine {
     mark(4, s);
   }
 
+  // Where the draw sweep may run beside the contact search and that goes tile
+  // by tile, its blocks join the search's launch: no fork and join between the
+  // step's kernels, which go on as programmatic dependents (5,000 slots 28.9 to
+  // 27.9 us a step, 207,000 slots 42.5 to 40.8).
+  bool draws_join_contacts() const {
+    return draws_early && hdp[0].n_cat > 0 && kContactSlots[shape[TK_CONTACTS]] > 0;
+  }
+
   int launches_per_step(bool with_photons) const {
     int n = 3 + 1 + 1 + (int)passes.size() + (react_ticket ? 0 : 1);
+    if (draws_join_contacts()) --n;
     for (const Pass& ps : passes)  // the sweeper-list contact shapes launch two kernels
       if (ps.kind == P_CONTACTS && kContactSlots[shape[TK_CONTACTS]] == 0) ++n;
     if (with_photons) n += (neblk > 0 ? 2 : 1) + (nphblk > 0 ? 1 : 0);
