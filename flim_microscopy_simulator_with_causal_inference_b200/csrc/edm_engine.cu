@@ -163,6 +163,7 @@ struct EdmEngine {
   int8_t *dye = nullptr, *ctmc = nullptr;
   int32_t *cell_start = nullptr, *cursor = nullptr, *cnt = nullptr, *bsum = nullptr;
   int nb_scan = 0;
+  bool small_scan = false;  // k_scan_replica instead of the tiled scan
   int32_t *grid_cnt = nullptr, *grid_delta = nullptr;
   int64_t* counters = nullptr;
   uint32_t* status = nullptr;
@@ -786,10 +787,14 @@ struct EdmEngine {
     // with proximity FRET the previous step's photon pass reads the bucket
     // starts and the list of particles placed after the sort, cleared here
     if (phot_uses_cells) join_photons(s);
-    k_scan_reduce<<<nbs, kScanThreads, 0, s>>>(cnt, n_cells, bsum, z);  // starts the chain
-    pdl_chain = true;
-    go(k_scan_bsum, 1, 1024, s, bsum, nbs);
-    go(k_scan_down, nbs, kScanThreads, s, cnt, n_cells, bsum, cell_start, cursor);
+    if (small_scan) {
+      go(k_scan_replica, R, 1024, s, dp, cnt, cell_start, cursor, z);
+    } else {
+      k_scan_reduce<<<nbs, kScanThreads, 0, s>>>(cnt, n_cells, bsum, z);  // starts the chain
+      pdl_chain = true;
+      go(k_scan_bsum, 1, 1024, s, bsum, nbs);
+      go(k_scan_down, nbs, kScanThreads, s, cnt, n_cells, bsum, cell_start, cursor);
+    }
     mark(1, s);
     cur ^= 1;
     DevState st = dev_state();
@@ -893,7 +898,7 @@ struct EdmEngine {
   }
 
   int launches_per_step(bool with_photons) const {
-    int n = 3 + 1 + 1 + (int)passes.size() + (react_ticket ? 0 : 1);
+    int n = (small_scan ? 1 : 3) + 1 + 1 + (int)passes.size() + (react_ticket ? 0 : 1);
     if (draws_join_contacts()) --n;
     for (const Pass& ps : passes)  // the sweeper-list contact shapes launch two kernels
       if (ps.kind == P_CONTACTS && kContactSlots[shape[TK_CONTACTS]] == 0) ++n;
@@ -1266,6 +1271,9 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   ALLOC(E->cnt, nc);
   E->nb_scan = (int)((nc + kScanTile - 1) / kScanTile);
   if (E->nb_scan < 1) E->nb_scan = 1;
+  E->small_scan = n_replicas <= 148;
+  for (const EdmDynParams& p : E->hdp)
+    if ((int64_t)p.nx * p.ny + 1 > kSmallScan) E->small_scan = false;
   ALLOC(E->bsum, (size_t)E->nb_scan);
   ALLOC(E->grid_cnt, ng);
   ALLOC(E->grid_delta, ng);
@@ -1892,6 +1900,7 @@ int edm_dynamics_step(EdmEngine* E, int32_t n_steps, void* stream) {
   if (!E || n_steps < 0) return fail(EDM_EINVAL, "edm_dynamics_step: bad argument");
   CUDA_TRY(cudaSetDevice(E->device));
   cudaStream_t s = (cudaStream_t)stream;
+  E->pdl_chain = false;  // whatever the caller queued comes first
   for (int i = 0; i < n_steps; ++i) E->enqueue_dynamics(s);
   CUDA_TRY(cudaGetLastError());
   return EDM_OK;
@@ -1984,6 +1993,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
     }
   };
   int done = 0;
+  E->pdl_chain = false;
   if (graph_chunk > 0 && s != nullptr) {
     while (n_steps - done >= graph_chunk) {
       const auto key = std::make_tuple(graph_chunk, with_photons ? 1 : 0, E->cur, E->rec_cap > 0 ? 1 : 0);
@@ -2001,6 +2011,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
         const int cur0 = E->cur;
         cudaGraph_t g;
         CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        E->pdl_chain = false;
         for (int i = 0; i < graph_chunk; ++i) body(s);
         E->join_beside(s);  // the capture ends on the origin stream
         CUDA_TRY(cudaStreamEndCapture(s, &g));
@@ -2015,6 +2026,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
       done += graph_chunk;
     }
   }
+  if (done > 0) E->pdl_chain = false;
   for (; done < n_steps; ++done) body(s);
   E->join_beside(s);  // whatever the caller queues next sees the photon and detection passes done
   CUDA_TRY(cudaGetLastError());
