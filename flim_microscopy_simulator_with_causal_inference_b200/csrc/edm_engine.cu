@@ -640,7 +640,11 @@ struct EdmEngine {
           react.kind[k] = kReactRecruit;
           react.more[k] = rec_after[ps.index];
           break;
-        case P_LOCAL_CDF: react.kind[k] = kReactCdf; break;
+        case P_LOCAL_CDF:
+          react.kind[k] = kReactCdf;
+          for (int d = 0; d < draw.n; ++d)
+            if (draw.kind[d] == kGroupRecruit && draw.index[d] == ps.index) react.more[k] |= 1u << d;
+          break;
         default:
           react.kind[k] = kReactMerge;
           merges = true;
