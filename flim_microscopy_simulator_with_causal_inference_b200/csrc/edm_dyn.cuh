@@ -76,6 +76,11 @@ struct DevState {
   int32_t* bind_count;   // [R]
   int64_t* bind_key;     // [R][kBindCap]
   int32_t* bind_ab;      // [R][kBindCap][2] local ids (a = reactant A role, b = B role)
+  // complexes that dissociate in the binding pass (slot, partner's slot), replica
+  // r's from its particle_offset up, those whose partner is alive (no binding
+  // leaves one so, but a state may hold one) from its last particle down
+  int2* dis;
+  int32_t* dis_count;    // [binding reactions][R][2]
   // catalytic contacts of the step: (enzyme slot, substrate-capable slot),
   // contact_cap per reaction.  With rep_contacts each replica has its own part
   // of the reaction's array and its own counts (k_react takes a replica per
@@ -574,15 +579,16 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int& total) {
 }
 
 // Buffers the step clears before its kernels use them (density grids and
-// their deltas, the placed-after-sort and contact counters, the draw list
-// length): cleared by the first scan kernel instead of one memset each.
+// their deltas, the placed-after-sort and contact counters, the draw and
+// dissociation list lengths): cleared by the first scan kernel instead of one memset each.
 struct StepZero {
-  int32_t* p[6];
-  int64_t n[6];
+  static constexpr int kCount = 7;
+  int32_t* p[kCount];
+  int64_t n[kCount];
 };
 
 __global__ void k_scan_reduce(const int32_t* __restrict__ cnt, int64_t n, int32_t* __restrict__ bsum, StepZero z) {
-  for (int k = 0; k < 6; ++k)
+  for (int k = 0; k < StepZero::kCount; ++k)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < z.n[k]; i += (int64_t)gridDim.x * blockDim.x)
       z.p[k][i] = 0;
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
@@ -612,7 +618,7 @@ __global__ void __launch_bounds__(1024) k_scan_replica(const EdmDynParams* __res
   const int64_t lo = p.cell_offset, hi = lo + (int64_t)p.nx * p.ny + 1, first = lo & ~(int64_t)3;
   const int slot0 = (int)p.particle_offset;
   pdl_enter();
-  for (int k = 0; k < 6; ++k)
+  for (int k = 0; k < StepZero::kCount; ++k)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < z.n[k]; i += (int64_t)gridDim.x * blockDim.x)
       z.p[k][i] = 0;
   // warp w takes the rounds' 128-cell stretches one after another
@@ -1886,13 +1892,20 @@ __global__ void __launch_bounds__(kBlock) k_particle_passes(const EdmDynParams* 
   }
 }
 
+// Whether the complex of local id `id` of reaction b dissociates in this step
+// (dynamics.py:609-654).
+__device__ __forceinline__ bool dissociates(const EdmDynParams& p, const DevState& st, int b, int id) {
+  return uniform1(p.seed, *st.d_step, EDM_S_DISSOC + 2 * b, (uint64_t)id, 0) < p.bind[b].prob_dissoc;
+}
+
 // Binding candidates of reaction b (dynamics.py:528-606): pairs (i < j)
 // passing every test of the pass-start state, keyed by the reference's pair
 // order (i, neighbour-cell ordinal seen from i, descending j).  Swept from one
 // of the two species (both distance tests are symmetric in the particles), a
 // tile of BLK * SPT slots per block, G lanes per sweeper, as the contact search;
 // with both species swept slot by slot in a lane each the pass was 36 us for a
-// 13,900-slot sensor membrane.
+// 13,900-slot sensor membrane.  The tile's complexes draw for their dissociation
+// on the way (st.dis).
 template <bool F64, int BLK, int SPT, int G>
 __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __restrict__ P,
                                                          const int2* __restrict__ blk, DevState st, Match m, int b) {
@@ -1909,6 +1922,17 @@ __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __r
   gather_matching<BLK, SPT>(st, m, (int64_t)(uint32_t)tile.y, end, list, n_list);
   __syncthreads();
   const int sweepers = n_list, lane = threadIdx.x & 31;
+  const uint8_t complex = fl_make(p.bind[b].product, true);
+  for (int k = threadIdx.x; k < BLK * SPT; k += BLK) {
+    const int64_t s = (int64_t)(uint32_t)tile.y + k;
+    if (s >= end || st.flags[s] != complex) continue;
+    const int id = slot_id(st, s) - (int)p.particle_offset;
+    const int partner = st.bond[p.particle_offset + id];
+    if (partner < 0 || !dissociates(p, st, b, id)) continue;
+    const int sj = st.slot_of_id[partner], awake = fl_alive(st.flags[sj]) ? 1 : 0;
+    const int q = atomicAdd(&st.dis_count[(b * st.n_rep + r) * 2 + awake], 1);
+    st.dis[awake ? end - 1 - q : p.particle_offset + q] = make_int2((int)s, sj);
+  }
   if (sweepers == 0) return;
   const EdmBind& B = p.bind[b];
   const Geo g(p);
@@ -1947,43 +1971,109 @@ __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __r
   }
 }
 
-// Sequential greedy application in pair order, re-checking the live state.
+// Dissociation of the complex in slot s, its partner in slot sj, of reaction b.
+// The binding passes change the grid counts at once: none of them reads them.
 template <bool F64>
-__global__ void k_bind_apply(const EdmDynParams* __restrict__ P, int n_rep, DevState st, int b) {
-  pdl_enter();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n_rep) return;
-  const EdmDynParams& p = P[r];
+__device__ __forceinline__ void dissociate_one(const EdmDynParams& p, const Geo& g, const DevState& st, int r, int b,
+                                               int64_t s, int64_t sj) {
   const EdmBind& B = p.bind[b];
-  int n = st.bind_count[r];
-  if (n > kBindCap) n = kBindCap;
-  st.bind_count[r] = 0;
-  if (n == 0) return;
-  int64_t* key = st.bind_key + (int64_t)r * kBindCap;
-  int32_t* ab = st.bind_ab + (int64_t)r * kBindCap * 2;
-  for (int i = 1; i < n; ++i) {
-    const int64_t k = key[i];
-    const int a = ab[2 * i], bb = ab[2 * i + 1];
-    int j = i - 1;
-    while (j >= 0 && key[j] > k) {
-      key[j + 1] = key[j];
-      ab[2 * (j + 1)] = ab[2 * j];
-      ab[2 * (j + 1) + 1] = ab[2 * j + 1];
-      --j;
-    }
-    key[j + 1] = k;
-    ab[2 * (j + 1)] = a;
-    ab[2 * (j + 1) + 1] = bb;
+  double x, y;
+  abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, s, g, x, y);
+  const uint8_t fj = st.flags[sj];
+  st.flags[s] = fl_make(B.ra, true);
+  st.flags[sj] = fl_make(B.rb, true);
+  const int newc = st.cell_post[s];
+  if constexpr (F64) {
+    ((double2*)st.pos_post)[sj] = ((const double2*)st.pos_post)[s];
+  } else {
+    ((float2*)st.pos_post)[sj] = ((const float2*)st.pos_post)[s];
+    st.lo_post[sj] = st.lo_post[s];
   }
+  rebucket(st, g, fl_alive(fj) ? st.cell_post[sj] : g.grave, newc);
+  st.cell_post[sj] = newc;
+  note_moved(st, r, p, sj);
+  st.bond[slot_id(st, s)] = -1;
+  st.bond[slot_id(st, sj)] = -1;
+  grid_change(p, DeltaArray{st.grid_cnt}, B.product, true, B.ra, true, x, y);
+  grid_change(p, DeltaArray{st.grid_cnt}, fl_species(fj), fl_alive(fj), B.rb, true, x, y);
+  atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_DISSOC], 1);
+}
+
+// Reaction b after its candidates, 1 + `parts` blocks per replica.  The first
+// applies the replica's candidates in pair order, each unless an earlier one took
+// one of its particles, and dissociates the new complexes whose draw says so; the
+// others dissociate the listed ones, which no candidate touches (the particles
+// were bound or dormant at the pass's start; one with a partner alive waits for
+// the candidates).  What bounds it is round trips, so
+// the candidates' state is fetched for all at once and their order settled in
+// shared memory, where a candidate waits only for earlier ones that share a
+// particle with it.  One thread per replica taking one candidate after the other,
+// a sweep over all slots for the dissociations and a merge of the grid changes
+// were three launches: 26 us against 10 for 13,900 slots, 167 against 19 for
+// 714,000 (150 candidates a step).
+constexpr int kBindThreads = 256;
+template <bool F64>
+__global__ void __launch_bounds__(kBindThreads, 4) k_bind_apply(const EdmDynParams* __restrict__ P, DevState st, int b,
+                                                           int parts) {
+  __shared__ int64_t key[kBindCap];
+  __shared__ int2 pair[kBindCap];  // in pair order
+  __shared__ int8_t state[kBindCap];
+  __shared__ int2 fresh[kBindCap];  // new complexes that dissociate
+  __shared__ int n_fresh, n_bound;
+  enum { kOpen, kTaken, kRejected };
+  const int r = blockIdx.x / (1 + parts), part = blockIdx.x % (1 + parts), tid = threadIdx.x;
+  const EdmDynParams& p = P[r];
+  prefetch_params(p);
+  pdl_enter();
+  const EdmBind& B = p.bind[b];
   const Geo g(p);
-  int64_t nb = 0;
-  for (int i = 0; i < n; ++i) {
-    const int a = ab[2 * i], bb = ab[2 * i + 1];
+  const int32_t* dis_count = st.dis_count + (b * st.n_rep + r) * 2;
+  if (part > 0) {
+    const int nd = *dis_count;
+    for (int q = (part - 1) * kBindThreads + tid; q < nd; q += parts * kBindThreads) {
+      const int2 e = st.dis[g.poff + q];
+      dissociate_one<F64>(p, g, st, r, b, e.x, e.y);
+    }
+    return;
+  }
+  const int n = min(st.bind_count[r], kBindCap), n_awake = dis_count[1];
+  if (n == 0 && n_awake == 0) return;
+  for (int i = tid; i < n; i += kBindThreads) key[i] = st.bind_key[(int64_t)r * kBindCap + i];
+  if (tid == 0) n_fresh = n_bound = 0;
+  __syncthreads();
+  if (tid == 0) st.bind_count[r] = 0;
+  for (int i = tid; i < n; i += kBindThreads) {
+    const int2 ab = ((const int2*)st.bind_ab)[(int64_t)r * kBindCap + i];
+    int rank = 0;
+    for (int j = 0; j < n; ++j) rank += key[j] < key[i] || (key[j] == key[i] && j < i);
+    pair[rank] = ab;
+    const uint8_t fa = st.flags[st.slot_of_id[g.poff + ab.x]], fb = st.flags[st.slot_of_id[g.poff + ab.y]];
+    const bool free = st.bond[g.poff + ab.x] < 0 && st.bond[g.poff + ab.y] < 0;
+    state[rank] = free && fa == fl_make(B.ra, true) && fb == fl_make(B.rb, true) ? kOpen : kRejected;
+  }
+  __syncthreads();
+  for (bool open = true; open;) {  // the first open candidate is settled in every round
+    open = false;
+    for (int i = tid; i < n; i += kBindThreads) {
+      if (((volatile int8_t*)state)[i] != kOpen) continue;
+      const int2 ab = pair[i];
+      int8_t now = kTaken;
+      for (int j = 0; j < i && now != kRejected; ++j) {
+        const int2 o = pair[j];
+        if (o.x != ab.x && o.x != ab.y && o.y != ab.x && o.y != ab.y) continue;
+        const int8_t other = ((volatile int8_t*)state)[j];
+        if (other == kTaken) now = kRejected;
+        else if (other == kOpen) now = kOpen;
+      }
+      if (now == kOpen) open = true;
+      else ((volatile int8_t*)state)[i] = now;
+    }
+    open = __syncthreads_or(open);
+  }
+  for (int i = tid; i < n; i += kBindThreads) {
+    if (state[i] != kTaken) continue;
+    const int a = pair[i].x, bb = pair[i].y;
     const int64_t sa = st.slot_of_id[g.poff + a], sb = st.slot_of_id[g.poff + bb];
-    const uint8_t fa = st.flags[sa], fb = st.flags[sb];
-    if (!fl_alive(fa) || !fl_alive(fb)) continue;
-    if (st.bond[g.poff + a] >= 0 || st.bond[g.poff + bb] >= 0) continue;
-    if (fl_species(fa) != B.ra || fl_species(fb) != B.rb) continue;
     double xa, ya, xb, yb;
     abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, sa, g, xa, ya);
     abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, sb, g, xb, yb);
@@ -1992,52 +2082,19 @@ __global__ void k_bind_apply(const EdmDynParams* __restrict__ P, int n_rep, DevS
     rebucket(st, g, st.cell_post[sb], g.grave);
     st.bond[g.poff + a] = (int32_t)(g.poff + bb);
     st.bond[g.poff + bb] = (int32_t)(g.poff + a);
-    grid_change(p, DeltaArray{st.grid_delta}, B.ra, true, B.product, true, xa, ya);
-    grid_change(p, DeltaArray{st.grid_delta}, B.rb, true, B.rb, false, xb, yb);
-    ++nb;
+    grid_change(p, DeltaArray{st.grid_cnt}, B.ra, true, B.product, true, xa, ya);
+    grid_change(p, DeltaArray{st.grid_cnt}, B.rb, true, B.rb, false, xb, yb);
+    atomicAdd(&n_bound, 1);
+    if (dissociates(p, st, b, a)) fresh[atomicAdd(&n_fresh, 1)] = make_int2((int)sa, (int)sb);
   }
-  atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_BINDINGS], nb);
+  __syncthreads();
+  if (tid == 0) atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_BINDINGS], n_bound);
+  for (int q = tid; q < n_fresh + n_awake; q += kBindThreads) {
+    const int2 e = q < n_fresh ? fresh[q] : st.dis[g.poff + p.n_particles - 1 - (q - n_fresh)];
+    dissociate_one<F64>(p, g, st, r, b, e.x, e.y);
+  }
 }
 
-// Dissociation of reaction b (dynamics.py:609-654).
-template <bool F64>
-__global__ void __launch_bounds__(kBlock) k_dissociate(const EdmDynParams* __restrict__ P, DevState st, Match m,
-                                                       int b) {
-  pdl_enter();
-  sweep4(st, m, [&](int r, int64_t s) {
-    const EdmDynParams& p = P[r];
-    const EdmBind& B = p.bind[b];
-    const Geo g(p);
-    const int id = slot_id(st, s) - (int)g.poff;
-    const int partner = st.bond[g.poff + id];
-    if (partner < 0) return;
-    const double u = uniform1(p.seed, *st.d_step, EDM_S_DISSOC + 2 * b, (uint64_t)id, 0);
-    if (!(u < B.prob_dissoc)) return;
-    const int64_t sj = st.slot_of_id[partner];
-    double x, y;
-    abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, s, g, x, y);
-    const uint8_t fj = st.flags[sj];
-    st.flags[s] = fl_make(B.ra, true);
-    st.flags[sj] = fl_make(B.rb, true);
-    const int newc = st.cell_post[s];
-    if constexpr (F64) {
-      ((double2*)st.pos_post)[sj] = ((const double2*)st.pos_post)[s];
-    } else {
-      ((float2*)st.pos_post)[sj] = ((const float2*)st.pos_post)[s];
-      st.lo_post[sj] = st.lo_post[s];
-    }
-    rebucket(st, g, fl_alive(fj) ? st.cell_post[sj] : g.grave, newc);
-    st.cell_post[sj] = newc;
-    note_moved(st, r, p, sj);
-    st.bond[g.poff + id] = -1;
-    st.bond[partner] = -1;
-    grid_change(p, DeltaArray{st.grid_delta}, B.product, true, B.ra, true, x, y);
-    grid_change(p, DeltaArray{st.grid_delta}, fl_species(fj), fl_alive(fj), B.rb, true, x, y);
-    atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_DISSOC], 1);
-  });
-}
-
-// grid_cnt += grid_delta; grid_delta = 0
 // Adaptation field update w += dt/tau_w (rho_PIP3 - w) on every cell of each
 // replica's adaptation grid (dynamics.py:1093-1112, 2227-2242); block row =
 // replica.
@@ -2118,6 +2175,7 @@ __global__ void k_local_cdf(const EdmDynParams* __restrict__ P, const int32_t* c
   local_cdf_of(P[blockIdx.x], cnt, cdf_all, e, tile);
 }
 
+// grid_cnt += grid_delta; grid_delta = 0
 __global__ void k_grid_merge(int32_t* __restrict__ cnt, int32_t* __restrict__ delta, int64_t n) {
   pdl_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {

@@ -42,7 +42,7 @@ int fail(int code, const std::string& msg) { return edm::report_error(code, msg)
     if (_e != cudaSuccess) return fail(EDM_ECUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
-enum PassKind { P_BIND_CAND, P_BIND_APPLY, P_DISSOC, P_CONTACTS, P_CAT, P_REC_CAND, P_REC_APPLY, P_DETACH, P_CONV, P_MERGE,
+enum PassKind { P_BIND_CAND, P_BIND_APPLY, P_CONTACTS, P_CAT, P_REC_CAND, P_REC_APPLY, P_DETACH, P_CONV, P_MERGE,
                 P_GROUP, P_DRAWS, P_ADAPT, P_LOCAL_CDF, P_REACT };
 struct Pass {
   PassKind kind;
@@ -169,6 +169,9 @@ struct EdmEngine {
   uint32_t* status = nullptr;
   int64_t *d_step = nullptr, *d_pstep = nullptr, *d_batch_key = nullptr;
   int32_t *rec_count = nullptr, *rec_id = nullptr, *rec_slot = nullptr, *bind_count = nullptr, *bind_ab = nullptr;
+  int2* dis = nullptr;
+  int32_t* dis_count = nullptr;
+  int dis_parts = 1;  // k_bind_apply's blocks per replica for the dissociations
   double* rec_xy = nullptr;
   int64_t* bind_key = nullptr;
   int32_t *emit_id = nullptr, *emit_n = nullptr, *emit_nd = nullptr, *emit_acc = nullptr;
@@ -266,6 +269,8 @@ struct EdmEngine {
     s.bind_count = bind_count;
     s.bind_key = bind_key;
     s.bind_ab = bind_ab;
+    s.dis = dis;
+    s.dis_count = dis_count;
     s.contacts = contacts;
     s.contact_count = contact_count;
     s.contact_cap = contact_cap;
@@ -356,8 +361,6 @@ struct EdmEngine {
       const EdmBind& B = p.bind[b];
       passes.push_back({P_BIND_CAND, b, match({B.ra}, 1)});
       passes.push_back({P_BIND_APPLY, b, none});
-      passes.push_back({P_DISSOC, b, match({B.product}, 1)});
-      writes({B.ra, B.rb, B.product});
     }
     // adaptation field, after binding and before catalysis (dynamics.py:2227-2242)
     if (p.adapt_grid >= 0) {
@@ -510,7 +513,7 @@ struct EdmEngine {
     draws_early = false;
     if (!(touched & pp_species)) {
       size_t b = 0;
-      while (b < first && (passes[b].kind == P_BIND_CAND || passes[b].kind == P_BIND_APPLY || passes[b].kind == P_DISSOC))
+      while (b < first && (passes[b].kind == P_BIND_CAND || passes[b].kind == P_BIND_APPLY))
         ++b;
       if (b < first) {
         at = b;
@@ -608,7 +611,7 @@ struct EdmEngine {
       return k == P_CAT || k == P_MERGE || k == P_GROUP || k == P_REC_APPLY || k == P_LOCAL_CDF;
     };
     while (start > 0 && fusable(passes[start - 1].kind)) --start;
-    bool pending = hdp[0].n_bind > 0;  // grid changes of passes before the region, in grid_delta
+    bool pending = false;  // grid changes of passes before the region, in grid_delta
     for (size_t i = 0; i < start; ++i) pending |= passes[i].kind == P_CAT;
     if (pending && start < passes.size() && passes[start].kind == P_MERGE) ++start;
     const size_t n = passes.size() - start;
@@ -788,6 +791,7 @@ struct EdmEngine {
     z.p[3] = contact_count, z.n[3] = contact_count ? (rep_contacts ? R : 1) * EDM_MAX_CAT : 0;
     z.p[4] = pl_count, z.n[4] = pl_count ? R : 0;
     z.p[5] = sw_count, z.n[5] = sw_count ? 1 : 0;
+    z.p[6] = dis_count, z.n[6] = dis_count ? (int64_t)R * hdp[0].n_bind * 2 : 0;
     // with proximity FRET the previous step's photon pass reads the bucket
     // starts and the list of particles placed after the sort, cleared here
     if (phot_uses_cells) join_photons(s);
@@ -825,7 +829,8 @@ struct EdmEngine {
       const Pass& ps = passes[i];
       if (pass_prof) cudaEventRecord(pass_prof[i], s);
       // the photon pass reads the flags and bonds that the reactions change
-      if (photons_late && ps.kind != P_CONTACTS && ps.kind != P_DRAWS && ps.kind != P_ADAPT && ps.kind != P_MERGE)
+      if (photons_late && ps.kind != P_BIND_CAND && ps.kind != P_CONTACTS && ps.kind != P_DRAWS &&
+          ps.kind != P_ADAPT && ps.kind != P_MERGE)
         join_photons(s);
       switch (ps.kind) {
         case P_BIND_CAND: {
@@ -834,8 +839,7 @@ struct EdmEngine {
             go(k_bind_candidates<F64, 128, 2, 8>, npblk_bs[t], 128, s, dp, pblk_bs[t], st, ps.match, ps.index);
           break;
         }
-        case P_BIND_APPLY: go(k_bind_apply<F64>, rb, 128, s, dp, R, st, ps.index); break;
-        case P_DISSOC: go(k_dissociate<F64>, sgrid, kBlock, s, dp, st, ps.match, ps.index); break;
+        case P_BIND_APPLY: go(k_bind_apply<F64>, R * (1 + dis_parts), kBindThreads, s, dp, st, ps.index, dis_parts); break;
         case P_CONTACTS:
           tune_mark(TK_CONTACTS, 0, s);
           launch_contacts<F64>(st, ps.match, draws_beside, s);
@@ -1293,6 +1297,14 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
   ALLOC(E->bind_count, n_replicas);
   ALLOC(E->bind_key, (size_t)n_replicas * kBindCap);
   ALLOC(E->bind_ab, (size_t)n_replicas * kBindCap * 2);
+  if (E->hdp[0].n_bind > 0) {
+    ALLOC(E->dis, np);
+    ALLOC(E->dis_count, (size_t)n_replicas * E->hdp[0].n_bind * 2);
+    double most = 0.0;  // bound on a replica's dissociations in a step
+    for (const EdmDynParams& q : E->hdp)
+      for (int b = 0; b < q.n_bind; ++b) most = std::max(most, (double)q.n_particles * q.bind[b].prob_dissoc);
+    E->dis_parts = (int)std::min(64.0, 1.0 + most / kBindThreads);
+  }
   for (const EdmDynParams& q : E->hdp)
     for (int g = 0; g < q.n_grids && g < EDM_MAX_GRIDS; ++g)
       if (q.grid[g].sensor >= 0 && q.grid[g].sensor < EDM_MAX_SPECIES) E->sensor_grids[q.grid[g].sensor] |= 1u << g;

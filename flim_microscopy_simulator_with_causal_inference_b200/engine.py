@@ -291,7 +291,7 @@ class Engine:
                                         _stream_handle(stream)), "edm_profile_steps")
         return dict(zip(self.PROFILE_GROUPS, out.astype(float).tolist()))
 
-    PASS_KINDS = ("bind_candidates", "bind_apply", "dissociation", "contacts", "catalytic", "recruit_candidates",
+    PASS_KINDS = ("bind_candidates", "bind_apply", "contacts", "catalytic", "recruit_candidates",
                   "recruit_apply", "detach", "convert", "grid_merge", "particle_passes", "pass_draws",
                   "adaptation", "local_cdf", "react")
 
