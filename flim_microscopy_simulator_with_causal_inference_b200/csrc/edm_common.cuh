@@ -2,8 +2,8 @@
 //
 // Keyed noise: Philox4x32-10 (Salmon et al., SC'11) with counter
 // (a, b, step_lo, stream<<16 | step_hi) and key = seed; 64-bit words map to
-// uniforms (x >> 11) * 2^-53.  Standard normals come from the Marsaglia polar
-// method with a fixed-order atanh-series logarithm, every float64 operation
+// uniforms (x >> 11) * 2^-53.  Standard normals come from the Box-Muller
+// transform with a fixed-order series logarithm, every float64 operation
 // an explicit round-to-nearest intrinsic (no contraction), so a host
 // implementation that evaluates the same sequence gets the same bits.
 #pragma once

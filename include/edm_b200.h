@@ -332,7 +332,8 @@ int edm_set_photons(EdmEngine* eng, int32_t replica, const int32_t* particle_idx
 
 /* One fused BD step of the whole pipeline loop body (pipeline.py:554-564):
  * dynamics step, photophysics, photon processing; n_steps times, with the
- * launch sequence captured into CUDA graphs of graph_chunk steps. */
+ * launch sequence captured into CUDA graphs of graph_chunk steps (a chunk's
+ * first pass goes without a graph, its second captures it). */
 int edm_pipeline_steps(EdmEngine* eng, int32_t n_steps, int32_t with_photons,
                        int32_t graph_chunk, void* stream);
 
@@ -430,10 +431,11 @@ int edm_ground_truth(EdmEngine* eng, double* fret_E, double* tau_DA,
 int edm_autotune(EdmEngine* eng, int32_t steps_per_shape, int32_t retune, void* stream);
 /* The launch shape in use per tuned kernel: shapes[k][4] = (threads per block,
  * minimum blocks per SM, candidates, chosen candidate; k_scatter candidates
- * 3 and 4 give a thread two and four slots, the others one; k_contacts candidates 0-1
- * gather a tile's sweepers per block, 2-7 sweep a global sweeper list, each
- * with 4, 8 or 16 lanes per sweeper), ms[k][2] = (time of the default shape, time of the chosen shape) from
- * the last tuning (0 if not tuned).  Either pointer may be NULL.  Returns the
+ * 3 and 4 give a thread two and four slots, the others one; k_contacts
+ * candidates 0-1 gather a tile's sweepers per block, 2-7 sweep a global
+ * sweeper list, each with 4, 8 or 16 lanes per sweeper), ms[k][2] = (time of
+ * the default shape, time of the chosen shape) from the last tuning (0 if not
+ * tuned).  Either pointer may be NULL.  Returns the
  * number of tuned kernels (3). */
 int edm_launch_shapes(EdmEngine* eng, int32_t* shapes, float* ms);
 /* Sets the launch shape of each tuned kernel: candidate[k] in
