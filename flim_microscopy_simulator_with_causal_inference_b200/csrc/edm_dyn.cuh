@@ -603,10 +603,12 @@ __global__ void k_scan_reduce(const int32_t* __restrict__ cnt, int64_t n, int32_
 // replica's slots are contiguous, so its bucket starts count from its first
 // slot): the block holds its counts in registers, a warp 128 of them per round.
 // One launch of latency instead of three: a 5,000-slot system's scan 10.5 to 8 us,
-// 24 replicas of 207,000 slots 12.1 to 10.6, 148 replicas of 880,000 slots 12.8 to
-// 11.2.  With more replicas than SMs the blocks take turns and the gain is gone
-// (16.0 and 16.0 us at 296 replicas, 15.1 against 17.6 at 600), so the tiled scan
-// over all cells stays there and above kSmallScan cells a replica.
+// its whole step 25.0 to 23.7, one of 13,600 slots 27.5 to 27.1, 100 replicas of
+// 538,000 65.1 to 64.2.  At 15,700 slots in one replica the two are even (29.8 and
+// 29.7 us in float64, 27.1 and 27.7 in float32), with six rounds instead of four
+// 22,900 slots take 33.0 us against 31.4 tiled: the line lies between.  With more
+// replicas than SMs the blocks take turns and the gain is gone as well (scans of
+// 16.0 and 16.0 us at 296 replicas, 17.6 against 15.1 at 600).
 constexpr int kSmallScanRounds = 4;
 constexpr int kSmallScan = 1024 * 4 * kSmallScanRounds - 4;
 __global__ void __launch_bounds__(1024) k_scan_replica(const EdmDynParams* __restrict__ P, int32_t* cnt,
