@@ -77,8 +77,9 @@ struct DevState {
   int64_t* bind_key;     // [R][kBindCap]
   int32_t* bind_ab;      // [R][kBindCap][2] local ids (a = reactant A role, b = B role)
   // complexes that dissociate in the binding pass (slot, partner's slot), replica
-  // r's from its particle_offset up, those whose partner is alive (no binding
-  // leaves one so, but a state may hold one) from its last particle down
+  // r's from its particle_offset up; from its last particle down the odd ones,
+  // whose partner is alive or bound to another (no binding leaves one so, but a
+  // state may hold one)
   int2* dis;
   int32_t* dis_count;    // [binding reactions][R][2]
   // catalytic contacts of the step: (enzyme slot, substrate-capable slot),
@@ -1931,9 +1932,10 @@ __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __r
     const int id = slot_id(st, s) - (int)p.particle_offset;
     const int partner = st.bond[p.particle_offset + id];
     if (partner < 0 || !dissociates(p, st, b, id)) continue;
-    const int sj = st.slot_of_id[partner], awake = fl_alive(st.flags[sj]) ? 1 : 0;
-    const int q = atomicAdd(&st.dis_count[(b * st.n_rep + r) * 2 + awake], 1);
-    st.dis[awake ? end - 1 - q : p.particle_offset + q] = make_int2((int)s, sj);
+    const int sj = st.slot_of_id[partner], back = st.bond[partner];
+    const int odd = fl_alive(st.flags[sj]) || back != p.particle_offset + id ? 1 : 0;
+    const int q = atomicAdd(&st.dis_count[(b * st.n_rep + r) * 2 + odd], 1);
+    st.dis[odd ? end - 1 - q : p.particle_offset + q] = make_int2((int)s, sj);
   }
   if (sweepers == 0) return;
   const EdmBind& B = p.bind[b];
@@ -1974,14 +1976,25 @@ __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __r
 }
 
 // Dissociation of the complex in slot s, its partner in slot sj, of reaction b.
+// Odd: the partner may be alive (and the complex itself), else it is dormant.
 // The binding passes change the grid counts at once: none of them reads them.
-template <bool F64>
+template <bool F64, bool Odd>
 __device__ __forceinline__ void dissociate_one(const EdmDynParams& p, const Geo& g, const DevState& st, int r, int b,
                                                int64_t s, int64_t sj) {
   const EdmBind& B = p.bind[b];
+  const DeltaArray sink{st.grid_cnt};
   double x, y;
   abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, s, g, x, y);
-  const uint8_t fj = st.flags[sj];
+  int from = g.grave;
+  if constexpr (Odd) {
+    const uint8_t fj = s == sj ? fl_make(B.ra, true) : st.flags[sj];
+    if (fl_alive(fj)) {  // an alive partner is counted where it stands
+      double xj, yj;
+      abs_pos<F64>(st.pos_post, st.lo_post, st.cell_post, sj, g, xj, yj);
+      grid_add(p, sink, fl_species(fj), xj, yj, -1);
+      from = st.cell_post[sj];
+    }
+  }
   st.flags[s] = fl_make(B.ra, true);
   st.flags[sj] = fl_make(B.rb, true);
   const int newc = st.cell_post[s];
@@ -1991,22 +2004,64 @@ __device__ __forceinline__ void dissociate_one(const EdmDynParams& p, const Geo&
     ((float2*)st.pos_post)[sj] = ((const float2*)st.pos_post)[s];
     st.lo_post[sj] = st.lo_post[s];
   }
-  rebucket(st, g, fl_alive(fj) ? st.cell_post[sj] : g.grave, newc);
+  rebucket(st, g, from, newc);
   st.cell_post[sj] = newc;
   note_moved(st, r, p, sj);
   st.bond[slot_id(st, s)] = -1;
   st.bond[slot_id(st, sj)] = -1;
-  grid_change(p, DeltaArray{st.grid_cnt}, B.product, true, B.ra, true, x, y);
-  grid_change(p, DeltaArray{st.grid_cnt}, fl_species(fj), fl_alive(fj), B.rb, true, x, y);
+  grid_change(p, sink, B.product, true, B.ra, true, x, y);
+  grid_add(p, sink, B.rb, x, y, +1);
   atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_DISSOC], 1);
+}
+
+// The dissociations of a replica that holds odd complexes, by one block: in
+// particle order, one after the other, each by the state the earlier ones left,
+// as the reference's loop (dynamics.py:609-654).  Complexes that share a partner
+// both dissociate and the last one places it; one whose partner is a complex
+// itself may end that one's bond.  Taken side by side, two of them would take the
+// shared partner out of its bucket twice, and the next sort would write past the
+// bucket.  Lists: n plain and n_odd odd entries of st.dis, and n_fresh of the
+// pass's new complexes.  Rare, so no faster than one dissociation at a time.
+template <bool F64>
+__device__ __noinline__ void dissociate_in_order(const EdmDynParams& p, const DevState& st, int r, int b, int n,
+                                                 int n_odd, int2* fresh, int n_fresh) {
+  const Geo g(p);
+  int2* plain = st.dis + p.particle_offset;
+  int2* odd = st.dis + p.particle_offset + p.n_particles - 1;
+  const int total = n + n_odd + n_fresh;
+  auto at = [&](int q) -> int2& {
+    return q < n ? plain[q] : (q < n + n_odd ? *(odd - (q - n)) : fresh[q - n - n_odd]);
+  };
+  for (int q = threadIdx.x; q < total; q += blockDim.x) at(q).x = slot_id(st, at(q).x);
+  __syncthreads();
+  // bitonic merges with every comparison ascending: positions past the end need no partner
+  for (int64_t k = 2; k < 2 * (int64_t)total; k <<= 1)
+    for (int64_t j = k - 1; j > 0; j = j == k - 1 ? k >> 2 : j >> 1) {
+      for (int q = threadIdx.x; q < total; q += blockDim.x) {
+        const int64_t o = q ^ j;
+        if (o <= q || o >= total) continue;
+        const int2 lo = at(q), hi = at((int)o);
+        if (lo.x <= hi.x) continue;
+        at(q) = hi;
+        at((int)o) = lo;
+      }
+      __syncthreads();
+    }
+  if (threadIdx.x != 0) return;
+  for (int q = 0; q < total; ++q) {
+    const int id = at(q).x, s = st.slot_of_id[id], partner = st.bond[id];
+    if (partner < 0 || st.flags[s] != fl_make(p.bind[b].product, true)) continue;
+    dissociate_one<F64, true>(p, g, st, r, b, s, st.slot_of_id[partner]);
+  }
 }
 
 // Reaction b after its candidates, 1 + `parts` blocks per replica.  The first
 // applies the replica's candidates in pair order, each unless an earlier one took
 // one of its particles, and dissociates the new complexes whose draw says so; the
-// others dissociate the listed ones, which no candidate touches (the particles
-// were bound or dormant at the pass's start; one with a partner alive waits for
-// the candidates).  What bounds it is round trips, so
+// others dissociate the listed ones, which neither a candidate nor another entry
+// touches (their particles were bound to one another, the partner dormant, at the
+// pass's start).  With an odd entry (DevState::dis) the first block takes all of
+// them after its candidates, in order.  What bounds it is round trips, so
 // the candidates' state is fetched for all at once and their order settled in
 // shared memory, where a candidate waits only for earlier ones that share a
 // particle with it.  One thread per replica taking one candidate after the other,
@@ -2015,8 +2070,8 @@ __device__ __forceinline__ void dissociate_one(const EdmDynParams& p, const Geo&
 // 714,000 (150 candidates a step).
 constexpr int kBindThreads = 256;
 template <bool F64>
-__global__ void __launch_bounds__(kBindThreads, 4) k_bind_apply(const EdmDynParams* __restrict__ P, DevState st, int b,
-                                                           int parts) {
+__global__ void __launch_bounds__(kBindThreads, 4) k_bind_apply(const EdmDynParams* __restrict__ P,
+                                                           const __grid_constant__ DevState st, int b, int parts) {
   __shared__ int64_t key[kBindCap];
   __shared__ int2 pair[kBindCap];  // in pair order
   __shared__ int8_t state[kBindCap];
@@ -2029,17 +2084,17 @@ __global__ void __launch_bounds__(kBindThreads, 4) k_bind_apply(const EdmDynPara
   pdl_enter();
   const EdmBind& B = p.bind[b];
   const Geo g(p);
-  const int32_t* dis_count = st.dis_count + (b * st.n_rep + r) * 2;
+  const int2 listed = ((const int2*)st.dis_count)[b * st.n_rep + r];  // plain, odd
   if (part > 0) {
-    const int nd = *dis_count;
-    for (int q = (part - 1) * kBindThreads + tid; q < nd; q += parts * kBindThreads) {
+    if (listed.y > 0) return;
+    for (int q = (part - 1) * kBindThreads + tid; q < listed.x; q += parts * kBindThreads) {
       const int2 e = st.dis[g.poff + q];
-      dissociate_one<F64>(p, g, st, r, b, e.x, e.y);
+      dissociate_one<F64, false>(p, g, st, r, b, e.x, e.y);
     }
     return;
   }
-  const int n = min(st.bind_count[r], kBindCap), n_awake = dis_count[1];
-  if (n == 0 && n_awake == 0) return;
+  const int n = min(st.bind_count[r], kBindCap);
+  if (n == 0 && listed.y == 0) return;
   for (int i = tid; i < n; i += kBindThreads) key[i] = st.bind_key[(int64_t)r * kBindCap + i];
   if (tid == 0) n_fresh = n_bound = 0;
   __syncthreads();
@@ -2091,10 +2146,11 @@ __global__ void __launch_bounds__(kBindThreads, 4) k_bind_apply(const EdmDynPara
   }
   __syncthreads();
   if (tid == 0) atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_BINDINGS], n_bound);
-  for (int q = tid; q < n_fresh + n_awake; q += kBindThreads) {
-    const int2 e = q < n_fresh ? fresh[q] : st.dis[g.poff + p.n_particles - 1 - (q - n_fresh)];
-    dissociate_one<F64>(p, g, st, r, b, e.x, e.y);
+  if (listed.y > 0) {
+    dissociate_in_order<F64>(p, st, r, b, listed.x, listed.y, fresh, n_fresh);
+    return;
   }
+  for (int q = tid; q < n_fresh; q += kBindThreads) dissociate_one<F64, false>(p, g, st, r, b, fresh[q].x, fresh[q].y);
 }
 
 // Adaptation field update w += dt/tau_w (rho_PIP3 - w) on every cell of each
