@@ -1169,7 +1169,10 @@ __global__ void __launch_bounds__(BS, MINB) k_move(const EdmDynParams* __restric
 //   alive particles of the sweeping species (E_c or S_c) visit their
 //   neighbour cells for the other species.  Both distance tests are
 //   symmetric in the two particles (the float32 differences change sign
-//   exactly), so either side finds the same pairs;
+//   exactly), so either side finds the same pairs.  A particle that a
+//   dissociation of the step woke lies in the bucket of the non-alive ones,
+//   where no neighbour sweep meets it: woken_contacts looks from it for the
+//   sweepers around the cell it was sorted from;
 // * late pairs, whose partner an earlier catalytic pass of the step turns
 //   into S_c, are few: the pass that converts a particle looks up its
 //   enzymes of the later reactions at once (late_contacts).
@@ -1183,6 +1186,8 @@ struct CatLists {
   uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   uint32_t partners[EDM_MAX_SPECIES];  // species the sweeper species looks for
   uint32_t from_enzyme;                // reactions swept from the enzyme side
+  uint32_t woken;                      // a dissociation can wake a species that sweeps look for: bit 0; among those
+                                       // a sweeping one: bit 1
 };
 static_assert(EDM_MAX_CAT <= 8, "rx_of holds a reaction set per byte");
 
@@ -1347,6 +1352,35 @@ __device__ __forceinline__ void finish_contacts(const EdmDynParams* __restrict__
   }
 }
 
+// Adds the pair (s, j) of replica r to the warp's queue in the lanes with `hit`
+// (every lane of the warp calls it); 32 waiting pairs are finished at once.
+template <bool F64>
+__device__ __forceinline__ void queue_contact(const EdmDynParams* __restrict__ P, const DevState& st,
+                                              const CatLists& L, const uint8_t* rx_of, bool hit, int s, int j, int r,
+                                              ContactQueue& Q, int& queued) {
+  const int lane = threadIdx.x & 31;
+  const unsigned who = __ballot_sync(0xffffffffu, hit);
+  if (!who) return;
+  if (hit) {
+    const int at = queued + __popc(who & ((1u << lane) - 1u));
+    Q.pair[at] = make_int2(s, j);
+    Q.rep[at] = r;
+  }
+  queued += __popc(who);
+  __syncwarp();
+  if (queued < 32) return;  // at most 31 + 32 wait here
+  finish_contacts<F64>(P, st, L, rx_of, Q, 32);
+  __syncwarp();
+  queued -= 32;
+  if (lane < queued) {
+    const int2 e = Q.pair[32 + lane];
+    const int32_t k = Q.rep[32 + lane];
+    Q.pair[lane] = e;
+    Q.rep[lane] = k;
+  }
+  __syncwarp();
+}
+
 // Sweeper s of replica r (one per group of G lanes, `have` false for a group
 // without one) against its neighbour slots: alive, of a species it sweeps
 // for, within the pre-move cutoff.  The pairs go to the warp's queue, `queued`
@@ -1357,7 +1391,6 @@ __device__ __forceinline__ void contact_sweep(const EdmDynParams* __restrict__ P
                                               ContactQueue& Q, int& queued) {
   const EdmDynParams& p = P[r];
   const Geo g(p);
-  const int lane = threadIdx.x & 31;
   const uint32_t pmask = L.partners[fl_species(st.flags[s])];
   const int c_pre = st.cell_pre[s];
   float2 oi = make_float2(0.f, 0.f);
@@ -1386,27 +1419,46 @@ __device__ __forceinline__ void contact_sweep(const EdmDynParams* __restrict__ P
               __fmaf_rn(fdx, fdx, fdy * fdy) < cutoff_f;
       }
     }
-    const unsigned who = __ballot_sync(0xffffffffu, hit);
-    if (!who) return;
-    if (hit) {
-      const int at = queued + __popc(who & ((1u << lane) - 1u));
-      Q.pair[at] = make_int2(s, j);
-      Q.rep[at] = r;
-    }
-    queued += __popc(who);
-    __syncwarp();
-    if (queued < 32) return;  // at most 31 + 32 wait here
-    finish_contacts<F64>(P, st, L, rx_of, Q, 32);
-    __syncwarp();
-    queued -= 32;
-    if (lane < queued) {
-      const int2 e = Q.pair[32 + lane];
-      const int32_t k = Q.rep[32 + lane];
-      Q.pair[lane] = e;
-      Q.rep[lane] = k;
-    }
-    __syncwarp();
+    queue_contact<F64>(P, st, L, rx_of, hit, s, j, r, Q, queued);
   });
+}
+
+// The contacts that the neighbour sweeps cannot meet: particles that this step's
+// binding passes woke (st.moved; nobody else has been placed yet), as the
+// neighbour of a sweeper.  The warp's groups of G lanes take a woken particle
+// each, part `part` of `parts` of the replica's, and walk the sweepers among its
+// neighbours and, where a woken particle can be one, among the woken.  One that
+// was alive before as well is met twice, which a pass does not mind.
+template <bool F64, int G>
+__device__ __noinline__ void woken_contacts(const EdmDynParams* __restrict__ P, const DevState& st, const CatLists& L,
+                                            const uint8_t* rx_of, int r, int part, int parts, ContactQueue& Q) {
+  const EdmDynParams& p = P[r];
+  const Geo g(p);
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int32_t* woken = st.moved + p.particle_offset;
+  const int n = min(st.moved_count[r], (int)p.n_particles);
+  int queued = 0;
+  for (int t0 = (part * warps + (threadIdx.x >> 5)) * (32 / G); t0 < n; t0 += parts * warps * (32 / G)) {
+    const int t = t0 + lane / G;
+    const int w = woken[t < n ? t : t0];
+    const uint8_t fw = st.flags[w];
+    const bool have = t < n && fl_alive(fw);
+    auto meets = [&](int j) {
+      const uint8_t fj = st.flags[j];
+      return fl_alive(fj) && j != w && rx_of[fl_species(fj) * EDM_MAX_SPECIES + fl_species(fw)] != 0 &&
+             sep_sq<F64>(st.pos_pre, st.cell_pre, j, w, g) < g.cutoff_sq();
+    };
+    for_neighbour_slots_grouped<G>(g, st, st.cell_pre[w], have, [&](int j, bool valid, int, int) {
+      queue_contact<F64>(P, st, L, rx_of, valid && meets(j), j, w, r, Q, queued);
+    });
+    if (!(L.woken & 2u)) continue;
+    for (int k0 = 0; k0 < n; k0 += G) {
+      const int k = k0 + (lane & (G - 1));
+      const int j = woken[min(k, n - 1)];
+      queue_contact<F64>(P, st, L, rx_of, have && k < n && meets(j), j, w, r, Q, queued);
+    }
+  }
+  finish_contacts<F64>(P, st, L, rx_of, Q, queued);
 }
 
 // ---- per-particle passes: recruitment candidates, detachments, conversions ----
@@ -1482,16 +1534,27 @@ __device__ __forceinline__ void draw_slot(const EdmDynParams& p, const DevState&
 // gathers its sweepers in shared memory.  One launch and one block's chain:
 // the form for systems that do not fill the chip.  With a draw plan D as many
 // blocks again take the tiles' draws (the draw sweep, k_pass_draws, beside the
-// search without a stream of its own).
+// search without a stream of its own); blocks beyond those, woken_parts per
+// replica, take the woken particles.
 template <bool F64, int BLK, int SPT, int G, int MINB>
 __global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __restrict__ P,
-                                                      const int2* __restrict__ blk, int ntiles, DevState st, Match m,
+                                                      const int2* __restrict__ blk, int ntiles,
+                                                      const __grid_constant__ DevState st, Match m,
                                                       const __grid_constant__ CatLists L,
-                                                      const DrawPlan* __restrict__ D, Match any) {
+                                                      const DrawPlan* __restrict__ D, Match any, int woken_parts) {
   __shared__ int32_t list[BLK * SPT];
   __shared__ ContactQueue queue[BLK / 32];
   __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   __shared__ int n_list;
+  const int woken = (int)blockIdx.x - (D ? 2 * ntiles : ntiles);
+  if (woken >= 0) {
+    if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
+    pdl_enter();
+    __syncthreads();
+    woken_contacts<F64, G>(P, st, L, (const uint8_t*)rx_of, woken / woken_parts, woken % woken_parts, woken_parts,
+                           queue[threadIdx.x >> 5]);
+    return;
+  }
   const bool draws = (int)blockIdx.x >= ntiles;
   const int2 b = blk[draws ? (int)blockIdx.x - ntiles : (int)blockIdx.x];
   const int64_t end = P[b.x].particle_offset + P[b.x].n_particles;
@@ -1537,19 +1600,28 @@ __global__ void __launch_bounds__(kBlock) k_sweep_list(const EdmDynParams* __res
   for (int k = threadIdx.x; k < n; k += kBlock) st.sw_list[at + k] = make_int2(list[k], b.x);
 }
 
-// The same sweep over the global list, one wave of blocks: no per-tile
+// The same sweep over the global list, one wave of sweep_blocks blocks (those
+// beyond take the woken particles): no per-tile
 // prologue and every group has a sweeper until the list ends, which pays when
 // the sweepers outnumber the chip's groups several times.
 template <bool F64, int G, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynParams* __restrict__ P, DevState st,
-                                                              const __grid_constant__ CatLists L) {
+__global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynParams* __restrict__ P,
+                                                              const __grid_constant__ DevState st,
+                                                              const __grid_constant__ CatLists L, int sweep_blocks,
+                                                              int woken_parts) {
   __shared__ ContactQueue queue[kBlock / 32];
   __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
   pdl_enter();
   __syncthreads();
+  if ((int)blockIdx.x >= sweep_blocks) {
+    const int woken = (int)blockIdx.x - sweep_blocks;
+    woken_contacts<F64, G>(P, st, L, (const uint8_t*)rx_of, woken / woken_parts, woken % woken_parts, woken_parts,
+                           queue[threadIdx.x >> 5]);
+    return;
+  }
   const int n = *st.sw_count, lane = threadIdx.x & 31;
-  const int stride = (int)gridDim.x * (kBlock / G);
+  const int stride = sweep_blocks * (kBlock / G);
   ContactQueue& Q = queue[threadIdx.x >> 5];
   int queued = 0;
   int t0 = (int)(blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * (32 / G);
@@ -1569,36 +1641,49 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynPara
 // substrate of the later reactions `late`: its alive neighbours of those
 // reactions' enzyme species passing the tests an enzyme-side sweep makes
 // (j seen from enzyme e at the opposite cell offset, the same float32
-// expressions), appended to the reactions' lists.
+// expressions), and its neighbours among the particles woken in the step, which
+// the cells do not hold; appended to the reactions' lists.
 template <bool F64>
 __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
                                            int64_t j, int id_j, int64_t step, uint32_t late,
                                            const ContactOut& out) {
   uint32_t emask = 0;
   for (uint32_t b = late; b; b &= b - 1) emask |= 1u << p.cat[__ffs(b) - 1].enzyme;
-  for_neighbour_slots(g, st, st.cell_pre[j], [&](int e, int, int dcx, int dcy) {
-    if (e == j) return;
-    const uint8_t fe = st.flags[e];
-    const int spe = fl_species(fe);
-    if (!fl_alive(fe) || !((emask >> spe) & 1u)) return;
-    double d2;
-    if constexpr (F64) {
-      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())) return;
-      d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
-    } else {
-      const float2 oe = ((const float2*)st.pos_pre)[e], oj = ((const float2*)st.pos_pre)[j];
-      const float fdx = __fmaf_rn(-(float)(-dcx), g.sxf, oe.x - oj.x);
-      const float fdy = __fmaf_rn(-(float)(-dcy), g.syf, oe.y - oj.y);
-      if (!((double)__fmaf_rn(fdx, fdx, fdy * fdy) < g.cutoff_sq())) return;
-      d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
-    }
+  auto file = [&](int e, int spe) {
+    const double d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
     for (uint32_t b = late; b; b &= b - 1) {
       const int c = __ffs(b) - 1;
       if (spe != p.cat[c].enzyme || d2 > p.cat[c].contact_sq) continue;
       if (!cat_draw_passes(p, st, r, c, slot_id(st, e) - (int)g.poff, id_j, step)) continue;
       out.file(c, e, (int)j);
     }
+  };
+  for_neighbour_slots(g, st, st.cell_pre[j], [&](int e, int, int dcx, int dcy) {
+    if (e == j) return;
+    const uint8_t fe = st.flags[e];
+    const int spe = fl_species(fe);
+    if (!fl_alive(fe) || !((emask >> spe) & 1u)) return;
+    if constexpr (F64) {
+      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())) return;
+    } else {
+      const float2 oe = ((const float2*)st.pos_pre)[e], oj = ((const float2*)st.pos_pre)[j];
+      const float fdx = __fmaf_rn(-(float)(-dcx), g.sxf, oe.x - oj.x);
+      const float fdy = __fmaf_rn(-(float)(-dcy), g.syf, oe.y - oj.y);
+      if (!((double)__fmaf_rn(fdx, fdx, fdy * fdy) < g.cutoff_sq())) return;
+    }
+    file(e, spe);
   });
+  uint32_t woken = 0;  // enzyme species that a dissociation can wake
+  for (int b = 0; b < p.n_bind; ++b) woken |= emask & (1u << p.bind[b].rb);
+  if (!woken) return;
+  const int n = min(st.moved_count[r], (int)p.n_particles);
+  for (int k = 0; k < n; ++k) {
+    const int e = st.moved[p.particle_offset + k];
+    const uint8_t fe = st.flags[e];
+    if (e != j && fl_alive(fe) && ((woken >> fl_species(fe)) & 1u) &&
+        sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())
+      file(e, fl_species(fe));
+  }
 }
 
 // Catalytic pass c (dynamics.py:825-983) over its contact list: the set of
@@ -1901,6 +1986,70 @@ __device__ __forceinline__ bool dissociates(const EdmDynParams& p, const DevStat
   return uniform1(p.seed, *st.d_step, EDM_S_DISSOC + 2 * b, (uint64_t)id, 0) < p.bind[b].prob_dissoc;
 }
 
+// Lists the candidate of particles id and idj (unlike, of the reaction's two
+// species, id's the one swept from; in contact before and after the move) when
+// idj is unbound and the pair's draw says so; offset(): the cell offset from id's
+// slot to idj's.
+template <typename Offset>
+__device__ __forceinline__ void list_candidate(const EdmDynParams& p, const Geo& g, const DevState& st, int r, int b,
+                                               int id, int idj, bool swept_ra, Offset offset) {
+  if (st.bond[g.poff + idj] >= 0) return;
+  const int lo = id < idj ? id : idj, hi = id < idj ? idj : id;
+  const double u = uniform1(p.seed, *st.d_step, EDM_S_BIND + 2 * b, (uint64_t)lo, (uint64_t)hi);
+  if (!(u < p.bind[b].prob_bind)) return;
+  int2 d = offset();
+  if (lo != id) d.x = -d.x, d.y = -d.y;
+  const int ordinal = (d.x + 1) * 3 + d.y + 1;
+  const int k = atomicAdd(&st.bind_count[r], 1);
+  if (k < kBindCap) {
+    st.bind_key[(int64_t)r * kBindCap + k] =
+        ((int64_t)lo << 36) | ((int64_t)ordinal << 32) | (int64_t)(0xFFFFFFFFu - (uint32_t)hi);
+    st.bind_ab[((int64_t)r * kBindCap + k) * 2] = swept_ra ? id : idj;
+    st.bind_ab[((int64_t)r * kBindCap + k) * 2 + 1] = swept_ra ? idj : id;
+  } else {
+    set_status(st.status, EDM_STATUS_BIND_CAP);
+  }
+}
+
+// Binding candidates whose unswept particle an earlier reaction of the step woke
+// (see woken_contacts): from the woken particle to the swept species m among its
+// neighbours and among the woken.  Of a homodimer's pairs the woken one's own
+// sweep has those with a higher partner in the cells.
+template <bool F64, int G>
+__device__ __noinline__ void woken_candidates(const EdmDynParams& p, const DevState& st, const Match& m, int r, int b,
+                                              int part, int parts) {
+  const Geo g(p);
+  const EdmBind& B = p.bind[b];
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int32_t* woken = st.moved + p.particle_offset;
+  const int n = min(st.moved_count[r], (int)p.n_particles);
+  const int swept = (m.mask[1] >> B.ra) & 1u ? B.ra : B.rb, other = swept == B.ra ? B.rb : B.ra;
+  for (int t0 = (part * warps + (threadIdx.x >> 5)) * (32 / G); t0 < n; t0 += parts * warps * (32 / G)) {
+    const int t = t0 + lane / G;
+    const int w = woken[t < n ? t : t0], idw = slot_id(st, w) - g.poff;
+    const bool have = t < n && st.flags[w] == fl_make(other, true) && st.bond[g.poff + idw] < 0;
+    auto meet = [&](int j) {
+      if (j == w || st.flags[j] != fl_make(swept, true)) return;
+      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, j, w, g) < g.cutoff_sq())) return;
+      if (sep_sq<F64>(st.pos_post, st.cell_post, j, w, g) > B.contact_sq) return;
+      const int idj = slot_id(st, j) - g.poff;
+      if (swept == other && idj > idw) return;
+      if (st.bond[g.poff + idj] >= 0) return;
+      list_candidate(p, g, st, r, b, idj, idw, swept == B.ra, [&] {
+        int xj, yj, xw, yw;
+        split_cell(st.cell_pre[j], g, xj, yj);
+        split_cell(st.cell_pre[w], g, xw, yw);
+        const int dx = xw - xj, dy = yw - yj;
+        return make_int2(dx > 1 ? dx - g.nx : (dx < -1 ? dx + g.nx : dx), dy > 1 ? dy - g.ny : (dy < -1 ? dy + g.ny : dy));
+      });
+    };
+    for_neighbour_slots_grouped<G>(g, st, st.cell_pre[w], have, [&](int j, bool valid, int, int) {
+      if (valid) meet(j);
+    });
+    for (int k = lane & (G - 1); have && k < n; k += G) meet(woken[k]);
+  }
+}
+
 // Binding candidates of reaction b (dynamics.py:528-606): pairs (i < j)
 // passing every test of the pass-start state, keyed by the reference's pair
 // order (i, neighbour-cell ordinal seen from i, descending j).  Swept from one
@@ -1908,12 +2057,21 @@ __device__ __forceinline__ bool dissociates(const EdmDynParams& p, const DevStat
 // tile of BLK * SPT slots per block, G lanes per sweeper, as the contact search;
 // with both species swept slot by slot in a lane each the pass was 36 us for a
 // 13,900-slot sensor membrane.  The tile's complexes draw for their dissociation
-// on the way (st.dis).
+// on the way (st.dis).  Blocks beyond the tiles, woken_parts per replica, take the
+// woken particles.
 template <bool F64, int BLK, int SPT, int G>
 __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __restrict__ P,
-                                                         const int2* __restrict__ blk, DevState st, Match m, int b) {
+                                                         const int2* __restrict__ blk, int ntiles,
+                                                         const __grid_constant__ DevState st,
+                                                         const __grid_constant__ Match m, int b, int woken_parts) {
   __shared__ int32_t list[BLK * SPT];
   __shared__ int n_list;
+  if ((int)blockIdx.x >= ntiles) {
+    const int woken = (int)blockIdx.x - ntiles;
+    pdl_enter();
+    woken_candidates<F64, G>(P[woken / woken_parts], st, m, woken / woken_parts, b, woken % woken_parts, woken_parts);
+    return;
+  }
   const int2 tile = blk[blockIdx.x];
   const int r = tile.x;
   const EdmDynParams& p = P[r];
@@ -1954,23 +2112,8 @@ __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __r
       if (sep_sq<F64>(st.pos_post, st.cell_post, s, j, g) > B.contact_sq) return;
       const int idj = slot_id(st, j) - g.poff;
       if (B.ra == B.rb && idj < id) return;  // seen from the other particle
-      if (st.bond[g.poff + idj] >= 0) return;
-      const int lo = id < idj ? id : idj, hi = id < idj ? idj : id;
-      const double u = uniform1(p.seed, *st.d_step, EDM_S_BIND + 2 * b, (uint64_t)lo, (uint64_t)hi);
-      if (!(u < B.prob_bind)) return;
-      int dcx = column - 1, dcy = row_offset(st.cell_pre[j] - base, g);
-      if (lo != id) dcx = -dcx, dcy = -dcy;
-      const int ordinal = (dcx + 1) * 3 + dcy + 1;
-      const bool swept_ra = other == B.rb;
-      const int k = atomicAdd(&st.bind_count[r], 1);
-      if (k < kBindCap) {
-        st.bind_key[(int64_t)r * kBindCap + k] =
-            ((int64_t)lo << 36) | ((int64_t)ordinal << 32) | (int64_t)(0xFFFFFFFFu - (uint32_t)hi);
-        st.bind_ab[((int64_t)r * kBindCap + k) * 2] = swept_ra ? id : idj;
-        st.bind_ab[((int64_t)r * kBindCap + k) * 2 + 1] = swept_ra ? idj : id;
-      } else {
-        set_status(st.status, EDM_STATUS_BIND_CAP);
-      }
+      list_candidate(p, g, st, r, b, id, idj, other == B.rb,
+                     [&] { return make_int2(column - 1, row_offset(st.cell_pre[j] - base, g)); });
     });
   }
 }

@@ -448,6 +448,22 @@ struct EdmEngine {
         ps.match = Match{{0u, 1u << (count && count[rb] < count[ra] ? rb : ra)}};
       }
     }
+    const uint32_t woken = woken_species(p.n_bind);
+    for (int sp = 0; sp < EDM_MAX_SPECIES; ++sp)
+      if (cat_lists.partners[sp] & woken) cat_lists.woken |= (woken >> sp) & 1u ? 3u : 1u;
+  }
+
+  // Species that the dissociations of the first n binding reactions wake.
+  uint32_t woken_species(int n) const {
+    uint32_t m = 0;
+    for (int b = 0; b < n; ++b) m |= 1u << hdp[0].bind[b].rb;
+    return m;
+  }
+  // Whether an earlier reaction of the step can wake the unswept species of a binding pass.
+  bool woken_can_bind(const Pass& ps) const {
+    const EdmBind& B = hdp[0].bind[ps.index];
+    const int other = (ps.match.mask[1] >> B.ra) & 1u ? B.rb : B.ra;
+    return (woken_species(ps.index) >> other) & 1u;
   }
 
   // The per-particle passes (recruitment candidates, detachments,
@@ -755,14 +771,16 @@ struct EdmEngine {
     constexpr int slots = kContactSlots[K], lanes = kContactLanes[K];
     const int t = tile_index(slots > 0 ? sh.block * slots : kBlock * kSweepSlots);
     if (npblk_bs[t] == 0) return;
+    const int woken = cat_lists.woken ? R * dis_parts : 0;
     if constexpr (slots > 0) {
       const int nt = npblk_bs[t];
-      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, with_draws ? 2 * nt : nt, sh.block, s, dp, pblk_bs[t], nt,
-         st, m, cat_lists, with_draws ? d_draw : nullptr, draw.any);
+      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, (with_draws ? 2 * nt : nt) + woken, sh.block, s, dp,
+         pblk_bs[t], nt, st, m, cat_lists, with_draws ? d_draw : nullptr, draw.any, dis_parts);
     } else {
       static_assert(sh.block == kBlock, "the list form's blocks");
       go(k_sweep_list, npblk_bs[t], kBlock, s, dp, pblk_bs[t], st, m);
-      go(k_contacts_list<F64, lanes, sh.min_blocks>, 148 * sh.min_blocks, kBlock, s, dp, st, cat_lists);
+      constexpr int sweep = 148 * sh.min_blocks;
+      go(k_contacts_list<F64, lanes, sh.min_blocks>, sweep + woken, kBlock, s, dp, st, cat_lists, sweep, dis_parts);
     }
   }
 
@@ -836,7 +854,8 @@ struct EdmEngine {
         case P_BIND_CAND: {
           const int t = tile_index(kBlock);
           if (npblk_bs[t] > 0)
-            go(k_bind_candidates<F64, 128, 2, 8>, npblk_bs[t], 128, s, dp, pblk_bs[t], st, ps.match, ps.index);
+            go(k_bind_candidates<F64, 128, 2, 8>, npblk_bs[t] + (woken_can_bind(ps) ? R * dis_parts : 0), 128, s, dp,
+               pblk_bs[t], npblk_bs[t], st, ps.match, ps.index, dis_parts);
           break;
         }
         case P_BIND_APPLY: go(k_bind_apply<F64>, R * (1 + dis_parts), kBindThreads, s, dp, st, ps.index, dis_parts); break;
