@@ -70,6 +70,7 @@ __device__ __forceinline__ void copies_wait() {
 constexpr int kReadoutWarps = 12, kGroup = 8, kStages = 2;
 
 __device__ __host__ constexpr int row_words(int nq) { return nq + (12 - nq % 8) % 8; }  // = 4 mod 8, at least nq
+constexpr size_t stage_bytes(int nq) { return sizeof(uint4) * kReadoutWarps * kStages * kGroup * row_words(nq); }
 
 // NQ: n_bins / 4 when known to the compiler (128 and 256 bins), else 0.
 template <int NQ>
@@ -185,9 +186,12 @@ extern "C" int edm_readout_lifetimes(const uint32_t* stack_dev, int64_t n_px, in
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t smem = sizeof(uint4) * kReadoutWarps * kStages * kGroup * row_words(n_bins / 4);
+  const size_t smem = stage_bytes(n_bins / 4);
   const auto kernel = n_bins == 256 ? k_readout<64> : (n_bins == 128 ? k_readout<32> : k_readout<0>);
-  if (const cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is the kernel's, not the call's: always the same, so that another
+  // thread's call with fewer bins cannot lower it before this launch
+  constexpr int most = (int)stage_bytes(64);
+  if (const cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
       a != cudaSuccess)
     return edm::report_error(EDM_ECUDA, std::string("edm_readout_lifetimes: ") + cudaGetErrorString(a));
   // blocks that fit an SM's 227 KB of shared memory
