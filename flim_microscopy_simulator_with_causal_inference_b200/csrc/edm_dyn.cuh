@@ -1534,9 +1534,11 @@ __device__ __forceinline__ void draw_slot(const EdmDynParams& p, const DevState&
 // gathers its sweepers in shared memory.  One launch and one block's chain:
 // the form for systems that do not fill the chip.  With a draw plan D as many
 // blocks again take the tiles' draws (the draw sweep, k_pass_draws, beside the
-// search without a stream of its own); blocks beyond those, woken_parts per
-// replica, take the woken particles.
-template <bool F64, int BLK, int SPT, int G, int MINB>
+// search without a stream of its own); with WOKEN blocks beyond those, woken_parts
+// per replica, take the woken particles.  A form of its own: with the branch and
+// its call in the only one, 24 replicas without binding took 40.8 us a step, 40.65
+// without.
+template <bool F64, int BLK, int SPT, int G, int MINB, bool WOKEN>
 __global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __restrict__ P,
                                                       const int2* __restrict__ blk, int ntiles,
                                                       const __grid_constant__ DevState st, Match m,
@@ -1546,8 +1548,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_contacts(const EdmDynParams* __re
   __shared__ ContactQueue queue[BLK / 32];
   __shared__ uint32_t rx_of[EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4];
   __shared__ int n_list;
-  const int woken = (int)blockIdx.x - (D ? 2 * ntiles : ntiles);
-  if (woken >= 0) {
+  if (const int woken = (int)blockIdx.x - (D ? 2 * ntiles : ntiles); WOKEN && woken >= 0) {
     if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
     pdl_enter();
     __syncthreads();
@@ -1604,7 +1605,7 @@ __global__ void __launch_bounds__(kBlock) k_sweep_list(const EdmDynParams* __res
 // beyond take the woken particles): no per-tile
 // prologue and every group has a sweeper until the list ends, which pays when
 // the sweepers outnumber the chip's groups several times.
-template <bool F64, int G, int MINB>
+template <bool F64, int G, int MINB, bool WOKEN>
 __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynParams* __restrict__ P,
                                                               const __grid_constant__ DevState st,
                                                               const __grid_constant__ CatLists L, int sweep_blocks,
@@ -1614,7 +1615,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynPara
   if (threadIdx.x < EDM_MAX_SPECIES * EDM_MAX_SPECIES / 4) rx_of[threadIdx.x] = L.rx_of[threadIdx.x];
   pdl_enter();
   __syncthreads();
-  if ((int)blockIdx.x >= sweep_blocks) {
+  if (WOKEN && (int)blockIdx.x >= sweep_blocks) {
     const int woken = (int)blockIdx.x - sweep_blocks;
     woken_contacts<F64, G>(P, st, L, (const uint8_t*)rx_of, woken / woken_parts, woken % woken_parts, woken_parts,
                            queue[threadIdx.x >> 5]);
@@ -2057,16 +2058,17 @@ __device__ __noinline__ void woken_candidates(const EdmDynParams& p, const DevSt
 // tile of BLK * SPT slots per block, G lanes per sweeper, as the contact search;
 // with both species swept slot by slot in a lane each the pass was 36 us for a
 // 13,900-slot sensor membrane.  The tile's complexes draw for their dissociation
-// on the way (st.dis).  Blocks beyond the tiles, woken_parts per replica, take the
-// woken particles.
-template <bool F64, int BLK, int SPT, int G>
+// on the way (st.dis).  With WOKEN blocks beyond the tiles, woken_parts per replica,
+// take the woken particles (a form of its own: the sensor membrane takes 45.7 us a
+// step with it where none can wake, 45.1 without).
+template <bool F64, int BLK, int SPT, int G, bool WOKEN>
 __global__ void __launch_bounds__(BLK) k_bind_candidates(const EdmDynParams* __restrict__ P,
                                                          const int2* __restrict__ blk, int ntiles,
                                                          const __grid_constant__ DevState st,
                                                          const __grid_constant__ Match m, int b, int woken_parts) {
   __shared__ int32_t list[BLK * SPT];
   __shared__ int n_list;
-  if ((int)blockIdx.x >= ntiles) {
+  if (WOKEN && (int)blockIdx.x >= ntiles) {
     const int woken = (int)blockIdx.x - ntiles;
     pdl_enter();
     woken_candidates<F64, G>(P[woken / woken_parts], st, m, woken / woken_parts, b, woken % woken_parts, woken_parts);

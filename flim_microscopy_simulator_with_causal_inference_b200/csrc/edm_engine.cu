@@ -765,23 +765,28 @@ struct EdmEngine {
     }
   }
 
-  template <bool F64, int K>  // row K of kShapes[TK_CONTACTS], kContactSlots, kContactLanes
-  void contacts_shape(const DevState& st, const Match& m, bool with_draws, cudaStream_t s) {
+  template <bool F64, int K, bool WOKEN>  // row K of kShapes[TK_CONTACTS], kContactSlots, kContactLanes
+  void contacts_form(const DevState& st, const Match& m, bool with_draws, cudaStream_t s) {
     constexpr LaunchShape sh = kShapes[TK_CONTACTS][K];
     constexpr int slots = kContactSlots[K], lanes = kContactLanes[K];
     const int t = tile_index(slots > 0 ? sh.block * slots : kBlock * kSweepSlots);
     if (npblk_bs[t] == 0) return;
-    const int woken = cat_lists.woken ? R * dis_parts : 0;
+    const int woken = WOKEN ? R * dis_parts : 0;
     if constexpr (slots > 0) {
       const int nt = npblk_bs[t];
-      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks>, (with_draws ? 2 * nt : nt) + woken, sh.block, s, dp,
+      go(k_contacts<F64, sh.block, slots, lanes, sh.min_blocks, WOKEN>, (with_draws ? 2 * nt : nt) + woken, sh.block, s, dp,
          pblk_bs[t], nt, st, m, cat_lists, with_draws ? d_draw : nullptr, draw.any, dis_parts);
     } else {
       static_assert(sh.block == kBlock, "the list form's blocks");
       go(k_sweep_list, npblk_bs[t], kBlock, s, dp, pblk_bs[t], st, m);
       constexpr int sweep = 148 * sh.min_blocks;
-      go(k_contacts_list<F64, lanes, sh.min_blocks>, sweep + woken, kBlock, s, dp, st, cat_lists, sweep, dis_parts);
+      go(k_contacts_list<F64, lanes, sh.min_blocks, WOKEN>, sweep + woken, kBlock, s, dp, st, cat_lists, sweep, dis_parts);
     }
+  }
+  template <bool F64, int K>
+  void contacts_shape(const DevState& st, const Match& m, bool with_draws, cudaStream_t s) {
+    if (cat_lists.woken) contacts_form<F64, K, true>(st, m, with_draws, s);
+    else contacts_form<F64, K, false>(st, m, with_draws, s);
   }
 
   template <bool F64>
@@ -853,9 +858,12 @@ struct EdmEngine {
       switch (ps.kind) {
         case P_BIND_CAND: {
           const int t = tile_index(kBlock);
-          if (npblk_bs[t] > 0)
-            go(k_bind_candidates<F64, 128, 2, 8>, npblk_bs[t] + (woken_can_bind(ps) ? R * dis_parts : 0), 128, s, dp,
-               pblk_bs[t], npblk_bs[t], st, ps.match, ps.index, dis_parts);
+          const int nt = npblk_bs[t];
+          if (nt > 0 && woken_can_bind(ps))
+            go(k_bind_candidates<F64, 128, 2, 8, true>, nt + R * dis_parts, 128, s, dp, pblk_bs[t], nt, st, ps.match,
+               ps.index, dis_parts);
+          else if (nt > 0)
+            go(k_bind_candidates<F64, 128, 2, 8, false>, nt, 128, s, dp, pblk_bs[t], nt, st, ps.match, ps.index, 0);
           break;
         }
         case P_BIND_APPLY: go(k_bind_apply<F64>, R * (1 + dis_parts), kBindThreads, s, dp, st, ps.index, dis_parts); break;
