@@ -84,8 +84,9 @@ struct DevState {
   int32_t* dis_count;    // [binding reactions][R][2]
   // catalytic contacts of the step: (enzyme slot, substrate-capable slot),
   // contact_cap per reaction.  With rep_contacts each replica has its own part
-  // of the reaction's array and its own counts (k_react takes a replica per
-  // block), without it one list per reaction serves all replicas.
+  // of the reaction's array, rep_contacts per particle and kRepContactsExtra, and
+  // its own counts (k_react takes a replica per block); 0: one list per reaction
+  // serves all replicas.
   int2* contacts;
   int32_t* contact_count;  // [EDM_MAX_CAT], or [R][EDM_MAX_CAT]
   int64_t contact_cap;      // per catalytic reaction
@@ -1292,7 +1293,7 @@ __device__ __forceinline__ void gather_matching(const DevState& st, const Match&
 }
 
 // Where replica r's listed contacts go.
-constexpr int kRepContactsExtra = 4096;  // per replica, beyond 4 per particle
+constexpr int kRepContactsExtra = 4096;
 struct ContactOut {
   int2* list;      // reaction c's part starts at list + c * stride
   int64_t stride;
@@ -1308,9 +1309,9 @@ struct ContactOut {
 __device__ __forceinline__ ContactOut contact_out(const DevState& st, const EdmDynParams& p, int r) {
   ContactOut o{st.contacts, st.contact_cap, st.contact_cap, st.contact_count, st.status};
   if (st.rep_contacts) {
-    const int64_t off = 4 * p.particle_offset + (int64_t)kRepContactsExtra * r;
+    const int64_t off = (int64_t)st.rep_contacts * p.particle_offset + (int64_t)kRepContactsExtra * r;
     o.list += off;
-    o.cap = r + 1 < st.n_rep ? 4 * p.n_particles + kRepContactsExtra : st.contact_cap - off;
+    o.cap = r + 1 < st.n_rep ? (int64_t)st.rep_contacts * p.n_particles + kRepContactsExtra : st.contact_cap - off;
     o.count += (int64_t)r * EDM_MAX_CAT;
   }
   return o;

@@ -115,8 +115,11 @@ constexpr int64_t kStatePack = 16384;
 // 2.1 million (5,000 to 430,000 particles with raised rates).
 constexpr double kReactEntries = 1.0e6;
 // With several replicas each has its own part of a reaction's contact list, so
-// the listed share of the contacts is kept small as well.
+// the listed share of the contacts is kept small as well, and the parts are made
+// for the worst state that one list for all replicas would hold (part_per_particle)
+// unless all of them took more than kReactContacts entries (2 GB).
 constexpr double kReactContactShare = 1.0 / 16.0;
+constexpr double kReactContacts = 268435456.0;
 
 // Choices of earlier tunings in this process, by (kernel, precision,
 // replicas, log2 of the slot count): later engines of the same kind reuse them.
@@ -204,7 +207,8 @@ struct EdmEngine {
   std::vector<uint64_t> pass_thr_host, cat_thr_host;
   ReactPlan react{};  // the passes of P_REACT (k_react)
   int react_threads = 0;
-  bool rep_contacts = false, rep_pl = false;
+  int rep_contacts = 0;
+  bool rep_pl = false;
   unsigned* react_ticket = nullptr;
   int2* contacts = nullptr;
   int32_t* contact_count = nullptr;
@@ -616,6 +620,33 @@ struct EdmEngine {
     return EDM_OK;
   }
 
+  // Contacts per reaction that one list for all replicas holds.
+  int64_t shared_contacts() const { return std::max<int64_t>(4 * N, 1 << 20); }
+
+  // Entries per particle of a replica's part of the contact list, beyond
+  // kRepContactsExtra: at least 4, and as many as a replica can list whose particles
+  // all stand in one place.  Of its n^2 / 4 pairs at most (enzymes times substrates)
+  // those whose draw is below the pass's threshold are listed, once by the search
+  // and once by each earlier reaction that makes the substrate; more than
+  // shared_contacts() pairs of the search, or listed ones of the conversions, one
+  // list for all replicas would not have held either.
+  double part_per_particle() const {
+    const double shared = (double)shared_contacts();
+    double most = 4.0;
+    for (int r = 0; r < R; ++r) {
+      const double n = (double)hdp[r].n_particles, pairs = 0.25 * n * n;
+      for (int c = 0; c < hdp[r].n_cat && n > 0; ++c) {
+        const double thr = std::ldexp((double)cat_thr_host[(size_t)r * EDM_MAX_CAT + c], -53);
+        double listed = thr * std::min(pairs, shared);
+        for (int b = 0; b < c; ++b)
+          if ((cat_late[b] >> c) & 1u) listed += std::min(thr * pairs, shared);
+        listed += 8.0 * std::sqrt(listed);  // the count of independent draws varies
+        most = std::max(most, std::ceil((listed - kRepContactsExtra) / n));
+      }
+    }
+    return most;
+  }
+
   // Hands the passes after the contact search and the draw sweep to k_react,
   // one block per replica, unless a replica's lists are so long that they want
   // the whole chip: the bound on its expected entries is its particles times
@@ -642,6 +673,8 @@ struct EdmEngine {
     if (most > kReactEntries) return EDM_OK;
     for (uint64_t t : cat_thr_host)
       if (R > 1 && std::ldexp((double)t, -53) > kReactContactShare) return EDM_OK;
+    const double part = R > 1 ? part_per_particle() : 4.0;
+    if (part > 4.0 && (part * (double)N + (double)kRepContactsExtra * R) * hdp[0].n_cat > kReactContacts) return EDM_OK;
     bool merges = false, cats = false;
     for (size_t i = start; i < passes.size(); ++i) {
       const Pass& ps = passes[i];
@@ -671,7 +704,7 @@ struct EdmEngine {
       }
     }
     react.n_groups = (int)groups.size();
-    rep_contacts = cats;
+    rep_contacts = cats ? (int)part : 0;
     rep_pl = true;
     react_threads = std::min(kReactThreads, std::max(128, ((int)(2.0 * most) + 31) / 32 * 32));
     passes.resize(start);
@@ -1359,7 +1392,8 @@ int edm_create(const EdmDynParams* dyn, const EdmPhotParams* phot, const EdmScop
     CUDA_TRY(cudaEventCreateWithFlags(&E->ev_fork, cudaEventDisableTiming));
     CUDA_TRY(cudaEventCreateWithFlags(&E->ev_join, cudaEventDisableTiming));
   }
-  E->contact_cap = std::max<int64_t>(4 * np + (int64_t)kRepContactsExtra * n_replicas, 1 << 20);  // per reaction
+  E->contact_cap = std::max<int64_t>(E->shared_contacts(),  // per reaction
+                                     (int64_t)E->rep_contacts * np + (int64_t)kRepContactsExtra * n_replicas);
   ALLOC(E->contacts, (size_t)E->contact_cap * std::max(1, E->hdp[0].n_cat));
   ALLOC(E->contact_count, (size_t)n_replicas * EDM_MAX_CAT);
   ALLOC(E->moved, np);
