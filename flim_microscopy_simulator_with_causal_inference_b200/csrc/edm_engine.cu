@@ -7,6 +7,7 @@
 // replicas; per-step work is enqueued on the caller's stream and can be
 // captured into CUDA graphs (the BD step index lives in device memory, so a
 // captured chunk replays with advancing keys).
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -114,6 +115,16 @@ constexpr int64_t kStatePack = 16384;
 // expected entries, 64 / 422 at 36,000, 253 / 916 at 573,000, 1,059 / 917 at
 // 2.1 million (5,000 to 430,000 particles with raised rates).
 constexpr double kReactEntries = 1.0e6;
+// Expected neighbours that a replica's conversions look at for late contacts in a
+// step, up to which k_react takes its passes: each conversion walks its cells in one
+// lane, and one block walks many at a time less well than the chip.  The bound is
+// per replica and counts all particles as enzymes and substrates alike, some ten
+// times too many.  Per BD step, k_react against the launches: one replica 104 / 110
+// us at 9.7e4 (130 particles per um^2), 202 / 201 at 4.1e4 and 254 / 209 at 1.0e5
+// (1,000), 333 / 337 at 3.3e4, 328 / 317 at 7.3e4 and 1,159 / 848 at 6.6e5 (4,000);
+// eight replicas, whose walks the launches' blocks share as well, 122 / 122 at
+// 1.2e5, 931 / 1,459 at 1.3e5, 512 / 458 at 1.5e5, 487 / 329 at 2.9e5.
+constexpr double kReactWalks = 65536.0;  // times the replicas, up to four
 // With several replicas each has its own part of a reaction's contact list, so
 // the listed share of the contacts is kept small as well, and the parts are made
 // for the worst state that one list for all replicas would hold (part_per_particle)
@@ -651,7 +662,8 @@ struct EdmEngine {
   // one block per replica, unless a replica's lists are so long that they want
   // the whole chip: the bound on its expected entries is its particles times
   // the passes' largest probabilities, plus four contacts per particle times
-  // the catalytic ones.
+  // the catalytic ones; and unless its conversions would look at so many
+  // neighbours (kReactWalks).
   int plan_react() {
     size_t start = passes.size();
     auto fusable = [](PassKind k) {
@@ -671,6 +683,17 @@ struct EdmEngine {
       most = std::max(most, e * (double)hdp[r].n_particles);
     }
     if (most > kReactEntries) return EDM_OK;
+    for (int r = 0; r < R; ++r) {
+      const EdmDynParams& q = hdp[r];
+      const double n = (double)q.n_particles, neighbours = 9.0 * n / ((double)q.nx * q.ny);
+      double walks = 0.0;
+      for (int c = 0; c < q.n_cat; ++c) {
+        const double near = 0.25 * n * n * M_PI * q.cat[c].contact_sq / (q.Lx * q.Ly);
+        if (cat_late[c])
+          walks += neighbours * std::min(n, near * std::ldexp((double)cat_thr_host[(size_t)r * EDM_MAX_CAT + c], -53));
+      }
+      if (walks > kReactWalks * std::min(R, 4)) return EDM_OK;
+    }
     for (uint64_t t : cat_thr_host)
       if (R > 1 && std::ldexp((double)t, -53) > kReactContactShare) return EDM_OK;
     const double part = R > 1 ? part_per_particle() : 4.0;
