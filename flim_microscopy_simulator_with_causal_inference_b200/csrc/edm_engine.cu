@@ -1058,8 +1058,14 @@ struct EdmEngine {
   bool photons_late = false;
   cudaStream_t phot_stream = nullptr, scope_stream = nullptr;
   // the current photon batch may name particles whose slots the sorts do not
-  // track (edm_set_photons, or a state set after the batch was made)
+  // track (edm_set_photons, or a state set after the batch was made).  A call
+  // under the caller's stream capture runs later, on a batch that may be the
+  // host's by then, and makes none now: it maps every slot and clears nothing.
   bool host_batch = false;
+  static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+  }
   bool phot_uses_cells = true;  // some replica's FRET is by proximity (a cell-list search)
   cudaEvent_t ev_phot_fork = nullptr, ev_phot_join = nullptr, ev_scope_join = nullptr;
   bool phot_pending = false, scope_pending = false;
@@ -2010,7 +2016,7 @@ int edm_photon_step(EdmEngine* E, void* stream) {
   if (!E || !E->has_phot) return fail(EDM_EINVAL, "edm_photon_step: engine has no photophysics");
   CUDA_TRY(cudaSetDevice(E->device));
   E->enqueue_photons((cudaStream_t)stream);
-  E->host_batch = false;
+  if (!E->capturing((cudaStream_t)stream)) E->host_batch = false;
   CUDA_TRY(cudaGetLastError());
   return EDM_OK;
 }
@@ -2045,7 +2051,7 @@ int edm_get_photons(EdmEngine* E, int32_t replica, int32_t* particle_idx, double
 int edm_scope_process(EdmEngine* E, void* stream) {
   if (!E || !E->has_scope) return fail(EDM_EINVAL, "edm_scope_process: engine has no microscope");
   CUDA_TRY(cudaSetDevice(E->device));
-  if (E->host_batch && E->N > 0)
+  if (E->N > 0 && (E->host_batch || E->capturing((cudaStream_t)stream)))
     k_slot_map<<<148 * 8, 256, 0, (cudaStream_t)stream>>>(E->ids[E->cur], E->slot_of_id[E->cur], E->N);
   E->enqueue_photon_positions((cudaStream_t)stream);
   E->enqueue_scope((cudaStream_t)stream);
@@ -2080,7 +2086,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
   if (with_photons && !E->has_scope) return fail(EDM_EINVAL, "edm_pipeline_steps: no photophysics/microscope");
   CUDA_TRY(cudaSetDevice(E->device));
   cudaStream_t s = (cudaStream_t)stream;
-  if (with_photons && n_steps > 0) E->host_batch = false;
+  if (with_photons && n_steps > 0 && !E->capturing(s)) E->host_batch = false;
   auto body = [&](cudaStream_t st) {
     E->enqueue_dynamics(st);  // beside the previous step's photon and detection passes
     if (with_photons) {
@@ -2099,9 +2105,7 @@ int edm_pipeline_steps(EdmEngine* E, int32_t n_steps, int32_t with_photons, int3
       const auto key = std::make_tuple(graph_chunk, with_photons ? 1 : 0, E->cur, E->rec_cap > 0 ? 1 : 0);
       auto it = E->graphs.find(key);
       if (it == E->graphs.end()) {
-        cudaStreamCaptureStatus capturing;
-        CUDA_TRY(cudaStreamIsCapturing(s, &capturing));
-        if (capturing == cudaStreamCaptureStatusNone && E->launched_once.insert(key).second) {
+        if (!E->capturing(s) && E->launched_once.insert(key).second) {
           for (int i = 0; i < graph_chunk; ++i) body(s);
           E->join_beside(s);
           CUDA_TRY(cudaGetLastError());
