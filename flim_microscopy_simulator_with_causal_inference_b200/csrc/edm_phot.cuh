@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
                                                        const int2* __restrict__ eblk, DevState st, PhotState ph,
                                                        int64_t* counters) {
   pdl_enter();
-  __shared__ int first[kBlock];  // first photon of each emitter within the tile
+  __shared__ long long first[kBlock];  // first photon of each emitter within the tile
   const Tile t = tile_of(eblk);
   const EdmPhotParams& pp = PP[t.r];
   const EdmDynParams& p = DP[t.r];
@@ -288,14 +288,14 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
   int64_t before = 0;
   for (int k = threadIdx.x; k < ordinal; k += kBlock) before += ph.tile_n[blockIdx.x - ordinal + k];
   const int64_t base = block_sum(before);
-  int total;
-  const int n_mine = t.s < e_end ? ph.emit_n[t.s] : 0;
+  long long total;  // of 256 emitters: 64 bits, as each may have 2^31 and the buffer drops what it cannot hold
+  const long long n_mine = t.s < e_end ? ph.emit_n[t.s] : 0;
   first[threadIdx.x] = block_exclusive_scan(n_mine, total);
   __syncthreads();
   const int64_t key = *ph.d_pstep;
   const Geo g(p);
   int n_donor_ch = 0, n_acc_ch = 0, n_fret = 0;
-  for (int i = threadIdx.x; i < total; i += kBlock) {
+  for (long long i = threadIdx.x; i < total; i += kBlock) {
     const int64_t k = base + i;
     if (k >= pp.max_photons) break;
     int lo = 0, hi = kBlock - 1;  // the last emitter whose first photon is at or before i
