@@ -123,16 +123,6 @@ struct DevState {
 constexpr int32_t kTracked = (int32_t)0x80000000;
 __device__ __forceinline__ int slot_id(const DevState& st, int64_t s) { return st.ids[s] & ~kTracked; }
 
-__device__ __forceinline__ int replica_of(const int64_t* __restrict__ rep_first, int R, int64_t s) {
-  int lo = 0, hi = R - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (rep_first[mid] <= s) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 // Particles a per-particle pass visits: the species set mask[1] of alive
 // particles and mask[0] of particles that are not alive.
 struct Match {

@@ -377,14 +377,9 @@ struct EdmEngine {
       passes.push_back({P_BIND_CAND, b, match({B.ra}, 1)});
       passes.push_back({P_BIND_APPLY, b, none});
     }
-    // adaptation field, after binding and before catalysis (dynamics.py:2227-2242)
-    if (p.adapt_grid >= 0) {
-      if (dirty[p.adapt_grid]) {
-        passes.push_back({P_MERGE, 0, none});
-        std::fill(dirty.begin(), dirty.end(), false);
-      }
-      passes.push_back({P_ADAPT, 0, none});
-    }
+    // adaptation field, after binding and before catalysis (dynamics.py:2227-2242);
+    // the binding passes leave no grid change pending
+    if (p.adapt_grid >= 0) passes.push_back({P_ADAPT, 0, none});
     if (p.n_cat > 0) {
       enzyme_mask = 0;
       uint32_t touched = 0;
