@@ -1634,9 +1634,9 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynPara
 // substrate of the later reactions `late`: its alive neighbours of those
 // reactions' enzyme species passing the tests an enzyme-side sweep makes
 // (j seen from enzyme e at the opposite cell offset, the same float32
-// expressions), and its neighbours among the particles woken in the step, which
-// the cells do not hold; appended to the reactions' lists.
-template <bool F64>
+// expressions), and with WOKEN its neighbours among the particles woken in the
+// step, which the cells do not hold; appended to the reactions' lists.
+template <bool F64, bool WOKEN>
 __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
                                            int64_t j, int id_j, int64_t step, uint32_t late,
                                            const ContactOut& out) {
@@ -1666,6 +1666,7 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
     }
     file(e, spe);
   });
+  if constexpr (!WOKEN) return;
   uint32_t woken = 0;  // enzyme species that a dissociation can wake
   for (int b = 0; b < p.n_bind; ++b) woken |= emask & (1u << p.bind[b].rb);
   if (!woken) return;
@@ -1685,7 +1686,7 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
 // radius and has its draw below the pass's threshold; the partner's current
 // species and the exact probability are left to test.
 // `late`: the later reactions whose substrate is this pass's product.
-template <bool F64, typename Sink>
+template <bool F64, bool WOKEN, typename Sink>
 __device__ __forceinline__ void catalytic_pair(const EdmDynParams& p, const DevState& st, int r, int cidx,
                                                uint32_t late, int2 es, const Sink& sink, const ContactOut& out) {
   const uint8_t fs = st.flags[es.y];
@@ -1705,12 +1706,12 @@ __device__ __forceinline__ void catalytic_pair(const EdmDynParams& p, const DevS
   if (u < peff && cas_u8(&st.flags[es.y], fs, fl_make(C.product, true))) {
     atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_CATALYTIC], 1);
     grid_change(p, sink, C.substrate, true, C.product, true, xs, ys);
-    if (late) late_contacts<F64>(p, g, st, r, es.y, ids, *st.d_step, late, out);
+    if (late) late_contacts<F64, WOKEN>(p, g, st, r, es.y, ids, *st.d_step, late, out);
   }
 }
 
 // One pass over one list for all replicas, for systems whose lists are long.
-template <bool F64>
+template <bool F64, bool WOKEN>
 __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __restrict__ P, DevState st, int cidx,
                                                        uint32_t late) {
   pdl_enter();
@@ -1721,7 +1722,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_catalytic(const EdmDynParams* __r
     const int2 es = list[q];
     int r = st.chunk_rep[es.x / kSweepChunk];
     while (r + 1 < st.n_rep && st.rep_first[r + 1] <= es.x) ++r;
-    catalytic_pair<F64>(P[r], st, r, cidx, late, es, DeltaArray{st.grid_delta}, contact_out(st, P[r], r));
+    catalytic_pair<F64, WOKEN>(P[r], st, r, cidx, late, es, DeltaArray{st.grid_delta}, contact_out(st, P[r], r));
   }
 }
 
@@ -2403,7 +2404,7 @@ struct ReactPlan {
   int n, n_groups;
 };
 
-template <bool F64>
+template <bool F64, bool WOKEN>
 __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __restrict__ P, DevState st,
                                                        const __grid_constant__ ReactPlan plan,
                                                        const PassGroup* __restrict__ groups,
@@ -2445,7 +2446,7 @@ __global__ void __launch_bounds__(kReactThreads) k_react(const EdmDynParams* __r
       case kReactCatalytic: {
         const int n = n_contact[idx] < out.cap ? n_contact[idx] : (int)out.cap;
         for (int q = tid; q < n; q += blockDim.x)
-          catalytic_pair<F64>(p, st, r, idx, plan.more[i], out.list[(int64_t)idx * out.stride + q], sink, out);
+          catalytic_pair<F64, WOKEN>(p, st, r, idx, plan.more[i], out.list[(int64_t)idx * out.stride + q], sink, out);
         break;
       }
       case kReactGroup: {

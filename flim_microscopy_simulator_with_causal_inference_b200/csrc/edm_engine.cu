@@ -227,6 +227,7 @@ struct EdmEngine {
   uint32_t enzyme_mask = 0;
   CatLists cat_lists{};
   uint32_t cat_late[EDM_MAX_CAT] = {};
+  bool late_woken = false;  // a dissociation can wake an enzyme of a late pair
   bool contact_sides_counted = false;  // sides chosen from a state's species counts
   int64_t* rep_first = nullptr;
   int32_t* chunk_rep = nullptr;  // replica of the first slot of each 128-slot chunk
@@ -390,7 +391,10 @@ struct EdmEngine {
         // particle it converts gets its late pairs for them at once
         cat_late[c] = 0;
         for (int c2 = c + 1; c2 < p.n_cat; ++c2)
-          if (p.cat[c2].substrate == p.cat[c].product) cat_late[c] |= 1u << c2;
+          if (p.cat[c2].substrate == p.cat[c].product) {
+            cat_late[c] |= 1u << c2;
+            late_woken |= (woken_species(p.n_bind) >> p.cat[c2].enzyme) & 1u;
+          }
       }
       if (enzyme_mask & touched) return fail(EDM_EUNSUP, "an enzyme species is also a catalytic substrate/product");
       passes.push_back({P_CONTACTS, 0, Match{{0u, 0u}}});
@@ -923,7 +927,7 @@ struct EdmEngine {
           launch_contacts<F64>(st, ps.match, draws_beside, s);
           tune_mark(TK_CONTACTS, 1, s);
           break;
-        case P_CAT: go(k_catalytic<F64>, cgrid, kBlock, s, dp, st, ps.index, cat_late[ps.index]); break;
+        case P_CAT: go(late_woken ? k_catalytic<F64, true> : k_catalytic<F64, false>, cgrid, kBlock, s, dp, st, ps.index, cat_late[ps.index]); break;
         case P_REC_APPLY: go(k_recruit_apply<F64>, rb, 128, s, dp, R, st, ps.index, d_draw, rec_after[ps.index]); break;
         case P_DRAWS: {
           // beside the following passes on the side stream (not while timing passes one by one)
@@ -963,7 +967,7 @@ struct EdmEngine {
             joined = true;
             pdl_chain = false;
           }
-          go(k_react<F64>, R, react_threads, s, dp, st, react, d_groups, d_draw, d_step, react_ticket);
+          go(late_woken ? k_react<F64, true> : k_react<F64, false>, R, react_threads, s, dp, st, react, d_groups, d_draw, d_step, react_ticket);
           break;
         case P_MERGE: go(k_grid_merge, gm > 0 ? gm : 1, 256, s, grid_cnt, grid_delta, n_grid); break;
       }
