@@ -542,30 +542,29 @@ __device__ __forceinline__ void store4_in(int32_t* a, int64_t i, int64_t lo, int
   if (i + 3 >= lo && i + 3 < hi) a[i + 3] = v.w;
 }
 
-template <typename T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T& total) {
-  __shared__ T warp_sums[32];
+__device__ __forceinline__ int block_exclusive_scan(int v, int& total) {
+  __shared__ int warp_sums[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  T x = v;
+  int x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const T y = __shfl_up_sync(0xffffffffu, x, o);
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   if (lane == 31) warp_sums[wid] = x;
   __syncthreads();
   if (wid == 0) {
     const int nw = blockDim.x >> 5;
-    T w = lane < nw ? warp_sums[lane] : T(0);
+    int w = lane < nw ? warp_sums[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const T y = __shfl_up_sync(0xffffffffu, w, o);
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += y;
     }
     if (lane < nw) warp_sums[lane] = w;
   }
   __syncthreads();
-  const T base = wid > 0 ? warp_sums[wid - 1] : T(0);
+  const int base = wid > 0 ? warp_sums[wid - 1] : 0;
   total = warp_sums[(blockDim.x >> 5) - 1];
   __syncthreads();
   return base + x - v;

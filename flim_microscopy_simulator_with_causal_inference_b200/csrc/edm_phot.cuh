@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
                                                        const int2* __restrict__ eblk, DevState st, PhotState ph,
                                                        int64_t* counters) {
   pdl_enter();
-  __shared__ long long first[kBlock];  // first photon of each emitter within the tile
+  __shared__ int first[kBlock];  // first photon of each emitter within the tile
   const Tile t = tile_of(eblk);
   const EdmPhotParams& pp = PP[t.r];
   const EdmDynParams& p = DP[t.r];
@@ -288,14 +288,24 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
   int64_t before = 0;
   for (int k = threadIdx.x; k < ordinal; k += kBlock) before += ph.tile_n[blockIdx.x - ordinal + k];
   const int64_t base = block_sum(before);
-  long long total;  // of 256 emitters: 64 bits, as each may have 2^31 and the buffer drops what it cannot hold
-  const long long n_mine = t.s < e_end ? ph.emit_n[t.s] : 0;
-  first[threadIdx.x] = block_exclusive_scan(n_mine, total);
+  const int64_t tile_total = ph.tile_n[blockIdx.x];
+  constexpr int kMost = INT32_MAX - kBlock;
+  int total;
+  if (tile_total <= kMost) {
+    first[threadIdx.x] = block_exclusive_scan(t.s < e_end ? ph.emit_n[t.s] : 0, total);
+  } else {
+    // more than any buffer below 64 GB holds: the indices past kMost are all
+    // dropped, and each thread adds up its emitter's first one in 64 bits
+    int64_t sum = 0;
+    for (int64_t e = e0; e < t.s && e < e_end; ++e) sum += ph.emit_n[e];
+    first[threadIdx.x] = (int)(sum < kMost ? sum : kMost);
+    total = kMost;
+  }
   __syncthreads();
   const int64_t key = *ph.d_pstep;
   const Geo g(p);
   int n_donor_ch = 0, n_acc_ch = 0, n_fret = 0;
-  for (long long i = threadIdx.x; i < total; i += kBlock) {
+  for (int i = threadIdx.x; i < total; i += kBlock) {
     const int64_t k = base + i;
     if (k >= pp.max_photons) break;
     int lo = 0, hi = kBlock - 1;  // the last emitter whose first photon is at or before i
@@ -347,7 +357,7 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
   __syncthreads();
   if (threadIdx.x != 0) return;
   if (e0 + kBlock >= e_end) {  // the replica's last tile
-    int64_t n = base + total;
+    int64_t n = base + tile_total;
     if (n > pp.max_photons) {
       n = pp.max_photons;
       set_status(st.status, EDM_STATUS_PHOTON_CAP);
