@@ -44,6 +44,80 @@ __device__ __forceinline__ void readout_pair(uint32_t na, uint32_t nb, double c,
   t.S = fma(dif, s, t.S);
 }
 
+// The six readouts of pixel px from its intensity, sum of n_k k and phasor sums.
+struct Readout {
+  double width, omega, nan;
+  int min_mean, min_phasor;
+  int64_t n_px;
+  double* out;
+  __device__ __forceinline__ void write(int64_t px, double In, double KW, double G, double S) const {
+    const double tau = In >= min_mean ? width * (KW + 0.5 * In) / In : nan;
+    const bool mask = In >= min_phasor;
+    const double g = mask ? G / In : 0.0, s = mask ? S / In : 0.0;
+    const bool valid = mask && g > 1e-10;
+    const double m2 = g * g + s * s;
+    out[0 * n_px + px] = In;
+    out[1 * n_px + px] = tau;
+    out[2 * n_px + px] = g;
+    out[3 * n_px + px] = s;
+    out[4 * n_px + px] = valid ? (s / g) / omega : nan;
+    out[5 * n_px + px] = (valid && m2 > 1e-10 && m2 < 1.0 - 1e-10) ? sqrt(1.0 / m2 - 1.0) / omega : nan;
+  }
+};
+
+// Exact float64 value of an integer v < 2^52: the double whose bits are
+// 2^52 + v, minus 2^52 (one add instead of an integer-to-double conversion).
+__device__ __forceinline__ double u52_to_f64(uint64_t v) {
+  const double d = __hiloint2double(0x43300000 | (int)(uint32_t)(v >> 32), (int)(uint32_t)v);
+  return __dsub_rn(d, 4503599627370496.0);
+}
+__device__ __forceinline__ void readout_pair(uint32_t na, uint32_t nb, int k, int kb, const double* c_k,
+                                             const double* s_k, uint64_t& I, uint64_t& KW, double& G, double& S) {
+  I += (uint64_t)na + nb;
+  KW += (uint64_t)na * (uint32_t)k + (uint64_t)nb * (uint32_t)kb;
+  G = fma(u52_to_f64((uint64_t)na + nb), c_k[k], G);
+  S = fma(__dsub_rn(u52_to_f64((uint64_t)na + 4294967296ull - nb), 4294967296.0), s_k[k], S);
+}
+
+// Short rows: a thread per pixel reads its row from both ends in 16-byte words, the
+// lanes of a warp 32 rows side by side.  Intensity and sum n_k k are integer sums.
+__global__ void __launch_bounds__(256) k_readout_rows(const uint32_t* __restrict__ stack, int64_t n_px, int n_bins,
+                                                      double T_ns, int harmonic, int min_mean, int min_phasor,
+                                                      double* __restrict__ out) {
+  __shared__ double c_k[256], s_k[256];
+  for (int k = threadIdx.x; k < n_bins; k += blockDim.x) {
+    const double phi = 2.0 * M_PI * harmonic * (k + 0.5) / n_bins;
+    c_k[k] = cos(phi);
+    s_k[k] = sin(phi);
+  }
+  __syncthreads();
+  const int nq = n_bins / 4;  // uint4 per pixel
+  const Readout R{T_ns / n_bins, 2.0 * M_PI * harmonic / T_ns, __longlong_as_double(0x7FF8000000000000ll),
+                  min_mean,      min_phasor,                   n_px,
+                  out};
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t px = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; px < n_px; px += step) {
+    const uint4* row = reinterpret_cast<const uint4*>(stack + px * (int64_t)n_bins);
+    uint64_t I = 0, KW = 0;
+    double G = 0.0, S = 0.0;
+    int q = 0;
+    for (; q < nq - 1 - q; ++q) {  // word q (bins 4q..4q+3) against word nq-1-q, reversed
+      const int qb = nq - 1 - q;
+      const uint4 a = __ldg(row + q), b = __ldg(row + qb);
+      readout_pair(a.x, b.w, 4 * q, 4 * qb + 3, c_k, s_k, I, KW, G, S);
+      readout_pair(a.y, b.z, 4 * q + 1, 4 * qb + 2, c_k, s_k, I, KW, G, S);
+      readout_pair(a.z, b.y, 4 * q + 2, 4 * qb + 1, c_k, s_k, I, KW, G, S);
+      readout_pair(a.w, b.x, 4 * q + 3, 4 * qb, c_k, s_k, I, KW, G, S);
+    }
+    if (q == nq - 1 - q) {  // odd word count: the middle word pairs within itself
+      const uint4 a = __ldg(row + q);
+      readout_pair(a.x, a.w, 4 * q, 4 * q + 3, c_k, s_k, I, KW, G, S);
+      readout_pair(a.y, a.z, 4 * q + 1, 4 * q + 2, c_k, s_k, I, KW, G, S);
+    }
+    R.write(px, (double)I, (double)KW, G, S);
+  }
+}
+
 __device__ __forceinline__ void copy16_async(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
                : "memory");
@@ -54,9 +128,9 @@ __device__ __forceinline__ void copies_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Bound: the stack's bytes from DRAM (4.19M pixels of 256 bins in 663 us, 6.8
-// TB/s; 1,087 us before).  A warp takes groups of kGroup pixels,
-// four lanes per pixel, and keeps kStages groups' rows on the way into its own
+// Long rows.  Bound: the stack's bytes from DRAM (4.19M pixels of 256 bins in 703 us,
+// 687 at the copy's rate; 1,090 by k_readout_rows).  A warp takes groups of kGroup
+// pixels, four lanes per pixel, and keeps kStages groups' rows on the way into its own
 // part of shared memory by 16-byte asynchronous copies: consecutive lanes copy
 // consecutive words of the rows, four 128-byte lines per instruction.  (A
 // thread per pixel reading its row from both ends touched 32 lines per
@@ -90,9 +164,9 @@ __global__ void __launch_bounds__(32 * kReadoutWarps) k_readout(const uint32_t* 
   const int nq = n_bins / 4, ld = row_words(nq);  // uint4 per pixel, and per row in shared memory
   const int lane = threadIdx.x & 31, sub = lane & 3, warp = threadIdx.x >> 5;
   uint4* mine = stage_mem + (size_t)warp * kStages * kGroup * ld;
-  const double width = T_ns / n_bins;
-  const double omega = 2.0 * M_PI * harmonic / T_ns;
-  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  const Readout R{T_ns / n_bins, 2.0 * M_PI * harmonic / T_ns, __longlong_as_double(0x7FF8000000000000ll),
+                  min_mean,      min_phasor,                   n_px,
+                  out};
   const int64_t groups = (n_px + kGroup - 1) / kGroup;
   const int64_t step = (int64_t)gridDim.x * kReadoutWarps;
   const uint4* words = reinterpret_cast<const uint4*>(stack);
@@ -156,19 +230,21 @@ __global__ void __launch_bounds__(32 * kReadoutWarps) k_readout(const uint32_t* 
     }
     const int64_t px = g * kGroup + (lane >> 2);
     if (sub != 0 || px >= n_px) continue;
-    const double In = t.I, KW = 0.5 * (n_bins - 1) * t.I - t.M;
-    const double tau = In >= min_mean ? width * (KW + 0.5 * In) / In : nan;
-    const bool mask = In >= min_phasor;
-    const double gg = mask ? t.G / In : 0.0, ss = mask ? t.S / In : 0.0;
-    const bool valid = mask && gg > 1e-10;
-    const double m2 = gg * gg + ss * ss;
-    out[0 * n_px + px] = In;
-    out[1 * n_px + px] = tau;
-    out[2 * n_px + px] = gg;
-    out[3 * n_px + px] = ss;
-    out[4 * n_px + px] = valid ? (ss / gg) / omega : nan;
-    out[5 * n_px + px] = (valid && m2 > 1e-10 && m2 < 1.0 - 1e-10) ? sqrt(1.0 / m2 - 1.0) / omega : nan;
+    R.write(px, t.I, 0.5 * (n_bins - 1) * t.I - t.M, t.G, t.S);
   }
+}
+
+// Pixels from which k_readout_rows is the faster.  k_readout spends a latency on
+// every eight pixels however short their rows, and unless it knows the row's length
+// (128 and 256 bins) the copies' index arithmetic is not hidden; k_readout_rows needs
+// many threads.  Rows / staged, us: 16 bins 7.4 / 7.4 at 10,000 pixels, 7.3 / 8.3 at
+// 30,000, 91 / 303 at 4.2M; 64 bins 7.6 / 7.3, 8.4 / 9.3, 303 / 389; 100 bins 39.9 /
+// 36.6 at 262,144, 68.6 / 68.6 at 524,288, 124.7 / 127.4 at 1.05M; 160 bins 111 / 109
+// at 524,288, 195 / 208 at 1.05M; 252 bins 29.8 / 27.7 at 65,536, 45.8 / 49.3 at
+// 131,072, 272 / 321 at 1.05M; 256 bins 290 / 221 there.
+int64_t rows_from(int n_bins) {
+  if (n_bins == 128 || n_bins == 256) return INT64_MAX;
+  return n_bins <= 96 ? 1 << 14 : (n_bins <= 176 ? 1 << 20 : 1 << 17);
 }
 
 }  // namespace
@@ -186,6 +262,17 @@ extern "C" int edm_readout_lifetimes(const uint32_t* stack_dev, int64_t n_px, in
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (n_px >= rows_from(n_bins)) {
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_readout_rows, 256, 0);
+    const int64_t want = (n_px + 255) / 256, cap = (int64_t)sms * std::max(1, per_sm);
+    k_readout_rows<<<(unsigned)std::min(want, cap), 256, 0, s>>>(stack_dev, n_px, n_bins, time_range_s * 1e9, harmonic,
+                                                                   min_counts_mean, min_counts_phasor, out_dev);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return edm::report_error(EDM_ECUDA, std::string("edm_readout_lifetimes: ") + cudaGetErrorString(e));
+    return EDM_OK;
+  }
   const size_t smem = stage_bytes(n_bins / 4);
   const auto kernel = n_bins == 256 ? k_readout<64> : (n_bins == 128 ? k_readout<32> : k_readout<0>);
   // the limit is the kernel's, not the call's: always the same, so that another
@@ -198,8 +285,8 @@ extern "C" int edm_readout_lifetimes(const uint32_t* stack_dev, int64_t n_px, in
   const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(5, (227 * 1024) / (smem + 4096)));
   const int64_t want = (n_px + kGroup * kReadoutWarps - 1) / (kGroup * kReadoutWarps), cap = (int64_t)sms * per_sm;
   const unsigned blocks = (unsigned)(want < cap ? want : cap);
-  kernel<<<blocks, 32 * kReadoutWarps, smem, (cudaStream_t)stream>>>(
-      stack_dev, n_px, n_bins, time_range_s * 1e9, harmonic, min_counts_mean, min_counts_phasor, out_dev);
+  kernel<<<blocks, 32 * kReadoutWarps, smem, s>>>(stack_dev, n_px, n_bins, time_range_s * 1e9, harmonic, min_counts_mean,
+                                                  min_counts_phasor, out_dev);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return edm::report_error(EDM_ECUDA, std::string("edm_readout_lifetimes: ") + cudaGetErrorString(e));
   return EDM_OK;
