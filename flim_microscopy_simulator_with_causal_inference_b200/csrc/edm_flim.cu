@@ -51,11 +51,16 @@ constexpr int kDim = 256;                  // pixels per side; the GEMM tiles as
 constexpr int kBM = 128;                   // UMMA M per CTA
 constexpr int kBK = 64;                    // K per stage: one 128-byte swizzle atom of bf16
 constexpr int kStageA = kBM * kBK * 2;     // 16 KB
-constexpr int kBN = 64;                    // UMMA N per CTA
-constexpr int kStageB = kBN * kBK * 2;     // 8 KB
-constexpr int kStage = kStageA + kStageB;  // multiple of 1024: every tile stays swizzle-aligned
-constexpr int kGemmStages = 4;
-constexpr int kGemmSmem = kGemmStages * kStage + 1024 + 256;
+// A CTA's N and the stages of its ring (see k_umma_gemm)
+template <int BN, int STAGES>
+struct GemmTile {
+  static constexpr int kStage = kStageA + BN * kBK * 2;  // multiple of 1024: every tile stays swizzle-aligned
+  static constexpr int kSmem = STAGES * kStage + 1024 + 256;
+  // kind::f16 instruction descriptor: FP32 D (bits 4-5 = 1), BF16 A (7-9 = 1)
+  // and B (10-12 = 1), both K-major, N/8 in bits 17-22, M/16 in bits 24-28.
+  static constexpr uint32_t kIdesc =
+      (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+};
 constexpr uint32_t kWaitLimit = 1u << 22;  // bounded mbarrier polls before reporting an error
 constexpr int kK1 = 512, kK2 = 768;        // K of the two GEMMs (hi/lo concatenations)
 
@@ -103,16 +108,11 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
   d |= (uint64_t)2 << 61;            // 128-byte swizzle
   return d;
 }
-// kind::f16 instruction descriptor: FP32 D (bits 4-5 = 1), BF16 A (7-9 = 1)
-// and B (10-12 = 1), both K-major, N/8 in bits 17-22, M/16 in bits 24-28.
-constexpr uint32_t kIdesc =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
           tmem_d),
-      "l"(a), "l"(b), "r"(kIdesc), "r"(acc)
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -143,7 +143,7 @@ struct GemmArgs {
 };
 
 // D[batch] = A[batch] (256 x K) . B[batch]^T (256 x K), both operands
-// K-major bf16.  One CTA per 128 x 64 tile and batch, 128 threads: thread 0
+// K-major bf16.  One CTA per 128 x kBN tile and batch, 128 threads: thread 0
 // streams K in 64-wide stages by TMA (a ring of kGemmStages, mbarrier-tracked)
 // and issues the MMAs; then each warp reads its 32 accumulator lanes (rows)
 // from tensor memory and writes them out.
@@ -152,10 +152,14 @@ struct GemmArgs {
 // of its loads.  One operand is the PSF band, zero farther than `taps` from the
 // diagonal: the 64-wide chunks of each section that hold no nonzero of this
 // tile's band rows are left out (a sum of exact zeros), and the stages in
-// flight cover the rest.  Eight CTAs per map instead of two with 256 columns
-// each and two stages: 15.8 to 7 and 8 us for the two products of one field of view.
+// flight cover the rest.  Few maps want many CTAs: eight per map with 64 columns
+// and four stages instead of two with 256 and two take the two products of one field
+// of view from 15.8 to 7 and 8 us.  Many maps fill the chip anyway, and there a map's
+// rows are read by two CTAs instead of eight (kManyMaps).
+template <int kBN, int kGemmStages>
 __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUtensorMap tmA,
                                                    const __grid_constant__ CUtensorMap tmB, GemmArgs args) {
+  constexpr int kStage = GemmTile<kBN, kGemmStages>::kStage;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + kGemmStages * kStage);  // full[stages], empty[stages], done
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __grid_constant__ CUten
       const uint64_t db = sw128_desc(smem_u32(smem + s * kStage + kStageA));
 #pragma unroll
       for (int j = 0; j < kBK / 16; ++j)  // K = 16 per MMA: +32 bytes = +2 in the start-address field
-        umma_bf16(tmem, da + 2 * j, db + 2 * j, (t > 0 || j > 0) ? 1u : 0u);
+        umma_bf16(tmem, da + 2 * j, db + 2 * j, GemmTile<kBN, kGemmStages>::kIdesc, (t > 0 || j > 0) ? 1u : 0u);
       umma_commit(empty0 + 8 * s);  // stage s is free once these MMAs have read it
       if (t + kGemmStages < n) {
         if (!mbar_wait(empty0 + 8 * s, (t / kGemmStages) & 1)) {
@@ -731,6 +735,19 @@ void launch_after(void (*kernel)(K...), dim3 grid, int block, size_t smem, cudaS
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// The projection's tile.  Whole projection, 128 x 64 x 4 stages / 128 x 256 x 2, us: 1
+// field of view 31 / 42, 16 38 / 45, 32 57.7 / 56.9, 64 99 / 85, 256 376 / 327 with 15
+// taps; 32 61 / 58, 256 408 / 334 with 127.  128 x 128 lies between or within 2 %.
+constexpr int kManyMaps = 32;  // replicas
+struct GemmForm {
+  void (*kernel)(const CUtensorMap, const CUtensorMap, GemmArgs);
+  int bn, smem;
+};
+GemmForm gemm_form(int n_replicas) {
+  if (n_replicas >= kManyMaps) return {k_umma_gemm<256, 2>, 256, GemmTile<256, 2>::kSmem};
+  return {k_umma_gemm<64, 4>, 64, GemmTile<64, 4>::kSmem};
+}
+
 int check_params(const EdmFlimParams& p) {
   if (p.nx != kDim || p.ny != kDim) return fail(EDM_EUNSUP, "FLIM acquisition: the GEMM path needs 256 x 256 pixels");
   if (p.n_replicas <= 0 || p.n_replicas > 4096) return fail(EDM_EINVAL, "FLIM acquisition: n_replicas out of 1..4096");
@@ -775,14 +792,15 @@ int edm_flim_create(const EdmFlimParams* params, int32_t device, EdmFlim** out) 
   FA(F->hist, R * npx * params->n_bins);
   FA(F->err, 1);
 #undef FA
+  const GemmForm gemm = gemm_form(params->n_replicas);
   if ((rc = make_map(&F->mA1, F->maps, kDim, kDim, 2 * R, kBM)) != EDM_OK ||
-      (rc = make_map(&F->mB1, F->g1, kK1, kDim, 1, kBN)) != EDM_OK ||
+      (rc = make_map(&F->mB1, F->g1, kK1, kDim, 1, gemm.bn)) != EDM_OK ||
       (rc = make_map(&F->mA2, F->a2, kK2, kDim, 1, kBM)) != EDM_OK ||
-      (rc = make_map(&F->mB2, F->b2, kK2, kDim, 2 * R, kBN)) != EDM_OK) {
+      (rc = make_map(&F->mB2, F->b2, kK2, kDim, 2 * R, gemm.bn)) != EDM_OK) {
     delete F;
     return rc;
   }
-  cudaError_t e = cudaFuncSetAttribute(k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+  cudaError_t e = cudaFuncSetAttribute(gemm.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm.smem);
   if (e == cudaSuccess) {
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -831,7 +849,8 @@ int edm_flim_project(EdmFlim* F, void* stream) {
   FL_TRY(cudaMemsetAsync(F->counts, 0, sizeof(int32_t) * R * 2 * npx, s));
   k_emitters<<<dim3(64, (unsigned)R), 256, 0, s>>>(p, F->bound_fraction, F->counts);
   launch_after(k_counts_to_bf16, dim3(148 * 8), 256, 0, s, (const int32_t*)F->counts, F->maps, R * 2 * npx, F->err);
-  const dim3 tiles((kDim / kBM) * (kDim / kBN), (unsigned)(2 * R));
+  const GemmForm gemm = gemm_form(p.n_replicas);
+  const dim3 tiles((kDim / kBM) * (kDim / gemm.bn), (unsigned)(2 * R));
   GemmArgs a1{};
   a1.sections = kK1 / kDim;
   a1.a_kwrap = kDim;  // A = [M | M]: the count map twice along K
@@ -840,7 +859,7 @@ int edm_flim_project(EdmFlim* F, void* stream) {
   a1.split_transpose = 1;
   a1.b2 = F->b2;
   a1.err = F->err;
-  launch_after(k_umma_gemm, tiles, 128, kGemmSmem, s, F->mA1, F->mB1, a1);
+  launch_after(gemm.kernel, tiles, 128, gemm.smem, s, F->mA1, F->mB1, a1);
   GemmArgs a2{};
   a2.sections = kK2 / kDim;
   a2.b_batched = 1;
@@ -848,7 +867,7 @@ int edm_flim_project(EdmFlim* F, void* stream) {
   a2.taps = p.half_taps;
   a2.out = F->I;
   a2.err = F->err;
-  launch_after(k_umma_gemm, tiles, 128, kGemmSmem, s, F->mA2, F->mB2, a2);
+  launch_after(gemm.kernel, tiles, 128, gemm.smem, s, F->mA2, F->mB2, a2);
   FL_TRY(cudaGetLastError());
   return EDM_OK;
 }
