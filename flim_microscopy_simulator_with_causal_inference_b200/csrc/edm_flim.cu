@@ -877,7 +877,13 @@ int edm_flim_histograms(EdmFlim* F, int32_t with_tau, void* stream) {
   FL_TRY(cudaSetDevice(F->device));
   const EdmFlimParams& p = F->p;
   const size_t total_px = (size_t)p.n_replicas * kDim * kDim;
-  const unsigned blocks = (unsigned)std::min<size_t>((total_px / 32 + kHistWarps - 1) / kHistWarps, (size_t)F->hist_blocks);
+  // Faint fields of 256 bins are bound by the histograms' writes, which many warps in
+  // flight spread over too many rows of memory: half as many blocks.  32 fields of 2
+  // photons a pixel 357 us with 10 blocks an SM, 399 with 20 (5 photons 386 / 402, 10
+  // photons 410 / 409, 20 photons 437 / 411).
+  const double photons = std::max(p.yield_free, p.yield_bound) * p.n_emitters / (double)(kDim * kDim);
+  const int resident = p.n_bins == 256 && photons < 8.0 ? std::max(1, F->hist_blocks / 2) : F->hist_blocks;
+  const unsigned blocks = (unsigned)std::min<size_t>((total_px / 32 + kHistWarps - 1) / kHistWarps, (size_t)resident);
   const auto kernel = p.n_bins == 256 ? k_hist<256> : k_hist<128>;
   launch_after(kernel, dim3(blocks), 32 * kHistWarps, 0, (cudaStream_t)stream, p, (const float*)F->I,
                (const int2*)F->alias, (const double*)F->sums, F->hist, with_tau ? F->tau : (double*)nullptr, 1u, 4u);
