@@ -104,9 +104,10 @@ int tile_index(int bs) {
 // state, bleached and dye flags.  Up to kStatePack particles bound for pageable
 // memory come down in one copy and are handed out by the host; a larger state's
 // fields, and any bound for pinned arrays, are copied straight to them.  Seven
-// copies to pageable memory cost some 14 us each however small: 5,000 particles
-// 115 us, in one copy 59; to pinned memory seven are faster (13,900 particles 77
-// against 117 us).
+// copies to pageable memory cost some 14 us each however small, the host's handing
+// out grows with the state: in one copy / in seven 57 / 106 us for 5,000 particles,
+// 107 / 129 for 16,384, 122 / 140 for 20,000, 154 / 148 for 24,000, 184 / 168 for
+// 32,000; to pinned memory seven are faster (13,900 particles 77 against 117 us).
 constexpr size_t kStateBytes = 28;
 constexpr int64_t kStatePack = 16384;
 
@@ -125,10 +126,13 @@ constexpr double kReactEntries = 1.0e6;
 // eight replicas, whose walks the launches' blocks share as well, 122 / 122 at
 // 1.2e5, 931 / 1,459 at 1.3e5, 512 / 458 at 1.5e5, 487 / 329 at 2.9e5.
 constexpr double kReactWalks = 65536.0;  // times the replicas, up to four
-// With several replicas each has its own part of a reaction's contact list, so
-// the listed share of the contacts is kept small as well, and the parts are made
+// With several replicas each has its own part of a reaction's contact list, made
 // for the worst state that one list for all replicas would hold (part_per_particle)
-// unless all of them took more than kReactContacts entries (2 GB).
+// unless all of them took more than kReactContacts entries (2 GB).  The parts grow
+// with the listed share of the contacts, so that is kept small as well.  This line is
+// the list's, not the clock's: eight replicas of 500 to 8,000 particles (130 per
+// um^2), k_react against the launches, 47 / 68, 61 / 99 and 89 / 114 us a step at a
+// share of 0.014, 58 / 96, 85 / 107 and 122 / 122 at 0.071.
 constexpr double kReactContactShare = 1.0 / 16.0;
 constexpr double kReactContacts = 268435456.0;
 
@@ -1046,8 +1050,10 @@ struct EdmEngine {
   // the first pass that changes flags or bonds.  Two launches of latency, it
   // takes 12 us: the first window is 5 us in a small system, the second 14, and
   // a step of 5,000 slots falls from 31.3 to 28.5 us, of 207,000 from 46.4 to
-  // 42.6; in a large system it competes with the move instead (1.9M slots 202
-  // against 206 us, 4.7M slots 324 against 332).  The last step of a call, a
+  // 42.6.  In a large system it competes with the move instead, and the two places
+  // cost the same over a wide range: late / early 109 / 109 us at 860,000 slots, 130
+  // / 132 at 1.1M, 202 / 203 at 1.9M, 128 / 130 at 1.5M in 96 replicas, 202 / 202 at
+  // 2.7M, 330 / 319 at 4.7M in 256.  The last step of a call, a
   // recorded step (its census reads the photon state) and proximity FRET (a
   // search over the step's own cell list) run it right after the step.  The
   // detection pass reads only the photon records, which carry their positions:

@@ -285,14 +285,15 @@ __global__ void __launch_bounds__(kBlock) k_phot_write(const EdmDynParams* __res
   const EdmDynParams& p = DP[t.r];
   const int64_t e0 = t.s - threadIdx.x, e_end = pp.emitter_offset + pp.n_emitters;
   const int ordinal = (int)((e0 - pp.emitter_offset) / kBlock);
+  const int n_mine = t.s < e_end ? ph.emit_n[t.s] : 0;
+  const int64_t tile_total = ph.tile_n[blockIdx.x];
   int64_t before = 0;
   for (int k = threadIdx.x; k < ordinal; k += kBlock) before += ph.tile_n[blockIdx.x - ordinal + k];
   const int64_t base = block_sum(before);
-  const int64_t tile_total = ph.tile_n[blockIdx.x];
   constexpr int kMost = INT32_MAX - kBlock;
   int total;
   if (tile_total <= kMost) {
-    first[threadIdx.x] = block_exclusive_scan(t.s < e_end ? ph.emit_n[t.s] : 0, total);
+    first[threadIdx.x] = block_exclusive_scan(n_mine, total);
   } else {
     // more than any buffer below 64 GB holds: the indices past kMost are all
     // dropped, and each thread adds up its emitter's first one in 64 bits
