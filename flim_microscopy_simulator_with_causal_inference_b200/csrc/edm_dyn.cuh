@@ -1633,15 +1633,55 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contacts_list(const EdmDynPara
 // substrate of the later reactions `late`: its alive neighbours of those
 // reactions' enzyme species passing the tests an enzyme-side sweep makes
 // (j seen from enzyme e at the opposite cell offset, the same float32
-// expressions), and with WOKEN its neighbours among the particles woken in the
-// step, which the cells do not hold; appended to the reactions' lists.
-template <bool F64, bool WOKEN>
+// expressions), appended to the reactions' lists.
+template <bool F64>
 __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
                                            int64_t j, int id_j, int64_t step, uint32_t late,
                                            const ContactOut& out) {
   uint32_t emask = 0;
   for (uint32_t b = late; b; b &= b - 1) emask |= 1u << p.cat[__ffs(b) - 1].enzyme;
-  auto file = [&](int e, int spe) {
+  for_neighbour_slots(g, st, st.cell_pre[j], [&](int e, int, int dcx, int dcy) {
+    if (e == j) return;
+    const uint8_t fe = st.flags[e];
+    const int spe = fl_species(fe);
+    if (!fl_alive(fe) || !((emask >> spe) & 1u)) return;
+    double d2;
+    if constexpr (F64) {
+      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())) return;
+      d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
+    } else {
+      const float2 oe = ((const float2*)st.pos_pre)[e], oj = ((const float2*)st.pos_pre)[j];
+      const float fdx = __fmaf_rn(-(float)(-dcx), g.sxf, oe.x - oj.x);
+      const float fdy = __fmaf_rn(-(float)(-dcy), g.syf, oe.y - oj.y);
+      if (!((double)__fmaf_rn(fdx, fdx, fdy * fdy) < g.cutoff_sq())) return;
+      d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
+    }
+    for (uint32_t b = late; b; b &= b - 1) {
+      const int c = __ffs(b) - 1;
+      if (spe != p.cat[c].enzyme || d2 > p.cat[c].contact_sq) continue;
+      if (!cat_draw_passes(p, st, r, c, slot_id(st, e) - (int)g.poff, id_j, step)) continue;
+      out.file(c, e, (int)j);
+    }
+  });
+}
+
+// And those of its neighbours among the particles woken in the step, which the
+// cells do not hold.
+template <bool F64>
+__device__ __forceinline__ void late_woken_contacts(const EdmDynParams& p, const Geo& g, const DevState& st, int r,
+                                                 int64_t j, int id_j, int64_t step, uint32_t late,
+                                                 const ContactOut& out) {
+  uint32_t enzymes = 0, woken = 0;
+  for (uint32_t b = late; b; b &= b - 1) enzymes |= 1u << p.cat[__ffs(b) - 1].enzyme;
+  for (int b = 0; b < p.n_bind; ++b) woken |= enzymes & (1u << p.bind[b].rb);
+  if (!woken) return;
+  const int n = min(st.moved_count[r], (int)p.n_particles);
+  for (int k = 0; k < n; ++k) {
+    const int e = st.moved[p.particle_offset + k];
+    const uint8_t fe = st.flags[e];
+    const int spe = fl_species(fe);
+    if (e == j || !fl_alive(fe) || !((woken >> spe) & 1u)) continue;
+    if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())) continue;
     const double d2 = sep_sq<F64>(st.pos_post, st.cell_post, e, j, g);
     for (uint32_t b = late; b; b &= b - 1) {
       const int c = __ffs(b) - 1;
@@ -1649,33 +1689,6 @@ __device__ __forceinline__ void late_contacts(const EdmDynParams& p, const Geo& 
       if (!cat_draw_passes(p, st, r, c, slot_id(st, e) - (int)g.poff, id_j, step)) continue;
       out.file(c, e, (int)j);
     }
-  };
-  for_neighbour_slots(g, st, st.cell_pre[j], [&](int e, int, int dcx, int dcy) {
-    if (e == j) return;
-    const uint8_t fe = st.flags[e];
-    const int spe = fl_species(fe);
-    if (!fl_alive(fe) || !((emask >> spe) & 1u)) return;
-    if constexpr (F64) {
-      if (!(sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())) return;
-    } else {
-      const float2 oe = ((const float2*)st.pos_pre)[e], oj = ((const float2*)st.pos_pre)[j];
-      const float fdx = __fmaf_rn(-(float)(-dcx), g.sxf, oe.x - oj.x);
-      const float fdy = __fmaf_rn(-(float)(-dcy), g.syf, oe.y - oj.y);
-      if (!((double)__fmaf_rn(fdx, fdx, fdy * fdy) < g.cutoff_sq())) return;
-    }
-    file(e, spe);
-  });
-  if constexpr (!WOKEN) return;
-  uint32_t woken = 0;  // enzyme species that a dissociation can wake
-  for (int b = 0; b < p.n_bind; ++b) woken |= emask & (1u << p.bind[b].rb);
-  if (!woken) return;
-  const int n = min(st.moved_count[r], (int)p.n_particles);
-  for (int k = 0; k < n; ++k) {
-    const int e = st.moved[p.particle_offset + k];
-    const uint8_t fe = st.flags[e];
-    if (e != j && fl_alive(fe) && ((woken >> fl_species(fe)) & 1u) &&
-        sep_sq<F64>(st.pos_pre, st.cell_pre, e, j, g) < g.cutoff_sq())
-      file(e, fl_species(fe));
   }
 }
 
@@ -1705,7 +1718,10 @@ __device__ __forceinline__ void catalytic_pair(const EdmDynParams& p, const DevS
   if (u < peff && cas_u8(&st.flags[es.y], fs, fl_make(C.product, true))) {
     atomic_add_i64(&st.counters[(int64_t)r * EDM_NCOUNTERS + EDM_C_CATALYTIC], 1);
     grid_change(p, sink, C.substrate, true, C.product, true, xs, ys);
-    if (late) late_contacts<F64, WOKEN>(p, g, st, r, es.y, ids, *st.d_step, late, out);
+    if (late) {
+      late_contacts<F64>(p, g, st, r, es.y, ids, *st.d_step, late, out);
+      if constexpr (WOKEN) late_woken_contacts<F64>(p, g, st, r, es.y, ids, *st.d_step, late, out);
+    }
   }
 }
 
